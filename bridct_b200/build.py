@@ -2,7 +2,7 @@
 
     python -m bridct_b200.build          # or __graft_entry__.build()
 
-Steps: regenerate csrc/sj_generated.cuh from csrc/gen_sj.py when the generator changed,
+Steps: regenerate csrc/sj_generated.cuh and csrc/sj_packed.cuh from csrc/gen_sj.py when it changed,
 compile each CUDA translation unit with nvcc (-gencode arch=compute_100a,code=sm_100a), the
 plain-form instantiations once per array height in parallel, and link one shared library
 with the CUDA runtime linked statically; then build the pipe runner against it.  Objects go to _build/ at the repository root.
@@ -50,10 +50,11 @@ def _run(cmd) -> None:
 
 def generate() -> None:
     gen = CSRC / "gen_sj.py"
-    hdr = CSRC / "sj_generated.cuh"
-    if _newer(hdr, [gen]):
-        r = subprocess.run([sys.executable, str(gen)], capture_output=True, text=True, check=True)
-        hdr.write_text(r.stdout)
+    for name, args in (("sj_generated.cuh", []), ("sj_packed.cuh", ["--packed"])):
+        hdr = CSRC / name
+        if _newer(hdr, [gen]):
+            r = subprocess.run([sys.executable, str(gen)] + args, capture_output=True, text=True, check=True)
+            hdr.write_text(r.stdout)
 
 
 def build(verbose: bool = False) -> Path:

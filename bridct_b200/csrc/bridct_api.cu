@@ -94,6 +94,37 @@ void build_fourstep_tables(int N, std::vector<float2>& tw, std::vector<float4>& 
   fill_fourstep_tables(N, tw.data(), post.data());
 }
 
+// Rotation tables of the split lines of N points (sj_split.cuh, SplitTab): stage-1 twiddles
+// w_N^{bc} s(A, c), then the post rotations with the stage-2 scale of each output (s(B, j); s(B/2, m)
+// for column A/2) and the orthonormal factor folded in.
+template <int N>
+static std::vector<float> build_split_tables() {
+  constexpr int A = Split<N>::A, B = Split<N>::B, copies = SplitTab<N>::kWords / 2;
+  std::vector<float> t;
+  t.reserve(SplitTab<N>::kFloats);
+  auto put = [&t](double x, double y) {
+    t.insert(t.end(), copies, (float)x);
+    t.insert(t.end(), copies, (float)y);
+  };
+  for (int c = 0; c < A / 2; ++c)
+    for (int b = 0; b < B; ++b) {
+      const double ang = -2 * M_PI * (double)b * c / N, s = sj_scale(A, c);
+      put(std::cos(ang) * s, std::sin(ang) * s);
+    }
+  for (int j = 0; j < B; ++j)
+    for (int c = 0; c < A / 2; ++c) {
+      if (c == 0 && j == 0) {
+        put(std::sqrt(1.0 / N), std::sqrt(2.0 / N) * sj_scale(B, B / 2) * std::cos(M_PI / 4));
+        continue;
+      }
+      const bool second = c == 0 && j >= B / 2;   // column A/2
+      const int k = second ? A / 2 + 2 * A * (j - B / 2) : c + A * j;
+      const double s = std::sqrt(2.0 / N) * (second ? sj_scale(B / 2, j - B / 2) : sj_scale(B, j));
+      put(s * std::cos(M_PI * k / (2.0 * N)), s * std::sin(M_PI * k / (2.0 * N)));
+    }
+  return t;
+}
+
 #define BRIDCT_DECL_H(H)                                                            \
   void plain_table_h##H(PlainLauncher (*row)[3], UnitLauncher* col, UnitLauncher* rowu); \
   int merged_strip_cols_h##H();                                                      \
@@ -184,6 +215,21 @@ DeviceCtx* device_ctx(int device) {
     d->fourstep[i].tw = (const float2*)mem;
     d->fourstep[i].post = (const float4*)((char*)mem + btw);
   }
+  const std::vector<float> split[4] = {build_split_tables<128>(), build_split_tables<256>(), build_split_tables<512>(),
+                                       build_split_tables<1024>()};
+  for (int i = 0; i < 4; ++i) {
+    void* mem = nullptr;
+    e = cudaMalloc(&mem, split[i].size() * sizeof(float));
+    if (e == cudaSuccess) {
+      d->table_mem.push_back(mem);
+      e = cudaMemcpy(mem, split[i].data(), split[i].size() * sizeof(float), cudaMemcpyHostToDevice);
+    }
+    if (e != cudaSuccess) {
+      cuda_fail(e, "split-line tables");
+      return nullptr;
+    }
+    d->split[i].t = (const float*)mem;
+  }
   DeviceCtx* raw = d.get();
   g_devices[device] = std::move(d);
   return raw;
@@ -192,6 +238,13 @@ DeviceCtx* device_ctx(int device) {
 FourStepTables DeviceCtx::tables(int n) const {
   if (n < 128) return FourStepTables{nullptr, nullptr};
   return fourstep[lg2(n) - 4];
+}
+
+LineTables DeviceCtx::line_tables(int h, int w) const {
+  LineTables t{tables(h), tables(w)};
+  if (h >= 128) t.scol = split[lg2(h) - 4];
+  if (w >= 128) t.srow = split[lg2(w) - 4];
+  return t;
 }
 
 int current_device(int* dev) {
@@ -228,7 +281,7 @@ int launch_plain_form(const bridct_plan* p, int mode, const float* x, float* y, 
 
 int launch_plain_layout(DeviceCtx* d, int h, int w, int mode, const float* x, float* y, long long batch,
                         const BatchLayout* lx, const BatchLayout* ly, cudaStream_t st) {
-  LineTables tab{d->tables(h), d->tables(w)};
+  const LineTables tab = d->line_tables(h, w);
   PlainLauncher fn = d->plain[lg2(h)][lg2(w)][mode];
   cudaError_t e = fn(x, y, batch, st, tab, d->launch, lx, ly);
   if (e != cudaSuccess) return cuda_fail(e, "plain kernel launch");

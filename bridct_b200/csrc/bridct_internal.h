@@ -21,8 +21,10 @@ struct DeviceCtx {
   UnitLauncher col_units[8][3] = {};    // merged column passes, by lg(column length) and mode
   UnitLauncher row_units[8][3] = {};    // merged row passes, by lg(row length) and mode
   FourStepTables fourstep[4] = {};      // N = 128, 256, 512, 1024
+  SplitTables split[4] = {};            // the same lengths
   std::vector<void*> table_mem;
   FourStepTables tables(int n) const;
+  LineTables line_tables(int h, int w) const;
 };
 
 void set_error(const std::string& s);

@@ -598,6 +598,153 @@ def generate() -> str:
 
 
 # ----------------------------------------------------------------------------------------
+# Programs over a value type T (sj_packed.cuh): T = F2 runs two lines at once with the packed
+# f32x2 instructions, T = float one line.  Both round every operation alike: a multiplication whose
+# only use is an addition is fused here, explicitly, and nothing else is contracted.
+# ----------------------------------------------------------------------------------------
+
+PACKED_LINES = (8, 16, 32, 64)      # whole lines in registers
+PACKED_LEAVES = (16, 32)            # stage 1 of a split line: real FFT over the A samples of one residue
+PACKED_STAGE2 = (8, 16, 32)         # stage 2: complex FFT over the B residues of one column
+
+
+def emit_packed(g: Graph, name: str, in_names: Sequence[str], outputs: Sequence[int],
+                out_names: Sequence[str], signature: str, doc: str) -> str:
+    """Emits a device function template over T computing outputs from inputs (in_names None: zero)."""
+    order = g.live(outputs)
+    uses: Dict[int, int] = {}
+    for n in order:
+        node = g.nodes[n]
+        for d in (node[1:3] if node[0] in ("add", "sub") else node[1:2] if node[0] in ("neg", "mul") else ()):
+            uses[d] = uses.get(d, 0) + 1
+    for o in outputs:
+        uses[o] = uses.get(o, 0) + 1
+    fused = set()
+    plan: Dict[int, tuple] = {}
+    for n in order:
+        node = g.nodes[n]
+        if node[0] not in ("add", "sub"):
+            continue
+        for m in (node[2], node[1]):
+            if g.nodes[m][0] == "mul" and uses[m] == 1 and m not in fused:
+                fused.add(m)
+                plan[n] = (m,)
+                break
+    lines = [f"// {doc}", "template <typename T>", f"__device__ __forceinline__ void {name}({signature}) {{"]
+    name_of: Dict[int, str] = {}
+    tmp = 0
+    for n in order:
+        node = g.nodes[n]
+        op = node[0]
+        if op == "in":
+            name_of[n] = f"i{node[1]}"
+            lines.append(f"  const T i{node[1]} = {in_names[node[1]]};")
+            continue
+        if n in fused:
+            continue
+        t = f"t{tmp}"
+        tmp += 1
+        if n in plan:
+            m = plan[n][0]
+            base, c = name_of[g.nodes[m][1]], g.nodes[m][2]
+            if op == "add":
+                expr = f"vfma({base}, {fconst(c)}, {name_of[node[2] if node[1] == m else node[1]]})"
+            elif node[2] == m:
+                expr = f"vfma({base}, {fconst(-c)}, {name_of[node[1]]})"
+            else:
+                expr = f"vfms({base}, {fconst(c)}, {name_of[node[2]]})"
+        elif op == "add":
+            expr = f"vadd({name_of[node[1]]}, {name_of[node[2]]})"
+        elif op == "sub":
+            expr = f"vsub({name_of[node[1]]}, {name_of[node[2]]})"
+        elif op == "neg":
+            expr = f"vneg({name_of[node[1]]})"
+        else:
+            expr = f"vmul({name_of[node[1]]}, {fconst(node[2])})"
+        lines.append(f"  const T {t} = {expr};")
+        name_of[n] = t
+    for o, nm in zip(outputs, out_names):
+        lines.append(f"  {nm} = {name_of[o]};")
+    lines.append("}")
+    return "\n".join(lines)
+
+
+def build_special(n: int):
+    """Stage 2 of columns 0 and A/2 of a split line (B = n residues), whose stage-1 values r0_b, r1_b
+    are real: inputs r0_0, r1_0, r0_1, r1_1, ...; outputs n complex values
+        0            (V_0, V_{N/2}) of column 0, both real, as one pair
+        1..n/2-1     V_{A j} of column 0
+        n/2 + m      V_{A/2 + A 2m} of column A/2
+    Column 0 is a real FFT (scaled by 1/s(n, j)).  Column A/2 is sum_b r1_b w_n^{b (d + 1/2)}, whose
+    values at odd d are the conjugates of those at n-1-d; the even ones are a complex FFT of length
+    n/2 (scaled by 1/s(n/2, m)) of (r1_j - i r1_{j+n/2}) w_n^{j/2}."""
+    def prog(g, ins):
+        z0 = rfft(g, ins[0::2], "S")
+        r1 = ins[1::2]
+        h = n // 2
+        folded = []
+        for j in range(h):
+            w = complex(math.cos(math.pi * j / n), -math.sin(math.pi * j / n))
+            folded.append(g.cmulc((r1[j], g.neg(r1[j + h])), w))
+        z1 = cfft(g, folded, "S")
+        outs = [z0[0][0], z0[h][0]]
+        for j in range(1, h):
+            outs += [z0[j][0], z0[j][1]]
+        for m in range(h):
+            outs += [z1[m][0], z1[m][1]]
+        return outs
+    g = Graph()
+    outs = prog(g, [g.inp(i) for i in range(2 * n)])
+    gt = Graph()
+    outs_t = prog(gt, [gt.inp(2 * n + i) for i in range(2 * n)])
+    adj = [gt.inp(i) for i in range(2 * n)]
+    back = transpose(gt, outs_t, 4 * n, adj)[2 * n:]
+    return (g, outs), (gt, back)
+
+
+def generate_packed() -> str:
+    parts = [
+        "// Generated by gen_sj.py --packed: Shao-Johnson programs over a value type T (F2: two lines at",
+        "// once in packed f32x2 instructions; float: one line, rounded alike).",
+        "// Do not edit by hand; rerun `python gen_sj.py --packed > sj_packed.cuh`.",
+        "#pragma once",
+        "",
+    ]
+
+    def both(n_in, fwd, tr, name, in_arr, out_arr, sig_f, sig_t, doc):
+        (g, outs), (gt, back) = fwd, tr
+        m = len(outs)
+        parts.append(emit_packed(g, name, [f"{in_arr}[{i}]" for i in range(n_in)], outs,
+                                 [f"{out_arr}[{i}]" for i in range(m)], sig_f, doc))
+        parts.append("")
+        parts.append(emit_packed(gt, name + "_t", [f"{out_arr}[{i}]" for i in range(m)] + ["T()"] * n_in, back,
+                                 [f"{in_arr}[{i}]" for i in range(n_in)], sig_t, "transpose of " + name))
+        parts.append("")
+
+    for n in PACKED_LINES:
+        (g, fwd), (gi, inv), (gr, rt) = build_line_ops(n)
+        arr = [f"v[{i}]" for i in range(n)]
+        for gg, o, nm, kind, ins in ((g, fwd, f"sjp_fwd_{n}", "orthonormal DCT-II", arr),
+                                     (gi, inv, f"sjp_inv_{n}", "orthonormal DCT-III", arr + ["T()"] * n),
+                                     (gr, rt, f"sjp_rt_{n}", "DCT-III(DCT-II(v))", arr)):
+            parts.append(emit_packed(gg, nm, ins, o, arr, f"T (&v)[{n}]", f"{kind}, length {n}"))
+            parts.append("")
+    for n in PACKED_LEAVES:
+        f, t = build_rfft_leaf(n)
+        m = len(f[1])
+        both(n, f, t, f"sjp_rfft_{n}", "x", "w", f"const T (&x)[{n}], T (&w)[{m}]", f"const T (&w)[{m}], T (&x)[{n}]",
+             f"scaled real FFT, length {n}: w = re[0..{n // 2}], im[1..{n // 2 - 1}]")
+    for n in PACKED_STAGE2:
+        f, t = build_cfft(n)
+        both(2 * n, f, t, f"sjp_cfft_{n}", "z", "z", f"T (&z)[{2 * n}]", f"T (&z)[{2 * n}]",
+             f"scaled complex FFT, length {n}, interleaved re/im")
+        f, t = build_special(n)
+        both(2 * n, f, t, f"sjp_special_{n}", "z", "z", f"T (&z)[{2 * n}]", f"T (&z)[{2 * n}]",
+             f"stage 2 of the two real columns of a line split over {n} residues")
+    return "\n".join(parts)
+
+
+# ----------------------------------------------------------------------------------------
 # Self-test (float64): python gen_sj.py --check
 # ----------------------------------------------------------------------------------------
 
@@ -671,5 +818,7 @@ if __name__ == "__main__":
     sys.setrecursionlimit(100000)
     if "--check" in sys.argv:
         self_check()
+    elif "--packed" in sys.argv:
+        sys.stdout.write(generate_packed() + "\n")
     else:
         sys.stdout.write(generate() + "\n")

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include "sj_kernels.cuh"
 #include "sj_blocks8.cuh"
+#include "sj_split.cuh"
 
 namespace bridct {
 
@@ -76,6 +77,49 @@ static cudaError_t launch_tiles(Kernel k, int smem, int bps, TileArgs a, const L
   long long grid = (long long)ctx.sm_count * bps;
   if (grid > a.ntiles) grid = a.ntiles;
   return launch_pdl(k, (unsigned)grid, (unsigned)threads, smem, st, pdl, a);
+}
+
+// One CTA per strip or row block of a pass of split lines.  Always with programmatic dependent launch:
+// the table copy overlaps the previous kernel's end (+1% on 128 MiB batches, +0..4% on 16 MiB ones,
+// -4% on 16 MiB of 512-point columns).
+template <typename Kernel>
+static cudaError_t launch_split(Kernel k, int smem, int threads, long long units, const SplitArgs& a, cudaStream_t st) {
+  if (kernel_blocks_per_sm(k, smem, threads) <= 0) return cudaErrorInvalidConfiguration;
+  if (units <= 0) return cudaSuccess;
+  if (units > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+  return launch_pdl(k, (unsigned)units, (unsigned)threads, smem, st, true, a);
+}
+
+// Narrow units (strips of 8 columns, blocks of 8 rows) take about half the time of a wide one, so they
+// pay where the wide ones leave SMs idle.  Measured on batches of 2^16..2^22 elements of nine shapes:
+// row blocks of 8 are 10..40% faster below one wide block per SM and 5..25% slower above; strips of 8
+// columns (32-byte row segments) are 2..10% faster up to 64 wide strips where the rows are few too,
+// and 10..30% slower from 128 strips on.
+template <int W> static bool few_rows(long long rows, const LaunchCtx& ctx) { return rows / RowGeo<W>::RB < ctx.sm_count; }
+
+// Column pass x -> y of `batch` H x W arrays (H >= 128).
+template <int H, int W, int MODE, bool GEN>
+cudaError_t launch_split_cols(const float* x, float* y, long long batch, const BatchLayout& lx, const BatchLayout& ly,
+                              SplitTables tab, const LaunchCtx& ctx, cudaStream_t st) {
+  using Wide = ColGeo<H>;
+  using Few = ColGeo<H, kFewPairs>;
+  const SplitArgs a{x, y, tab, W, lx, ly, nullptr};
+  const long long units = batch * (W / Wide::TC);
+  if ((units <= 64 && (W < 128 || few_rows<cmax(W, 128)>(batch * H, ctx))) || (GEN && lx.small_units))
+    return launch_split(k_split_cols<H, GEN ? 0 : W, MODE, kFewPairs>, Few::kSmem, Few::T, batch * (W / Few::TC), a, st);
+  return launch_split(k_split_cols<H, GEN ? 0 : W, MODE, col_pairs<H>()>, Wide::kSmem, Wide::T, units, a, st);
+}
+
+// Row pass in place in y (W >= 128).
+template <int H, int W, int MODE, bool GEN>
+cudaError_t launch_split_rows(float* y, long long batch, const BatchLayout& ly, SplitTables tab, const LaunchCtx& ctx,
+                              cudaStream_t st) {
+  using Wide = RowGeo<W>;
+  using Few = RowGeo<W, kFewPairs>;
+  const SplitArgs a{y, y, tab, W, ly, ly, nullptr};
+  if (few_rows<W>(batch * H, ctx) || (GEN && ly.small_units))
+    return launch_split(k_split_rows<W, GEN ? H : 0, MODE, kFewPairs>, Few::kSmem, Few::T, batch * H / Few::RB, a, st);
+  return launch_split(k_split_rows<W, GEN ? H : 0, MODE, 8>, Wide::kSmem, Wide::T, batch * H / Wide::RB, a, st);
 }
 
 // Route of an (H, W, MODE) batch: whole 32768-float arrays as single tiles in the modes where that
@@ -169,53 +213,29 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
     TileArgs a{x, y, batch, batch * H, tab, lx, ly};
     return launch_tiles(k, Gm::kSmemWhole, bps, a, ctx, st);
   } else {
-    // Round trips of 128-point register lines run 128-thread CTAs without register prefetch:
-    // every warp has a line and two CTAs share an SM, which measured +8..13% over one 256-thread
-    // CTA with prefetch; forward and inverse measured 5..9% slower that way and keep 256 threads.
-    constexpr int TC_T = H == 128 && MODE == LM_RT ? 128 : kThreads;
-    constexpr int TR_T = W == 128 && MODE == LM_RT ? 128 : kThreads;
-    constexpr int kSmemC = Gm::template strip_smem_used<MODE, TC_T>(Gm::kTC);
-    constexpr int kSmemCs = Gm::template strip_smem_used<MODE, TC_T>(Gm::kTCs);
-    constexpr int kSmemR = Gm::template rows_smem_used<MODE, TR_T>(Gm::kRB);
-    constexpr int kSmemRs = Gm::template rows_smem_used<MODE, TR_T>(Gm::kRBs);
-    auto kc = k_colstrip<H, W, Gm::kTC, MODE, TC_T, GEN>;
-    auto kr = k_full<H, W, Gm::kRB, false, true, MODE, TR_T, GEN>;
-    const int bpc = kernel_blocks_per_sm(kc, kSmemC, TC_T);
-    const int bpr = kernel_blocks_per_sm(kr, kSmemR, TR_T);
-    // One column-strip launch and one row-block launch over the whole batch.  Cutting the batch
-    // into L2-sized chunks (so that the intermediate stays in L2 between the two passes) measured
-    // slower on every two-pass shape: the four-step kernels are bound by shared-memory latency,
-    // not by HBM, while every chunk adds two launch tails (128 MiB batches +16..48% unchunked,
-    // 2048 x 256^2 1669 -> 2129 GB/s).
-    const long long nb = batch;
+    // One column launch and one row launch over the whole batch.  Lines of 128 points and more run as
+    // split lines; shorter columns (32 x 1024 round trips, 64 x 1024) and 64-point rows as register
+    // lines.
     cudaError_t e;
-    const bool few = nb * (W / Gm::kTC) < 2LL * ctx.sm_count;   // passes below a full grid: PDL
-    const bool small = few || (GEN && lx.small_units);
-    if (small) {   // few arrays (or asked for): smaller strips and row blocks
-      auto kcs = k_colstrip<H, W, Gm::kTCs, MODE, TC_T, GEN>;
-      TileArgs ac{x, y, nb * (W / Gm::kTCs), nb * H, tab, lx, ly};
-      e = launch_tiles(kcs, kSmemCs, kernel_blocks_per_sm(kcs, kSmemCs, TC_T), ac, ctx, st, TC_T,
-                       few);
+    if constexpr (H >= 128) {
+      e = launch_split_cols<H, W, MODE, GEN>(x, y, batch, lx, ly, tab.scol, ctx, st);
     } else {
-      TileArgs ac{x, y, nb * (W / Gm::kTC), nb * H, tab, lx, ly};
-      e = launch_tiles(kc, kSmemC, bpc, ac, ctx, st, TC_T, false);
+      auto kc = k_colstrip<H, W, Gm::kTC, MODE, kThreads, GEN>;
+      constexpr int smem = Gm::strip_smem(Gm::kTC);
+      const bool few = batch * (W / Gm::kTC) < 2LL * ctx.sm_count;   // below a full grid: PDL
+      TileArgs ac{x, y, batch * (W / Gm::kTC), batch * H, tab, lx, ly};
+      e = launch_tiles(kc, smem, kernel_blocks_per_sm(kc, smem), ac, ctx, st, kThreads, few);
     }
     if (e != cudaSuccess) return e;
-    if constexpr (Gm::kNarrowRows) {
-      auto krn = k_full<H, W, Gm::kRBn, false, true, MODE, 128, GEN>;
-      TileArgs ar{y, y, nb * H / Gm::kRBn, nb * H, tab, ly, ly};
-      e = launch_tiles(krn, Gm::kSmemRowsN, kernel_blocks_per_sm(krn, Gm::kSmemRowsN, 128), ar, ctx, st, 128, few);
-    } else if (nb * H / Gm::kRB < 2LL * ctx.sm_count || (GEN && lx.small_units)) {
-      auto krs = k_full<H, W, Gm::kRBs, false, true, MODE, TR_T, GEN>;
-      TileArgs ar{y, y, nb * H / Gm::kRBs, nb * H, tab, ly, ly};
-      e = launch_tiles(krs, kSmemRs, kernel_blocks_per_sm(krs, kSmemRs, TR_T), ar, ctx, st, TR_T,
-                       few);
+    if constexpr (W >= 128) {
+      return launch_split_rows<H, W, MODE, GEN>(y, batch, ly, tab.srow, ctx, st);
     } else {
-      TileArgs ar{y, y, nb * H / Gm::kRB, nb * H, tab, ly, ly};
-      e = launch_tiles(kr, kSmemR, bpr, ar, ctx, st, TR_T, false);
+      auto kr = k_full<H, W, Gm::kRB, false, true, MODE, kThreads, GEN>;
+      constexpr int smem = Gm::rows_smem(Gm::kRB);
+      const bool few = batch * H / Gm::kRB < 2LL * ctx.sm_count;
+      TileArgs ar{y, y, batch * H / Gm::kRB, batch * H, tab, ly, ly};
+      return launch_tiles(kr, smem, kernel_blocks_per_sm(kr, smem), ar, ctx, st, kThreads, few);
     }
-    if (e != cudaSuccess) return e;
-    return cudaSuccess;
   }
 }
 
@@ -237,26 +257,32 @@ using UnitLauncher = cudaError_t (*)(const float*, float*, const PassUnit*, long
 template <int H, int MODE>
 cudaError_t launch_col_units(const float* x, float* y, const PassUnit* units, long long n, cudaStream_t st,
                              LineTables tab, const LaunchCtx& ctx) {
-  using Gm = Geometry<H, 1024>;
-  constexpr int TC_T = H == 128 && MODE == LM_RT ? 128 : kThreads;
-  auto k = k_colstrip<H, 1024, Gm::kTC, MODE, TC_T, false, true>;
-  TileArgs a{x, y, n, n * H, tab, BatchLayout{}, BatchLayout{}, units};
-  return launch_tiles(k, Gm::kSmemStrip, kernel_blocks_per_sm(k, Gm::kSmemStrip, TC_T), a, ctx, st, TC_T, false);
+  if constexpr (H >= 128) {
+    using Geo = ColGeo<H>;
+    return launch_split(k_split_cols<H, 0, MODE, col_pairs<H>()>, Geo::kSmem, Geo::T, n,
+                        SplitArgs{x, y, tab.scol, 0, BatchLayout{}, BatchLayout{}, units}, st);
+  } else {
+    using Gm = Geometry<H, 1024>;
+    auto k = k_colstrip<H, 1024, Gm::kTC, MODE, kThreads, false, true>;
+    constexpr int smem = Gm::strip_smem(Gm::kTC);
+    TileArgs a{x, y, n, n * H, tab, BatchLayout{}, BatchLayout{}, units};
+    return launch_tiles(k, smem, kernel_blocks_per_sm(k, smem), a, ctx, st, kThreads, false);
+  }
 }
 
 template <int W, int MODE>
 cudaError_t launch_row_units(const float* x, float* y, const PassUnit* units, long long n, cudaStream_t st,
                              LineTables tab, const LaunchCtx& ctx) {
-  using Gm = Geometry<1024, W>;
-  if constexpr (Gm::kNarrowRows) {
-    auto k = k_full<1024, W, Gm::kRBn, false, true, MODE, 128, false, true>;
-    TileArgs a{x, y, n, n * Gm::kRBn, tab, BatchLayout{}, BatchLayout{}, units};
-    return launch_tiles(k, Gm::kSmemRowsN, kernel_blocks_per_sm(k, Gm::kSmemRowsN, 128), a, ctx, st, 128, false);
+  if constexpr (W >= 128) {
+    using Geo = RowGeo<W>;
+    return launch_split(k_split_rows<W, W, MODE, 8>, Geo::kSmem, Geo::T, n,
+                        SplitArgs{x, y, tab.srow, 0, BatchLayout{}, BatchLayout{}, units}, st);
   } else {
-    constexpr int TR_T = W == 128 && MODE == LM_RT ? 128 : kThreads;
-    auto k = k_full<1024, W, Gm::kRB, false, true, MODE, TR_T, false, true>;
+    using Gm = Geometry<1024, W>;
+    auto k = k_full<1024, W, Gm::kRB, false, true, MODE, kThreads, false, true>;
+    constexpr int smem = Gm::rows_smem(Gm::kRB);
     TileArgs a{x, y, n, n * Gm::kRB, tab, BatchLayout{}, BatchLayout{}, units};
-    return launch_tiles(k, Gm::kSmemRows, kernel_blocks_per_sm(k, Gm::kSmemRows, TR_T), a, ctx, st, TR_T, false);
+    return launch_tiles(k, smem, kernel_blocks_per_sm(k, smem), a, ctx, st, kThreads, false);
   }
 }
 

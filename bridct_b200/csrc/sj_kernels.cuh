@@ -32,9 +32,15 @@ __host__ __device__ constexpr int reg_line_max(int N, int other, int mode, bool 
   return N == 128 && (two_pass || other >= 128 || mode == LM_RT || other <= 32) ? 128 : 64;
 }
 
+// Rotation tables of the split lines (sj_split.cuh), in global memory.
+struct SplitTables {
+  const float* t = nullptr;   // tw, then post (SplitTab<N>::kFloats floats, 16-byte aligned)
+};
+
 struct LineTables {
   FourStepTables col;   // for line length h (used when h >= 128)
   FourStepTables row;   // for line length w (used when w >= 128)
+  SplitTables scol, srow;
 };
 
 // Where the arrays of a launch live in a general layout (kernels instantiated with GEN): array b

@@ -1,0 +1,538 @@
+// Long lines (128..1024 points) of the plain form, two lines per thread.
+//
+// A line of N = A * B points is split as in sj_lines.cuh: stage 1 runs, for each residue b < B, the
+// SJ scaled real FFT of length A of v[B a + b] (v: Makhoul's reorder of x); stage 2 runs, for each
+// column c < A / 2, the SJ scaled complex FFT of length B over the twiddled stage-1 outputs and the
+// post rotation that gives y[c + A d] and y[N - c - A d].  The real columns 0 and A/2 make one
+// stage-2 task together (sjp_special), so a line has B stage-1 and A/2 stage-2 tasks of 2B values.
+//
+// What bounds long lines is instruction issue (about 35 thread instructions per element and pass
+// when one warp holds whole lines and each thread one value at a time), so here
+//   * a thread runs the same task of TWO lines in packed f32x2 arithmetic (F2): one issue slot does
+//     two additions or multiply-adds, and one 64-bit access moves two values.  The packed
+//     instructions run at half the rate of the scalar ones, so the arithmetic pipe is as busy as
+//     before and half the issue slots are free for everything else;
+//   * the lanes of a warp hold different lines at the same (or a few adjacent) b or c, so twiddles
+//     and post coefficients are broadcast loads, offsets are compile-time constants and nothing is
+//     conflicted or gathered;
+//   * column lines come from and go to global memory directly (a row of the strip is one coalesced
+//     segment): shared memory carries the stage-1 / stage-2 exchange only, one write and one read
+//     per element instead of six.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "sj_kernels.cuh"
+
+namespace bridct {
+
+// ---- value types of the packed programs --------------------------------------------------------
+struct F2 {
+  unsigned long long v = 0;
+};
+__device__ __forceinline__ F2 f2_make(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_split(F2 a, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+__device__ __forceinline__ F2 vadd(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 vsub(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 vmul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 vneg(F2 a) {
+  float x, y;
+  f2_split(a, x, y);
+  return f2_make(-x, -y);
+}
+__device__ __forceinline__ F2 vmul(F2 a, float c) { return vmul(a, f2_make(c, c)); }
+__device__ __forceinline__ F2 vfma(F2 a, float c, F2 b) { return vfma(a, f2_make(c, c), b); }
+__device__ __forceinline__ F2 vfms(F2 a, float c, F2 b) { return vfma(a, f2_make(c, c), vneg(b)); }
+__device__ __forceinline__ F2 vbcast(float c, F2) { return f2_make(c, c); }
+
+}  // namespace bridct
+
+#include "sj_packed.cuh"
+
+namespace bridct {
+
+// ---- split geometry and tables ------------------------------------------------------------
+template <int N> struct Split;
+template <> struct Split<128> { static constexpr int A = 16, B = 8; };
+template <> struct Split<256> { static constexpr int A = 32, B = 8; };
+template <> struct Split<512> { static constexpr int A = 32, B = 16; };
+template <> struct Split<1024> { static constexpr int A = 32, B = 32; };
+
+template <int A> struct Leaf;
+template <> struct Leaf<16> {
+  static __device__ __forceinline__ void fwd(const F2 (&x)[16], F2 (&w)[16]) { sjp_rfft_16<F2>(x, w); }
+  static __device__ __forceinline__ void tr(const F2 (&w)[16], F2 (&x)[16]) { sjp_rfft_16_t<F2>(w, x); }
+};
+template <> struct Leaf<32> {
+  static __device__ __forceinline__ void fwd(const F2 (&x)[32], F2 (&w)[32]) { sjp_rfft_32<F2>(x, w); }
+  static __device__ __forceinline__ void tr(const F2 (&w)[32], F2 (&x)[32]) { sjp_rfft_32_t<F2>(w, x); }
+};
+template <int B> struct Stage2;
+#define BRIDCT_STAGE2(B)                                                                       \
+  template <> struct Stage2<B> {                                                               \
+    static __device__ __forceinline__ void fwd(F2 (&z)[2 * B]) { sjp_cfft_##B<F2>(z); }        \
+    static __device__ __forceinline__ void tr(F2 (&z)[2 * B]) { sjp_cfft_##B##_t<F2>(z); }     \
+    static __device__ __forceinline__ void sfwd(F2 (&z)[2 * B]) { sjp_special_##B<F2>(z); }    \
+    static __device__ __forceinline__ void str(F2 (&z)[2 * B]) { sjp_special_##B##_t<F2>(z); } \
+  };
+BRIDCT_STAGE2(8)
+BRIDCT_STAGE2(16)
+BRIDCT_STAGE2(32)
+#undef BRIDCT_STAGE2
+
+// Rotations of one line length, A/2 * B of each kind:
+//   tw[c * B + b]          (x, y) = w_N^{b c} s(A, c), c = 1..A/2-1
+//   post[j * A/2 + c]      (P, Q): y[k] = P vr + Q vi and y[N-k] = Q vr - P vi for complex stage-2
+//     output j of task c (k = c + A j; task 0: see sjp_special, its output 0 is y[0] = P vr and
+//     y[N/2] = Q vi)
+// Each CTA keeps them in shared memory: read through L1 they cost the row pass a third of its time.
+// Up to 512 points every coefficient is stored twice, so that one 128-bit load gives two packed
+// operands without a move per coefficient; 1024-point lines have no room for that.
+template <int N> struct SplitTab {
+  static constexpr bool kDup = N <= 512;
+  static constexpr int kEntries = Split<N>::A / 2 * Split<N>::B;   // of each kind
+  static constexpr int kWords = kDup ? 4 : 2;                      // floats of an entry
+  static constexpr int kFloats = 2 * kEntries * kWords;
+};
+// Starts copying the tables to shared memory (cp.async: the caller waits and synchronizes).
+template <int N, int T>
+__device__ __forceinline__ void split_stage_tables(SplitTables tab, float* s) {
+  for (int i = threadIdx.x; i < SplitTab<N>::kFloats / 4; i += T) cp_async16(s + 4 * i, tab.t + 4 * i);
+}
+// Entry i of the tables at t (shared memory) as two packed operands.
+template <int N>
+__device__ __forceinline__ void split_coef(const float* t, int i, F2& a, F2& b) {
+  if constexpr (SplitTab<N>::kDup) {
+    const float4 v = *reinterpret_cast<const float4*>(t + 4 * i);
+    a = f2_make(v.x, v.y);
+    b = f2_make(v.z, v.w);
+  } else {
+    const float2 v = *reinterpret_cast<const float2*>(t + 2 * i);
+    a = f2_make(v.x, v.x);
+    b = f2_make(v.y, v.y);
+  }
+}
+
+// Stage-1 tail: the twiddled columns 1..A/2-1 and the two real columns into the exchange slots
+// ex(c, part), part 0 = re and 1 = im (task 0: columns 0 and A/2).
+template <int N, typename Put>
+__device__ __forceinline__ void split_put(const F2 (&w)[Split<N>::A], int b, const float* tab, const Put& put) {
+  constexpr int A = Split<N>::A, B = Split<N>::B;
+  put(0, 0, w[0]);
+  put(0, 1, w[A / 2]);
+#pragma unroll
+  for (int c = 1; c < A / 2; ++c) {
+    F2 tx, ty;
+    split_coef<N>(tab, c * B + b, tx, ty);
+    const F2 wr = w[c], wi = w[A / 2 + c];
+    put(c, 0, vfma(vneg(wi), ty, vmul(wr, tx)));
+    put(c, 1, vfma(wi, tx, vmul(wr, ty)));
+  }
+}
+// Its transpose.
+template <int N, typename Get>
+__device__ __forceinline__ void split_get(F2 (&w)[Split<N>::A], int b, const float* tab, const Get& get) {
+  constexpr int A = Split<N>::A, B = Split<N>::B;
+  w[0] = get(0, 0);
+  w[A / 2] = get(0, 1);
+#pragma unroll
+  for (int c = 1; c < A / 2; ++c) {
+    F2 tx, ty;
+    split_coef<N>(tab, c * B + b, tx, ty);
+    const F2 tr = get(c, 0), ti = get(c, 1);
+    w[c] = vfma(ti, ty, vmul(tr, tx));
+    w[A / 2 + c] = vfma(vneg(tr), ty, vmul(ti, tx));
+  }
+}
+
+// Stage 2 of task c on its 2B exchange values z, with the post rotation: on return z[2j] and z[2j+1]
+// are y[k_j] and y[N - k_j] (y[0] and y[N/2] for j = 0 of task 0).
+template <int N>
+__device__ __forceinline__ void split_stage2(F2 (&z)[2 * Split<N>::B], int c, const float* tab) {
+  constexpr int A = Split<N>::A, B = Split<N>::B;
+  if (c == 0) Stage2<B>::sfwd(z);
+  else Stage2<B>::fwd(z);
+  const float* post = tab + SplitTab<N>::kEntries * SplitTab<N>::kWords;
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    F2 p, q;
+    split_coef<N>(post, j * (A / 2) + c, p, q);
+    const F2 vr = z[2 * j], vi = z[2 * j + 1];
+    z[2 * j] = vmul(vr, p);
+    z[2 * j + 1] = vmul(j == 0 && c == 0 ? vi : vr, q);
+    if (j > 0 || c != 0) {
+      z[2 * j] = vfma(vi, q, z[2 * j]);
+      z[2 * j + 1] = vfma(vneg(vi), p, z[2 * j + 1]);
+    }
+  }
+}
+// Its transpose: z holds y[k_j], y[N - k_j] on entry and the adjoint exchange values on return.
+template <int N>
+__device__ __forceinline__ void split_stage2_t(F2 (&z)[2 * Split<N>::B], int c, const float* tab) {
+  constexpr int A = Split<N>::A, B = Split<N>::B;
+  const float* post = tab + SplitTab<N>::kEntries * SplitTab<N>::kWords;
+#pragma unroll
+  for (int j = 0; j < B; ++j) {
+    F2 p, q;
+    split_coef<N>(post, j * (A / 2) + c, p, q);
+    const F2 yk = z[2 * j], yn = z[2 * j + 1];
+    z[2 * j] = vmul(yk, p);
+    z[2 * j + 1] = vmul(j == 0 && c == 0 ? yn : yk, q);
+    if (j > 0 || c != 0) {
+      z[2 * j] = vfma(yn, q, z[2 * j]);
+      z[2 * j + 1] = vfma(vneg(yn), p, z[2 * j + 1]);
+    }
+  }
+  if (c == 0) Stage2<B>::str(z);
+  else Stage2<B>::tr(z);
+}
+
+// Calls f(slot, k): z[slot] of task c is y[k].
+template <int N, typename Fn>
+__device__ __forceinline__ void split_outputs(int c, const Fn& f) {
+  constexpr int A = Split<N>::A, B = Split<N>::B;
+  if (c == 0) {
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      const int k = j < B / 2 ? A * j : A / 2 + 2 * A * (j - B / 2);
+      f(2 * j, k);
+      f(2 * j + 1, j == 0 ? N / 2 : N - k);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      f(2 * j, c + A * j);
+      f(2 * j + 1, N - A * j - c);
+    }
+  }
+}
+
+// Source row (Makhoul) of element a of residue b: v[n], n = B a + b.
+template <int N>
+__device__ __forceinline__ int split_src(int a, int b) {
+  constexpr int A = Split<N>::A, B = Split<N>::B;
+  return a < A / 2 ? 2 * B * a + 2 * b : 2 * N - 1 - 2 * B * a - 2 * b;
+}
+
+// ---- the lines of a tile in shared memory ---------------------------------------------------------
+// GROUPS groups of LP line pairs, T threads: thread t holds pair t % LP and tasks t / LP, ... (group
+// major) of either stage.  get(g, i) is element i of the thread's pair of group g, put(g, i, v) takes
+// the result, ex(g) the thread's first exchange slot: slot (c, part, b) lies c * CS + (part * B + b) * LP
+// further on.  The exchange may overlie what get() reads: a barrier lies between.  IN_PLACE: put()
+// may also overlie the exchange.
+template <int N, int LP> __host__ __device__ constexpr int split_cs() {
+  // a half-warp spans 16 / LP tasks c: padding keeps their slots in different banks
+  return 2 * Split<N>::B * LP + (LP < 16 ? LP : 0);
+}
+template <int N, int MODE, int T, int GROUPS, int LP, bool IN_PLACE, typename Get, typename Put, typename Ex>
+__device__ __forceinline__ void split_lines(const Get& get, const Put& put, const Ex& ex, const float* tab) {
+  constexpr int A = Split<N>::A, B = Split<N>::B, CS = split_cs<N, LP>();
+  constexpr int N1 = GROUPS * B * LP, N2 = GROUPS * (A / 2) * LP;   // threads' tasks of the two stages
+  constexpr int R1 = (N1 + T - 1) / T, R2 = (N2 + T - 1) / T;
+  static_assert(N1 % 32 == 0 && N2 % 32 == 0, "whole warps");
+  const int t = threadIdx.x / LP;
+  constexpr int TP = T / LP;
+  auto on1 = [&](int r) { return N1 % T == 0 || (int)threadIdx.x + r * T < N1; };
+  auto on2 = [&](int r) { return N2 % T == 0 || (int)threadIdx.x + r * T < N2; };
+  if constexpr (MODE != LM_INV) {
+    F2 w[R1][A];
+#pragma unroll
+    for (int r = 0; r < R1; ++r) {
+      const int i = t + r * TP, g = i / B, b = i % B;
+      if (on1(r)) {
+        F2 v[A];
+#pragma unroll
+        for (int e = 0; e < A; ++e) v[e] = get(g, split_src<N>(e, b));
+        Leaf<A>::fwd(v, w[r]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R1; ++r) {
+      const int i = t + r * TP, g = i / B, b = i % B;
+      if (on1(r)) {
+        F2* e = ex(g) + b * LP;
+        split_put<N>(w[r], b, tab, [&](int c, int part, F2 val) { e[c * CS + part * B * LP] = val; });
+      }
+    }
+    __syncthreads();
+    F2 z[IN_PLACE && MODE == LM_FWD ? R2 : 1][2 * B];
+#pragma unroll
+    for (int r = 0; r < R2; ++r) {
+      const int i = t + r * TP, g = i / (A / 2), c = i % (A / 2);
+      F2(&zr)[2 * B] = z[IN_PLACE && MODE == LM_FWD ? r : 0];
+      if (on2(r)) {
+        F2* e = ex(g) + c * CS;
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+          zr[2 * q] = e[q * LP];
+          zr[2 * q + 1] = e[(B + q) * LP];
+        }
+        split_stage2<N>(zr, c, tab);
+        if constexpr (MODE == LM_RT) {
+          split_stage2_t<N>(zr, c, tab);
+#pragma unroll
+          for (int q = 0; q < B; ++q) {
+            e[q * LP] = zr[2 * q];
+            e[(B + q) * LP] = zr[2 * q + 1];
+          }
+        } else if constexpr (!IN_PLACE) {
+          split_outputs<N>(c, [&](int j, int k) { put(g, k, zr[j]); });
+        }
+      }
+    }
+    if constexpr (MODE == LM_RT || IN_PLACE) __syncthreads();
+    if constexpr (MODE == LM_FWD && IN_PLACE) {
+#pragma unroll
+      for (int r = 0; r < R2; ++r) {
+        const int i = t + r * TP, g = i / (A / 2), c = i % (A / 2);
+        if (on2(r)) split_outputs<N>(c, [&](int j, int k) { put(g, k, z[r][j]); });
+      }
+    }
+  } else {
+    F2 z[R2][2 * B];
+#pragma unroll
+    for (int r = 0; r < R2; ++r) {
+      const int i = t + r * TP, g = i / (A / 2), c = i % (A / 2);
+      if (on2(r)) {
+        split_outputs<N>(c, [&](int j, int k) { z[r][j] = get(g, k); });
+        split_stage2_t<N>(z[r], c, tab);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R2; ++r) {
+      const int i = t + r * TP, g = i / (A / 2), c = i % (A / 2);
+      if (on2(r)) {
+        F2* e = ex(g) + c * CS;
+#pragma unroll
+        for (int q = 0; q < B; ++q) {
+          e[q * LP] = z[r][2 * q];
+          e[(B + q) * LP] = z[r][2 * q + 1];
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if constexpr (MODE != LM_FWD) {
+    F2 v[IN_PLACE ? R1 : 1][A];
+#pragma unroll
+    for (int r = 0; r < R1; ++r) {
+      const int i = t + r * TP, g = i / B, b = i % B;
+      F2(&vr)[A] = v[IN_PLACE ? r : 0];
+      if (on1(r)) {
+        const F2* e = ex(g) + b * LP;
+        F2 w[A];
+        split_get<N>(w, b, tab, [&](int c, int part) { return e[c * CS + part * B * LP]; });
+        Leaf<A>::tr(w, vr);
+        if constexpr (!IN_PLACE) {
+#pragma unroll
+          for (int e2 = 0; e2 < A; ++e2) put(g, split_src<N>(e2, b), vr[e2]);
+        }
+      }
+    }
+    if constexpr (IN_PLACE) {
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < R1; ++r) {
+        const int i = t + r * TP, g = i / B, b = i % B;
+        if (on1(r)) {
+#pragma unroll
+          for (int e = 0; e < A; ++e) put(g, split_src<N>(e, b), v[r][e]);
+        }
+      }
+    }
+  }
+}
+
+// ---- column pass -------------------------------------------------------------------------------
+struct SplitArgs {
+  const float* x;
+  float* y;
+  SplitTables tab;
+  int width;              // run-time layouts: columns of an array
+  BatchLayout lx, ly;     // run-time layouts
+  const PassUnit* units;  // one strip or row block per unit, where set
+};
+
+// A strip of TC columns is copied to shared memory (cp.async: loads into registers would be limited
+// by the L1 that the exchange leaves), transformed, and stored from registers, each row of the strip
+// one coalesced segment.  A thread holds two adjacent columns.  Strips of 16 columns are 64 bytes
+// wide: rows 2k and 2k + 1 share a 128-byte line and swap places in every other line, so that the
+// rows 2b, 2b + 2 (stage 1) and c, c + 1 (stage 2) which a half-warp reads lie in different banks.
+// Calls on a few arrays take strips of 8 columns (LP = 4), so that they spread over more SMs.
+template <int N> __host__ __device__ constexpr int col_pairs() { return N >= 512 ? 8 : 16; }
+constexpr int kFewPairs = 4;
+template <int N, int LP = col_pairs<N>()> struct ColGeo {
+  static constexpr int TC = 2 * LP;
+  static constexpr int T = 128;
+  static constexpr int kExch = Split<N>::A / 2 * split_cs<N, LP>() * 2;   // floats; covers the N x TC strip
+  static constexpr int kSmem = (kExch + SplitTab<N>::kFloats) * 4;
+};
+template <int TC>
+__device__ __forceinline__ int strip_row(int r) {
+  return TC == 16 ? (r >> 1) * 32 + (((r ^ (r >> 1)) & 1) << 4) : r * TC;
+}
+
+// One strip: x and y at its first element, rows xp / yp floats apart (W > 0: W apart).
+template <int N, int W, int MODE, int LP>
+__device__ __forceinline__ void split_col_unit(const float* x, float* y, long long xp, long long yp, float* smem,
+                                               const float* tab) {
+  using Geo = ColGeo<N, LP>;
+  constexpr int TC = Geo::TC, Q = TC / 4, T = Geo::T;
+#pragma unroll
+  for (int k = 0; k < N * Q / T; ++k) {
+    const int i = threadIdx.x + k * T, r = i / Q, c = (i % Q) * 4;
+    cp_async16(smem + strip_row<TC>(r) + c, x + (W > 0 ? (long long)(r * W) : r * xp) + c);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  const int p = 2 * (threadIdx.x % LP);
+  float* yt = y + p;
+  split_lines<N, MODE, T, 1, LP, false>(
+      [&](int, int i) {
+        const float2 v = *reinterpret_cast<const float2*>(smem + strip_row<TC>(i) + p);
+        return f2_make(v.x, v.y);
+      },
+      [&](int, int i, F2 v) {
+        float2 f;
+        f2_split(v, f.x, f.y);
+        *reinterpret_cast<float2*>(yt + (W > 0 ? (long long)(i * W) : i * yp)) = f;
+      },
+      [&](int) { return reinterpret_cast<F2*>(smem) + p / 2; }, tab);
+}
+
+// W > 0: strips of contiguous N x W arrays; W = 0: run-time layouts, or units.
+template <int N, int W, int MODE, int LP>
+__global__ void __launch_bounds__(128) k_split_cols(SplitArgs a) {
+  using Geo = ColGeo<N, LP>;
+  constexpr int TC = Geo::TC;
+  extern __shared__ float smem[];
+  float* tab = smem + Geo::kExch;
+  split_stage_tables<N, Geo::T>(a.tab, tab);
+  griddep_wait();
+  griddep_trigger();
+  if constexpr (W > 0) {
+    constexpr int S = W / TC;
+    const unsigned arr = blockIdx.x / S, s = blockIdx.x % S;
+    const long long off = (long long)arr * N * W + s * TC;
+    split_col_unit<N, W, MODE, LP>(a.x + off, a.y + off, W, W, smem, tab);
+  } else if (a.units) {
+    const PassUnit u = a.units[blockIdx.x];
+    split_col_unit<N, 0, MODE, LP>(a.x + u.off, a.y + u.off, u.ld, u.ld, smem, tab);
+  } else {
+    const unsigned S = a.width / TC, arr = blockIdx.x / S, s = blockIdx.x % S;
+    split_col_unit<N, 0, MODE, LP>(a.x + layout_row<N>(a.lx, (long long)arr * N) + s * TC,
+                                   a.y + layout_row<N>(a.ly, (long long)arr * N) + s * TC, a.lx.ld, a.ly.ld, smem, tab);
+  }
+}
+
+// ---- row pass ----------------------------------------------------------------------------------
+// Rows are staged whole in shared memory in groups of 2 LP, at pitch N + 32 / LP floats: a thread holds
+// rows p and p + LP of a group, and a warp LP such pairs at 32 / LP adjacent b's (or c's), so the
+// scalar walks along the rows hit bank (32 / LP) p + b: conflict-free.
+template <int N> __host__ __device__ constexpr int row_groups() { return N <= 256 ? 2 : 1; }
+template <int N, int LP = 8, int GROUPS = LP == 8 ? row_groups<N>() : 1> struct RowGeo {
+  static constexpr int P = N + 32 / LP;
+  static constexpr int T = 128;
+  static constexpr int RB = 2 * LP * GROUPS;
+  static constexpr int kExch = Split<N>::A / 2 * split_cs<N, LP>() * 2;
+  static constexpr int GP = 2 * LP * P > kExch ? 2 * LP * P : kExch;   // floats of one group
+  static constexpr int kTile = GROUPS * GP;
+  static constexpr int kSmem = (kTile + SplitTab<N>::kFloats) * 4;
+};
+
+// All rows of a tile of GROUPS groups, GP floats apart.
+template <int N, int MODE, int T, int GROUPS, int LP, int GP>
+__device__ __forceinline__ void split_rows(float* tile, const float* tab) {
+  constexpr int P = N + 32 / LP;
+  const int p = threadIdx.x % LP;
+  float* rows = tile + p * P;
+  split_lines<N, MODE, T, GROUPS, LP, true>(
+      [&](int g, int i) { return f2_make(rows[g * GP + i], rows[g * GP + i + LP * P]); },
+      [&](int g, int i, F2 v) { f2_split(v, rows[g * GP + i], rows[g * GP + i + LP * P]); },
+      [&](int g) { return reinterpret_cast<F2*>(tile + g * GP) + p; }, tab);
+}
+
+// Stores `bytes` (a multiple of 16) of shared memory to global memory asynchronously.
+__device__ __forceinline__ void bulk_store(float* dst, const float* src, int bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+               "r"(static_cast<unsigned>(__cvta_generic_to_shared(src))), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit_wait() {
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+// RB rows, row r at xrow(r) and yrow(r), in place or x -> y.
+template <int N, int MODE, int LP, typename XRow, typename YRow>
+__device__ __forceinline__ void split_row_unit(const XRow& xrow, const YRow& yrow, float* smem, const float* tab) {
+  using Geo = RowGeo<N, LP>;
+  constexpr int P = Geo::P, RB = Geo::RB, T = Geo::T, Q = N / 4;
+  auto srow = [&](int r) { return smem + (r / (2 * LP)) * Geo::GP + (r % (2 * LP)) * P; };
+#pragma unroll
+  for (int k = 0; k < RB * Q / T; ++k) {
+    const int i = threadIdx.x + k * T, r = i / Q, c = (i % Q) * 4;
+    cp_async16(srow(r) + c, xrow(r) + c);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  split_rows<N, MODE, T, Geo::RB / (2 * LP), LP, Geo::GP>(smem, tab);
+  fence_async();
+  __syncthreads();
+  if (threadIdx.x < RB) {
+    bulk_store(yrow(threadIdx.x), srow(threadIdx.x), N * 4);
+    bulk_commit_wait();
+  }
+}
+
+// RB consecutive rows of a (batch * H) x N matrix per CTA.  H = 0: contiguous rows; H > 0: run-time
+// layouts of arrays of H rows, or units.
+template <int N, int H, int MODE, int LP>
+__global__ void __launch_bounds__(128) k_split_rows(SplitArgs a) {
+  using Geo = RowGeo<N, LP>;
+  extern __shared__ float smem[];
+  float* tab = smem + Geo::kTile;
+  split_stage_tables<N, Geo::T>(a.tab, tab);
+  griddep_wait();
+  griddep_trigger();
+  const long long first = (long long)blockIdx.x * Geo::RB;
+  if constexpr (H == 0) {
+    split_row_unit<N, MODE, LP>([&](int r) { return a.x + (first + r) * N; },
+                                [&](int r) { return a.y + (first + r) * N; }, smem, tab);
+  } else if (a.units) {
+    const PassUnit u = a.units[blockIdx.x];
+    split_row_unit<N, MODE, LP>([&](int r) { return a.x + u.off + r * u.ld; },
+                                [&](int r) { return a.y + u.off + r * u.ld; }, smem, tab);
+  } else {
+    split_row_unit<N, MODE, LP>([&](int r) { return a.x + layout_row<H>(a.lx, first + r); },
+                                [&](int r) { return a.y + layout_row<H>(a.ly, first + r); }, smem, tab);
+  }
+}
+
+}  // namespace bridct
