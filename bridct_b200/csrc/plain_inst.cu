@@ -40,8 +40,8 @@ void BRIDCT_CAT(plain_table_h, BRIDCT_H)(PlainLauncher (*row)[3], UnitLauncher* 
 int BRIDCT_CAT(merged_strip_cols_h, BRIDCT_H)() { return ColGeo<BRIDCT_H>::TC; }
 int BRIDCT_CAT(merged_block_rows_w, BRIDCT_H)() { return RowGeo<BRIDCT_H>::RB; }
 #elif BRIDCT_H >= 32
-int BRIDCT_CAT(merged_strip_cols_h, BRIDCT_H)() { return Geometry<BRIDCT_H, 1024>::kTC; }
-int BRIDCT_CAT(merged_block_rows_w, BRIDCT_H)() { return Geometry<1024, BRIDCT_H>::kRB; }
+int BRIDCT_CAT(merged_strip_cols_h, BRIDCT_H)() { return PairColGeo<BRIDCT_H>::TC; }
+int BRIDCT_CAT(merged_block_rows_w, BRIDCT_H)() { return PairRowGeo<BRIDCT_H>::RB; }
 #else
 int BRIDCT_CAT(merged_strip_cols_h, BRIDCT_H)() { return 0; }
 int BRIDCT_CAT(merged_block_rows_w, BRIDCT_H)() { return 0; }

@@ -7,24 +7,6 @@
 
 namespace bridct {
 
-// Tile-class batches of at most this many floats (16 MiB) take the small-batch tiles where
-// small_batch_tiles says so.
-constexpr long long kSmallBatchFloats = 4LL << 20;
-
-// Shapes and modes whose 16 MiB batches measured faster with tiles of half the 8192-float target
-// (several CTAs per SM instead of one uneven wave of large tiles; 24 shapes A/B'd on one box):
-// 8x16 +17%, 16x16 +16%, 32x16 +9..12%, 16x64 +8..14%, 32x32 +8..10%, 16x32 +6..10%, 8x32 +4..10%,
-// 16x8 +5%, 64x8 +4..7%, and the inverse and round trip of 32x64 (+10..13%) and the round trip of
-// 8x64 (+9%).  Tiles of 64-point register lines (64x16, 64x32, 64x64: one thread per line, so a
-// 4096-float tile leaves most threads idle) and of 128-point lines measured 5..25% slower.  64x64
-// round trips instead take two arrays per 128-thread CTA (a thread for each register line): +11%;
-// forward equal, inverse 5% slower that way.
-__host__ __device__ constexpr bool small_batch_tiles(int h, int w, int mode) {
-  return (h == 8 && (w == 16 || w == 32)) || (h == 16 && w <= 64) || (h == 32 && (w == 16 || w == 32)) ||
-         (h == 64 && w == 8) || (h == 32 && w == 64 && mode != LM_FWD) || (h == 8 && w == 64 && mode == LM_RT) ||
-         (h == 64 && w == 64 && mode == LM_RT);
-}
-
 struct LaunchCtx {
   int sm_count;
 };
@@ -37,7 +19,7 @@ int kernel_setup(const void* kernel, int smem, int threads);   // bridct_api.cu
 
 // Blocks per SM for a kernel at a given dynamic shared-memory size (set up once per device).
 template <typename Kernel>
-static int kernel_blocks_per_sm(Kernel k, int smem, int threads = kThreads) {
+static int kernel_blocks_per_sm(Kernel k, int smem, int threads) {
   return kernel_setup(reinterpret_cast<const void*>(k), smem, threads);
 }
 
@@ -45,17 +27,9 @@ static int kernel_blocks_per_sm(Kernel k, int smem, int threads = kThreads) {
 // CTAs may be scheduled, and run up to their first global access, while the previous kernel in
 // the stream finishes, which hides most of the launch gap between back-to-back launches (the two
 // passes of a two-pass shape, or consecutive calls).
-// With pdl = false it is an ordinary launch (the kernels' griddepcontrol instructions are then
-// no-ops).  Measured on 128 MiB batches of every shape (two A/B runs on one box): +1..5% on every
-// single-kernel shape, but 6..10% slower on most two-pass shapes with full-grid passes (the passes
-// of the few-array geometry keep it: one 1024 x 1024 array 529 -> 577 GB/s).
 template <typename... Params, typename... Args>
 static cudaError_t launch_pdl(void (*k)(Params...), unsigned grid, unsigned threads, int smem, cudaStream_t st,
-                              bool pdl, Args... args) {
-  if (!pdl) {
-    k<<<grid, threads, smem, st>>>(args...);
-    return cudaGetLastError();
-  }
+                              Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -69,25 +43,15 @@ static cudaError_t launch_pdl(void (*k)(Params...), unsigned grid, unsigned thre
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
-template <typename Kernel>
-static cudaError_t launch_tiles(Kernel k, int smem, int bps, TileArgs a, const LaunchCtx& ctx,
-                                cudaStream_t st, int threads = kThreads, bool pdl = true) {
-  if (bps <= 0) return cudaErrorInvalidConfiguration;
-  if (a.ntiles <= 0) return cudaSuccess;
-  long long grid = (long long)ctx.sm_count * bps;
-  if (grid > a.ntiles) grid = a.ntiles;
-  return launch_pdl(k, (unsigned)grid, (unsigned)threads, smem, st, pdl, a);
-}
-
-// One CTA per strip or row block of a pass of split lines.  Always with programmatic dependent launch:
-// the table copy overlaps the previous kernel's end (+1% on 128 MiB batches, +0..4% on 16 MiB ones,
+// One CTA per strip or row block of a pass of split lines.  The table copy overlaps the previous
+// kernel's end (programmatic dependent launch: +1% on 128 MiB batches, +0..4% on 16 MiB ones,
 // -4% on 16 MiB of 512-point columns).
 template <typename Kernel>
 static cudaError_t launch_split(Kernel k, int smem, int threads, long long units, const SplitArgs& a, cudaStream_t st) {
   if (kernel_blocks_per_sm(k, smem, threads) <= 0) return cudaErrorInvalidConfiguration;
   if (units <= 0) return cudaSuccess;
   if (units > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
-  return launch_pdl(k, (unsigned)units, (unsigned)threads, smem, st, true, a);
+  return launch_pdl(k, (unsigned)units, (unsigned)threads, smem, st, a);
 }
 
 // Narrow units (strips of 8 columns, blocks of 8 rows) take about half the time of a wide one, so they
@@ -122,13 +86,85 @@ cudaError_t launch_split_rows(float* y, long long batch, const BatchLayout& ly, 
   return launch_split(k_split_rows<W, GEN ? H : 0, MODE, 8>, Wide::kSmem, Wide::T, batch * H / Wide::RB, a, st);
 }
 
-// Route of an (H, W, MODE) batch: whole 32768-float arrays as single tiles in the modes where that
-// measured faster than two passes; other shapes above 16384 floats take the two passes.
-__host__ __device__ constexpr bool whole_array_route(int H, int W, int MODE) {
-  return H * W == 32768 && (MODE == LM_INV || H == 1024 || H == 64 || (H == 32 && MODE == LM_FWD));
+// Arrays and threads per CTA and resident CTAs of the whole-array tiles (k_pair_tile), the fastest of
+// 3 to 8 combinations measured per shape on 128 MiB batches.  Shapes up to 64 x 64 run one warp per
+// CTA with a line pair per thread: 12 to 32 independent warps per SM overlap one another's loads,
+// transforms and stores, where 128-thread CTAs of the same tiles measured 5..30% slower.  Shapes with a
+// longer axis take the smallest tile that gives every thread a task of both stages, at the register
+// limit that keeps 12 or more warps per SM.
+struct TileCfg {
+  int arrays, threads, blocks;
+};
+__host__ __device__ constexpr TileCfg tile_cfg(int h, int w) {
+  const int m = cmax(h, w);
+  if (m <= 64) return {64 * m / (h * w), 32, m == 64 ? 12 : m == 32 ? 20 : 24};
+  if (m == 128) {
+    if (h <= 16) return {2048 / (h * w), 64, 16};
+    if (w == 8) return {4, 64, 10};
+    if (w == 16) return {2, 128, 8};
+    if (h == 32 || w == 32) return {1, 64, 10};
+    return {1, 64, 6};
+  }
+  if (m == 256) {
+    if (h <= 16) return {4096 / (h * w), 64, 10};
+    if (h == 64 || w == 64) return {1, 128, 3};
+    return {h == 32 ? 1 : 32 / w, 128, 5};
+  }
+  if (m == 512) {
+    if (h <= 16) return {8192 / (h * w), 128, 5};
+    if (h == 32) return {1, 128, 3};
+    if (w == 8) return {1, 64, 8};
+    return {1, w == 32 ? 256 : 128, w == 32 ? 2 : 4};
+  }
+  return {w == 1024 ? 16 / h : 1, 128, 3};
 }
-__host__ __device__ constexpr bool two_pass_route(int H, int W, int MODE) {
-  return H * W > 16384 && !whole_array_route(H, W, MODE);
+// The same for batches that do not fill the GPU: half as many arrays per tile, or twice the threads
+// (16 MiB batches +8% on average over the shapes, up to +27%; 128 MiB batches 5..30% slower).
+__host__ __device__ constexpr TileCfg tile_cfg_few(int h, int w) {
+  const TileCfg c = tile_cfg(h, w);
+  const int m = cmax(h, w);
+  if (m <= 16) return {h * w == 256 ? 4 : 8, 64, 12};
+  if (m <= 64) return c.arrays > 1 ? TileCfg{c.arrays / 2, 32, c.blocks} : TileCfg{1, 64, 6};
+  if (m == 128) {
+    if (h <= 16 || w == 16) return c;
+    if (h == 32) return {1, 128, 7};
+    return {c.arrays, 128, w == 8 || w == 32 ? 5 : 3};
+  }
+  if (m == 256) {
+    if (w == 8) return c;
+    if (w == 16) return {1, 128, 5};
+    return {c.arrays, c.threads * 2, c.threads == 64 ? 5 : c.blocks == 3 ? 2 : 3};
+  }
+  if (m == 512) return h == 512 ? c : TileCfg{c.arrays, 256, c.blocks == 5 ? 3 : 2};
+  return c;
+}
+// Whether a batch that makes `tiles` full tiles takes the smaller ones: below one wave, unless the full
+// tiles fit in less than half of the GPU's slots and the smaller ones (twice the slots) do not: back to
+// back launches then overlap (programmatic dependent launch), which is worth more (+5..25% at 8 MiB).
+static inline bool few_tiles(long long tiles, TileCfg c, const LaunchCtx& ctx) {
+  const double waves = (double)tiles / ((double)c.blocks * ctx.sm_count);
+  return waves < 1 && (tiles <= ctx.sm_count || waves < 0.225 || waves > 0.45);
+}
+// Whole arrays up to 16384 floats, except 128 x 128 (register lines of one thread each, below: +15..20%
+// over split lines there).
+__host__ __device__ constexpr bool pair_tile_route(int h, int w) {
+  return h * w <= 16384 && !(h == 128 && w == 128) && !(h == 8 && w == 8);
+}
+
+template <int SMEM, typename Kernel>
+static cudaError_t launch_pair_tile(Kernel k, TileCfg c, long long batch, TileArgs a, cudaStream_t st) {
+  if (kernel_blocks_per_sm(k, SMEM, c.threads) <= 0) return cudaErrorInvalidConfiguration;
+  a.ntiles = (batch + c.arrays - 1) / c.arrays;
+  if (a.ntiles > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+  return launch_pdl(k, (unsigned)a.ntiles, (unsigned)c.threads, SMEM, st, a);
+}
+
+// The classes of a ragged batch that the merged passes take (bridct_ragged_set_schedule): shapes above
+// 16384 floats, without the 32768-float arrays in the modes that ran as whole-array tiles before the
+// passes of split lines overtook them (the schedules a caller may set stay the same).
+__host__ __device__ constexpr bool merged_route(int H, int W, int MODE) {
+  const bool whole = H * W == 32768 && (MODE == LM_INV || H == 1024 || H == 64 || (H == 32 && MODE == LM_FWD));
+  return H * W > 16384 && !whole;
 }
 
 // GEN: the batch has general layouts (strided arrays or an offset table, BatchLayout); the same
@@ -138,7 +174,6 @@ template <int H, int W, int MODE, bool GEN>
 cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStream_t st,
                               LineTables tab, const LaunchCtx& ctx, const BatchLayout& lx,
                               const BatchLayout& ly) {
-  using Gm = Geometry<H, W>;
   if (batch <= 0) return cudaSuccess;
   if constexpr (H == 8 && W == 8 && !GEN) {
     // Measured on B200 (GB/s, device-resident, back-to-back launches): the double-buffered kernel
@@ -154,7 +189,7 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
       const long long ntiles = (batch + kB8dbThreads - 1) / kB8dbThreads;
       long long grid = (long long)ctx.sm_count * bps;
       if (grid > ntiles) grid = ntiles;
-      return launch_pdl(k, (unsigned)grid, kB8dbThreads, smem, st, true, x, y, batch);
+      return launch_pdl(k, (unsigned)grid, kB8dbThreads, smem, st, x, y, batch);
     }
     auto k = k_blocks8<MODE>;
     constexpr int smem = kB8Chunks * 16;
@@ -163,78 +198,44 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
     const long long ntiles = (batch + kB8Threads - 1) / kB8Threads;
     long long grid = (long long)ctx.sm_count * bps;
     if (grid > ntiles) grid = ntiles;
-    return launch_pdl(k, (unsigned)grid, kB8Threads, smem, st, true, x, y, batch);
-  } else if constexpr (Gm::kTile) {
-    // 16384-float tiles instead of 8192 where they measured faster on 128 MiB batches: 64-wide
-    // arrays up to 64 high (+6..14%, except the 64 x 64 inverse, -2%) and forward/inverse of
-    // 8..32 x 128 (+17..22%); narrower tiles, 64 x 128 and those round trips measured 5..21%
-    // slower with them (64 x 8 and 64 x 16, whose 8192-float tiles give half the threads a column
-    // line, 5-8% slower too).
-    constexpr bool kBig = (W == 64 && H <= 64 && !(H == 64 && MODE == LM_INV)) ||
-                          (W == 128 && H <= 32 && MODE != LM_RT);
-    // Forward / inverse tiles of 128-point register columns and 8..32 columns hold one CTA per SM
-    // (227+ registers), so their tiles are sized against one CTA's shared memory (kTRWide): twice
-    // the arrays, so that 128 instead of 64 threads have a column line (+18..26%); round trips
-    // (128-thread CTAs, two per SM) measured 18-20% slower that way, and so did 32768-float tiles
-    // of 8..32 x 128 (all rows busy, but no register prefetch at that size): -20%.
-    constexpr bool kWide = H == 128 && W <= 32 && MODE != LM_RT;
-    constexpr int TR = kWide ? Gm::kTRWide : kBig ? Gm::kTRBig : Gm::kTR;
-    // 128 x 128 tiles (both passes 128-point register lines, 255 registers) and round trips of
-    // tiles with a 128-point axis run 128-thread CTAs: two CTAs share an SM (128 x 128 +31..64%
-    // over one 256-thread CTA with register prefetch, in which half the warps have no line; the
-    // round trips +3..30% together with their register lines).  Forward / inverse tiles that mix
-    // 128-point register lines with many short lines measured 5..13% slower that way.
-    constexpr int T = (H == 128 && W == 128) || (MODE == LM_RT && (H == 128 || W == 128)) ? 128 : kThreads;
-    // Shared memory as the kernel uses it (no exchange buffer for register lines), except the
-    // 128 x 128 round trip, which measured 2-3% faster at two CTAs per SM than at three.
-    constexpr int smem = H == 128 && W == 128 && MODE == LM_RT ? Gm::kSmemFull : Gm::template tile_smem<MODE, T>(TR / H);
-    if constexpr (Gm::kTRSmall < TR && small_batch_tiles(H, W, MODE)) {
-      if (batch * H * W <= kSmallBatchFloats) {
-        constexpr bool k64 = H == 64 && W == 64;   // two arrays, 128 threads (see small_batch_tiles)
-        constexpr int TS = k64 ? 128 : T;
-        constexpr int TRS = k64 ? Gm::kTR : Gm::kTRSmall;
-        constexpr int SMS = Gm::template tile_smem<MODE, TS>(TRS / H);
-        auto ks = k_full<H, W, TRS, true, true, MODE, TS, GEN>;
-        TileArgs a{x, y, (batch * H + TRS - 1) / TRS, batch * H, tab, lx, ly};
-        return launch_tiles(ks, SMS, kernel_blocks_per_sm(ks, SMS, TS), a, ctx, st, TS);
-      }
-    }
-    auto k = k_full<H, W, TR, true, true, MODE, T, GEN>;
+    return launch_pdl(k, (unsigned)grid, kB8Threads, smem, st, x, y, batch);
+  } else if constexpr (pair_tile_route(H, W)) {
+    constexpr TileCfg c = tile_cfg(H, W), f = tile_cfg_few(H, W);
+    constexpr bool has_few = f.arrays != c.arrays || f.threads != c.threads;
+    const TileArgs a{x, y, 0, batch * H, tab, lx, ly};
+    if (has_few && few_tiles((batch + c.arrays - 1) / c.arrays, c, ctx))
+      return launch_pair_tile<PairTileGeo<H, W, f.arrays>::kSmem>(
+          k_pair_tile<H, W, f.arrays, MODE, f.threads, f.blocks, GEN>, f, batch, a, st);
+    return launch_pair_tile<PairTileGeo<H, W, c.arrays>::kSmem>(
+        k_pair_tile<H, W, c.arrays, MODE, c.threads, c.blocks, GEN>, c, batch, a, st);
+  } else if constexpr (H * W <= 16384) {
+    // Register tiles, persistent CTAs.  The 128 x 128 round trip is given shared memory for two CTAs per
+    // SM only, which measured 2-3% faster than three.
+    constexpr int ARR = H == 8 ? 128 : 1, T = H == 8 ? 256 : 128;
+    constexpr int smem = H == 128 && MODE == LM_RT ? 110 * 1024 : RegTileGeo<H, W, ARR>::kSmem;
+    auto k = k_reg_tile<H, W, ARR, MODE, T, GEN>;
     const int bps = kernel_blocks_per_sm(k, smem, T);
-    TileArgs a{x, y, (batch * H + TR - 1) / TR, batch * H, tab, lx, ly};
-    return launch_tiles(k, smem, bps, a, ctx, st, T);
-  } else if constexpr (whole_array_route(H, W, MODE)) {
-    // Whole 32768-float arrays as tiles (one CTA per SM, both passes in shared memory) instead of
-    // the two passes, where that measured faster: every inverse (+5..21%), forward of 1024 x 32,
-    // 32 x 1024 and 64 x 512 (+2..14%), round trips of 1024 x 32 and 64 x 512 (+2..6%); round
-    // trips of 128 x 256 and 256 x 128 measured 30% slower.
-    auto k = k_full<H, W, H, true, true, MODE, kThreads, GEN>;
-    const int bps = kernel_blocks_per_sm(k, Gm::kSmemWhole);
-    TileArgs a{x, y, batch, batch * H, tab, lx, ly};
-    return launch_tiles(k, Gm::kSmemWhole, bps, a, ctx, st);
+    if (bps <= 0) return cudaErrorInvalidConfiguration;
+    const long long tiles = (batch + ARR - 1) / ARR, slots = (long long)ctx.sm_count * bps;
+    return launch_pdl(k, (unsigned)(tiles < slots ? tiles : slots), T, smem, st,
+                      TileArgs{x, y, tiles, batch * H, tab, lx, ly});
   } else {
-    // One column launch and one row launch over the whole batch.  Lines of 128 points and more run as
-    // split lines; shorter columns (32 x 1024 round trips, 64 x 1024) and 64-point rows as register
-    // lines.
+    // One column launch and one row launch over the whole batch.
     cudaError_t e;
     if constexpr (H >= 128) {
       e = launch_split_cols<H, W, MODE, GEN>(x, y, batch, lx, ly, tab.scol, ctx, st);
     } else {
-      auto kc = k_colstrip<H, W, Gm::kTC, MODE, kThreads, GEN>;
-      constexpr int smem = Gm::strip_smem(Gm::kTC);
-      const bool few = batch * (W / Gm::kTC) < 2LL * ctx.sm_count;   // below a full grid: PDL
-      TileArgs ac{x, y, batch * (W / Gm::kTC), batch * H, tab, lx, ly};
-      e = launch_tiles(kc, smem, kernel_blocks_per_sm(kc, smem), ac, ctx, st, kThreads, few);
+      using Geo = PairColGeo<H>;
+      e = launch_split(k_pair_cols<H, MODE, GEN>, 0, Geo::T, batch * (W / Geo::TC), SplitArgs{x, y, {}, W, lx, ly, nullptr},
+                       st);
     }
     if (e != cudaSuccess) return e;
     if constexpr (W >= 128) {
       return launch_split_rows<H, W, MODE, GEN>(y, batch, ly, tab.srow, ctx, st);
     } else {
-      auto kr = k_full<H, W, Gm::kRB, false, true, MODE, kThreads, GEN>;
-      constexpr int smem = Gm::rows_smem(Gm::kRB);
-      const bool few = batch * H / Gm::kRB < 2LL * ctx.sm_count;
-      TileArgs ar{y, y, batch * H / Gm::kRB, batch * H, tab, ly, ly};
-      return launch_tiles(kr, smem, kernel_blocks_per_sm(kr, smem), ar, ctx, st, kThreads, few);
+      using Geo = PairRowGeo<W>;
+      return launch_split(k_pair_rows<W, GEN ? H : 0, MODE>, Geo::kSmem, Geo::T, batch * H / Geo::RB,
+                          SplitArgs{y, y, {}, W, ly, ly, nullptr}, st);
     }
   }
 }
@@ -262,11 +263,9 @@ cudaError_t launch_col_units(const float* x, float* y, const PassUnit* units, lo
     return launch_split(k_split_cols<H, 0, MODE, col_pairs<H>()>, Geo::kSmem, Geo::T, n,
                         SplitArgs{x, y, tab.scol, 0, BatchLayout{}, BatchLayout{}, units}, st);
   } else {
-    using Gm = Geometry<H, 1024>;
-    auto k = k_colstrip<H, 1024, Gm::kTC, MODE, kThreads, false, true>;
-    constexpr int smem = Gm::strip_smem(Gm::kTC);
-    TileArgs a{x, y, n, n * H, tab, BatchLayout{}, BatchLayout{}, units};
-    return launch_tiles(k, smem, kernel_blocks_per_sm(k, smem), a, ctx, st, kThreads, false);
+    using Geo = PairColGeo<H>;
+    return launch_split(k_pair_cols<H, MODE, true>, 0, Geo::T, n,
+                        SplitArgs{x, y, {}, 0, BatchLayout{}, BatchLayout{}, units}, st);
   }
 }
 
@@ -278,11 +277,9 @@ cudaError_t launch_row_units(const float* x, float* y, const PassUnit* units, lo
     return launch_split(k_split_rows<W, W, MODE, 8>, Geo::kSmem, Geo::T, n,
                         SplitArgs{x, y, tab.srow, 0, BatchLayout{}, BatchLayout{}, units}, st);
   } else {
-    using Gm = Geometry<1024, W>;
-    auto k = k_full<1024, W, Gm::kRB, false, true, MODE, kThreads, false, true>;
-    constexpr int smem = Gm::rows_smem(Gm::kRB);
-    TileArgs a{x, y, n, n * Gm::kRB, tab, BatchLayout{}, BatchLayout{}, units};
-    return launch_tiles(k, smem, kernel_blocks_per_sm(k, smem), a, ctx, st, kThreads, false);
+    using Geo = PairRowGeo<W>;
+    return launch_split(k_pair_rows<W, W, MODE>, Geo::kSmem, Geo::T, n,
+                        SplitArgs{x, y, {}, 0, BatchLayout{}, BatchLayout{}, units}, st);
   }
 }
 

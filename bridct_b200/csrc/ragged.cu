@@ -459,7 +459,7 @@ BRIDCT_API size_t bridct_ragged_launch_count(const bridct_ragged* r) {
   size_t n = r->merged.size() + (r->units.empty() ? 0 : 1);
   for (const RaggedClass& c : r->classes)
     if (c.schedule == BRIDCT_RAGGED_CLASS_LAUNCH || c.schedule == BRIDCT_RAGGED_CLASS_LAUNCH_SMALL)
-      n += c.h * c.w <= 16384 || whole_array_route(c.h, c.w, c.mode) ? 1 : 2;
+      n += c.h * c.w <= 16384 ? 1 : 2;
   return n;
 }
 
@@ -484,7 +484,7 @@ BRIDCT_API int bridct_ragged_set_schedule(bridct_ragged* r, const int* schedules
       return BRIDCT_INVALID_ARGUMENT;
     }
     const RaggedClass& c = r->classes[i];
-    if (schedules[i] == BRIDCT_RAGGED_MERGED && !two_pass_route(c.h, c.w, c.mode)) {
+    if (schedules[i] == BRIDCT_RAGGED_MERGED && !merged_route(c.h, c.w, c.mode)) {
       set_error("bridct_ragged_set_schedule: class " + std::to_string(i) + " is not a two-pass shape");
       return BRIDCT_INVALID_ARGUMENT;
     }

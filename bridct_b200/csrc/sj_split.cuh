@@ -240,16 +240,15 @@ __device__ __forceinline__ int split_src(int a, int b) {
 // ---- the lines of a tile in shared memory ---------------------------------------------------------
 // GROUPS groups of LP line pairs, T threads: thread t holds pair t % LP and tasks t / LP, ... (group
 // major) of either stage.  get(g, i) is element i of the thread's pair of group g, put(g, i, v) takes
-// the result, ex(g) the thread's first exchange slot: slot (c, part, b) lies c * CS + (part * B + b) * LP
-// further on.  The exchange may overlie what get() reads: a barrier lies between.  IN_PLACE: put()
+// the result, ex(g) is the thread's place in the first of the group's N exchange slots, which lie ES
+// floats apart.  The exchange may overlie what get() reads: a barrier lies between.  IN_PLACE: put()
 // may also overlie the exchange.
-template <int N, int LP> __host__ __device__ constexpr int split_cs() {
-  // a half-warp spans 16 / LP tasks c: padding keeps their slots in different banks
-  return 2 * Split<N>::B * LP + (LP < 16 ? LP : 0);
-}
-template <int N, int MODE, int T, int GROUPS, int LP, bool IN_PLACE, typename Get, typename Put, typename Ex>
+// Slot (c, part, b) is number c * 2B + part * B + (b ^ (c % S)), S = 16 / LP: where a half-warp spans
+// several tasks c, their slots of one b then lie in different banks.
+template <int N, int MODE, int T, int GROUPS, int LP, int ES, bool IN_PLACE, typename Get, typename Put, typename Ex>
 __device__ __forceinline__ void split_lines(const Get& get, const Put& put, const Ex& ex, const float* tab) {
-  constexpr int A = Split<N>::A, B = Split<N>::B, CS = split_cs<N, LP>();
+  constexpr int A = Split<N>::A, B = Split<N>::B, S = LP < 16 ? 16 / LP : 1;
+  auto at = [](float* e) -> F2& { return *reinterpret_cast<F2*>(e); };
   constexpr int N1 = GROUPS * B * LP, N2 = GROUPS * (A / 2) * LP;   // threads' tasks of the two stages
   constexpr int R1 = (N1 + T - 1) / T, R2 = (N2 + T - 1) / T;
   static_assert(N1 % 32 == 0 && N2 % 32 == 0, "whole warps");
@@ -274,8 +273,10 @@ __device__ __forceinline__ void split_lines(const Get& get, const Put& put, cons
     for (int r = 0; r < R1; ++r) {
       const int i = t + r * TP, g = i / B, b = i % B;
       if (on1(r)) {
-        F2* e = ex(g) + b * LP;
-        split_put<N>(w[r], b, tab, [&](int c, int part, F2 val) { e[c * CS + part * B * LP] = val; });
+        float* e = ex(g);
+        split_put<N>(w[r], b, tab, [&](int c, int part, F2 val) {
+          at(e + (b ^ (c % S)) * ES + (c * 2 + part) * (B * ES)) = val;
+        });
       }
     }
     __syncthreads();
@@ -285,19 +286,21 @@ __device__ __forceinline__ void split_lines(const Get& get, const Put& put, cons
       const int i = t + r * TP, g = i / (A / 2), c = i % (A / 2);
       F2(&zr)[2 * B] = z[IN_PLACE && MODE == LM_FWD ? r : 0];
       if (on2(r)) {
-        F2* e = ex(g) + c * CS;
+        float* e = ex(g) + c * (2 * B * ES);
 #pragma unroll
         for (int q = 0; q < B; ++q) {
-          zr[2 * q] = e[q * LP];
-          zr[2 * q + 1] = e[(B + q) * LP];
+          float* eq = e + ((q % S) ^ (c % S)) * ES + (q - q % S) * ES;
+          zr[2 * q] = at(eq);
+          zr[2 * q + 1] = at(eq + B * ES);
         }
         split_stage2<N>(zr, c, tab);
         if constexpr (MODE == LM_RT) {
           split_stage2_t<N>(zr, c, tab);
 #pragma unroll
           for (int q = 0; q < B; ++q) {
-            e[q * LP] = zr[2 * q];
-            e[(B + q) * LP] = zr[2 * q + 1];
+            float* eq = e + ((q % S) ^ (c % S)) * ES + (q - q % S) * ES;
+            at(eq) = zr[2 * q];
+            at(eq + B * ES) = zr[2 * q + 1];
           }
         } else if constexpr (!IN_PLACE) {
           split_outputs<N>(c, [&](int j, int k) { put(g, k, zr[j]); });
@@ -327,11 +330,12 @@ __device__ __forceinline__ void split_lines(const Get& get, const Put& put, cons
     for (int r = 0; r < R2; ++r) {
       const int i = t + r * TP, g = i / (A / 2), c = i % (A / 2);
       if (on2(r)) {
-        F2* e = ex(g) + c * CS;
+        float* e = ex(g) + c * (2 * B * ES);
 #pragma unroll
         for (int q = 0; q < B; ++q) {
-          e[q * LP] = z[r][2 * q];
-          e[(B + q) * LP] = z[r][2 * q + 1];
+          float* eq = e + ((q % S) ^ (c % S)) * ES + (q - q % S) * ES;
+          at(eq) = z[r][2 * q];
+          at(eq + B * ES) = z[r][2 * q + 1];
         }
       }
     }
@@ -344,9 +348,11 @@ __device__ __forceinline__ void split_lines(const Get& get, const Put& put, cons
       const int i = t + r * TP, g = i / B, b = i % B;
       F2(&vr)[A] = v[IN_PLACE ? r : 0];
       if (on1(r)) {
-        const F2* e = ex(g) + b * LP;
+        float* e = ex(g);
         F2 w[A];
-        split_get<N>(w, b, tab, [&](int c, int part) { return e[c * CS + part * B * LP]; });
+        split_get<N>(w, b, tab, [&](int c, int part) {
+          return at(e + (b ^ (c % S)) * ES + (c * 2 + part) * (B * ES));
+        });
         Leaf<A>::tr(w, vr);
         if constexpr (!IN_PLACE) {
 #pragma unroll
@@ -389,8 +395,8 @@ constexpr int kFewPairs = 4;
 template <int N, int LP = col_pairs<N>()> struct ColGeo {
   static constexpr int TC = 2 * LP;
   static constexpr int T = 128;
-  static constexpr int kExch = Split<N>::A / 2 * split_cs<N, LP>() * 2;   // floats; covers the N x TC strip
-  static constexpr int kSmem = (kExch + SplitTab<N>::kFloats) * 4;
+  static constexpr int kTile = N * TC;   // the strip, then the exchange
+  static constexpr int kSmem = (kTile + SplitTab<N>::kFloats) * 4;
 };
 template <int TC>
 __device__ __forceinline__ int strip_row(int r) {
@@ -412,7 +418,7 @@ __device__ __forceinline__ void split_col_unit(const float* x, float* y, long lo
   __syncthreads();
   const int p = 2 * (threadIdx.x % LP);
   float* yt = y + p;
-  split_lines<N, MODE, T, 1, LP, false>(
+  split_lines<N, MODE, T, 1, LP, TC, false>(
       [&](int, int i) {
         const float2 v = *reinterpret_cast<const float2*>(smem + strip_row<TC>(i) + p);
         return f2_make(v.x, v.y);
@@ -422,7 +428,7 @@ __device__ __forceinline__ void split_col_unit(const float* x, float* y, long lo
         f2_split(v, f.x, f.y);
         *reinterpret_cast<float2*>(yt + (W > 0 ? (long long)(i * W) : i * yp)) = f;
       },
-      [&](int) { return reinterpret_cast<F2*>(smem) + p / 2; }, tab);
+      [&](int) { return smem + p; }, tab);
 }
 
 // W > 0: strips of contiguous N x W arrays; W = 0: run-time layouts, or units.
@@ -431,7 +437,7 @@ __global__ void __launch_bounds__(128) k_split_cols(SplitArgs a) {
   using Geo = ColGeo<N, LP>;
   constexpr int TC = Geo::TC;
   extern __shared__ float smem[];
-  float* tab = smem + Geo::kExch;
+  float* tab = smem + Geo::kTile;
   split_stage_tables<N, Geo::T>(a.tab, tab);
   griddep_wait();
   griddep_trigger();
@@ -459,22 +465,20 @@ template <int N, int LP = 8, int GROUPS = LP == 8 ? row_groups<N>() : 1> struct 
   static constexpr int P = N + 32 / LP;
   static constexpr int T = 128;
   static constexpr int RB = 2 * LP * GROUPS;
-  static constexpr int kExch = Split<N>::A / 2 * split_cs<N, LP>() * 2;
-  static constexpr int GP = 2 * LP * P > kExch ? 2 * LP * P : kExch;   // floats of one group
-  static constexpr int kTile = GROUPS * GP;
+  static constexpr int kTile = RB * P;
   static constexpr int kSmem = (kTile + SplitTab<N>::kFloats) * 4;
 };
 
-// All rows of a tile of GROUPS groups, GP floats apart.
-template <int N, int MODE, int T, int GROUPS, int LP, int GP>
+// All rows of a tile of GROUPS groups of 2 LP rows at pitch P.
+template <int N, int MODE, int T, int GROUPS, int LP>
 __device__ __forceinline__ void split_rows(float* tile, const float* tab) {
-  constexpr int P = N + 32 / LP;
+  constexpr int P = N + 32 / LP, GP = 2 * LP * P;
   const int p = threadIdx.x % LP;
   float* rows = tile + p * P;
-  split_lines<N, MODE, T, GROUPS, LP, true>(
+  split_lines<N, MODE, T, GROUPS, LP, 2 * LP, true>(
       [&](int g, int i) { return f2_make(rows[g * GP + i], rows[g * GP + i + LP * P]); },
       [&](int g, int i, F2 v) { f2_split(v, rows[g * GP + i], rows[g * GP + i + LP * P]); },
-      [&](int g) { return reinterpret_cast<F2*>(tile + g * GP) + p; }, tab);
+      [&](int g) { return tile + g * GP + 2 * p; }, tab);
 }
 
 // Stores `bytes` (a multiple of 16) of shared memory to global memory asynchronously.
@@ -494,7 +498,7 @@ template <int N, int MODE, int LP, typename XRow, typename YRow>
 __device__ __forceinline__ void split_row_unit(const XRow& xrow, const YRow& yrow, float* smem, const float* tab) {
   using Geo = RowGeo<N, LP>;
   constexpr int P = Geo::P, RB = Geo::RB, T = Geo::T, Q = N / 4;
-  auto srow = [&](int r) { return smem + (r / (2 * LP)) * Geo::GP + (r % (2 * LP)) * P; };
+  auto srow = [&](int r) { return smem + r * P; };
 #pragma unroll
   for (int k = 0; k < RB * Q / T; ++k) {
     const int i = threadIdx.x + k * T, r = i / Q, c = (i % Q) * 4;
@@ -502,7 +506,7 @@ __device__ __forceinline__ void split_row_unit(const XRow& xrow, const YRow& yro
   }
   cp_async_wait_all();
   __syncthreads();
-  split_rows<N, MODE, T, Geo::RB / (2 * LP), LP, Geo::GP>(smem, tab);
+  split_rows<N, MODE, T, Geo::RB / (2 * LP), LP>(smem, tab);
   fence_async();
   __syncthreads();
   if (threadIdx.x < RB) {
@@ -532,6 +536,212 @@ __global__ void __launch_bounds__(128) k_split_rows(SplitArgs a) {
   } else {
     split_row_unit<N, MODE, LP>([&](int r) { return a.x + layout_row<H>(a.lx, first + r); },
                                 [&](int r) { return a.y + layout_row<H>(a.ly, first + r); }, smem, tab);
+  }
+}
+
+// ---- lines of 64 points and fewer: two per thread in registers -----------------------------------
+template <int N, int MODE>
+__device__ __forceinline__ void pair_line(F2 (&v)[N]) {
+  static_assert(N <= 64, "register lines");
+  if constexpr (N == 8) MODE == LM_FWD ? sjp_fwd_8<F2>(v) : MODE == LM_INV ? sjp_inv_8<F2>(v) : sjp_rt_8<F2>(v);
+  if constexpr (N == 16) MODE == LM_FWD ? sjp_fwd_16<F2>(v) : MODE == LM_INV ? sjp_inv_16<F2>(v) : sjp_rt_16<F2>(v);
+  if constexpr (N == 32) MODE == LM_FWD ? sjp_fwd_32<F2>(v) : MODE == LM_INV ? sjp_inv_32<F2>(v) : sjp_rt_32<F2>(v);
+  if constexpr (N == 64) MODE == LM_FWD ? sjp_fwd_64<F2>(v) : MODE == LM_INV ? sjp_inv_64<F2>(v) : sjp_rt_64<F2>(v);
+}
+// Two rows in shared memory, in place: 128-bit accesses (8 consecutive rows at a pitch of 4 mod 32
+// floats are 4 banks apart).
+template <int N, int MODE>
+__device__ __forceinline__ void pair_rows(float* r0, float* r1) {
+  F2 v[N];
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const float4 p = *reinterpret_cast<const float4*>(r0 + i), q = *reinterpret_cast<const float4*>(r1 + i);
+    v[i] = f2_make(p.x, q.x);
+    v[i + 1] = f2_make(p.y, q.y);
+    v[i + 2] = f2_make(p.z, q.z);
+    v[i + 3] = f2_make(p.w, q.w);
+  }
+  pair_line<N, MODE>(v);
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    float4 p, q;
+    f2_split(v[i], p.x, q.x);
+    f2_split(v[i + 1], p.y, q.y);
+    f2_split(v[i + 2], p.z, q.z);
+    f2_split(v[i + 3], p.w, q.w);
+    *reinterpret_cast<float4*>(r0 + i) = p;
+    *reinterpret_cast<float4*>(r1 + i) = q;
+  }
+}
+
+// Column pass of 32- and 64-point columns: a thread holds two adjacent columns, straight from and to
+// global memory (a warp's row segment is 256 bytes).
+template <int N> struct PairColGeo {
+  static constexpr int T = 32;
+  static constexpr int TC = 2 * T;
+};
+template <int N, int MODE, bool GEN>
+__global__ void __launch_bounds__(32) k_pair_cols(SplitArgs a) {
+  constexpr int TC = PairColGeo<N>::TC;
+  griddep_wait();
+  griddep_trigger();
+  const float* x;
+  float* y;
+  long long xp = a.width, yp = a.width;
+  if (GEN && a.units) {
+    const PassUnit u = a.units[blockIdx.x];
+    x = a.x + u.off;
+    y = a.y + u.off;
+    xp = yp = u.ld;
+  } else {
+    const unsigned S = a.width / TC, arr = blockIdx.x / S, s = blockIdx.x % S;
+    if (GEN) {
+      x = a.x + layout_row<N>(a.lx, (long long)arr * N) + s * TC;
+      y = a.y + layout_row<N>(a.ly, (long long)arr * N) + s * TC;
+      xp = a.lx.ld;
+      yp = a.ly.ld;
+    } else {
+      const long long off = (long long)arr * N * a.width + s * TC;
+      x = a.x + off;
+      y = a.y + off;
+    }
+  }
+  x += 2 * threadIdx.x;
+  y += 2 * threadIdx.x;
+  F2 v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float2 f = __ldg(reinterpret_cast<const float2*>(x + i * xp));
+    v[i] = f2_make(f.x, f.y);
+  }
+  pair_line<N, MODE>(v);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float2 f;
+    f2_split(v[i], f.x, f.y);
+    *reinterpret_cast<float2*>(y + i * yp) = f;
+  }
+}
+
+// Row pass of 32- and 64-point rows in place: 64 rows per warp, staged in shared memory.
+template <int N> struct PairRowGeo {
+  static constexpr int T = 32;
+  static constexpr int RB = 64;
+  static constexpr int P = N + 4;
+  static constexpr int kSmem = RB * P * 4;
+};
+template <int N, int H, int MODE>
+__global__ void __launch_bounds__(32) k_pair_rows(SplitArgs a) {
+  using Geo = PairRowGeo<N>;
+  constexpr int P = Geo::P, Q = N / 4;
+  extern __shared__ float smem[];
+  griddep_wait();
+  griddep_trigger();
+  const long long first = (long long)blockIdx.x * Geo::RB;
+  auto row = [&](int r) -> float* {
+    if (H == 0) return a.y + (first + r) * N;
+    if (a.units) return a.y + a.units[blockIdx.x].off + r * a.units[blockIdx.x].ld;
+    return a.y + layout_row<cmax(H, 1)>(a.ly, first + r);
+  };
+#pragma unroll 8
+  for (int i = threadIdx.x; i < Geo::RB * Q; i += 32) cp_async16(smem + i / Q * P + i % Q * 4, row(i / Q) + i % Q * 4);
+  cp_async_wait_all();
+  __syncwarp();
+  const int r = (threadIdx.x / 8) * 16 + threadIdx.x % 8;
+  pair_rows<N, MODE>(smem + r * P, smem + (r + 8) * P);
+  __syncwarp();
+#pragma unroll 8
+  for (int i = threadIdx.x; i < Geo::RB * Q; i += 32)
+    *reinterpret_cast<float4*>(row(i / Q) + i % Q * 4) = *reinterpret_cast<const float4*>(smem + i / Q * P + i % Q * 4);
+}
+
+// ---- whole arrays in one tile ------------------------------------------------------------------
+// ARR arrays of H x W in shared memory, row pitch W + 4 and arrays AP floats apart (8- and 16-column
+// arrays are padded so that the 4 or 2 arrays which a half-warp's 16 column pairs span lie in different
+// banks).  Columns: adjacent columns make a pair (64-bit accesses, a half-warp reads 128 contiguous
+// bytes); a split line's exchange slots are the rows of its own columns.  Rows: rows r and r + 8 of 16
+// make a pair.
+template <int H, int W, int ARR> struct PairTileGeo {
+  static constexpr int P = W + 4;
+  static constexpr int AP = W == 8 ? H * P + (40 - H * P % 32) % 32 : W == 16 ? H * P + (48 - H * P % 32) % 32 : H * P;
+  static constexpr int TR = ARR * H;
+  static constexpr int kTile = ARR * AP;
+  static constexpr int kTabC = H >= 128 ? SplitTab<cmax(H, 128)>::kFloats : 0;
+  static constexpr int kTabR = W >= 128 && W != H ? SplitTab<cmax(W, 128)>::kFloats : 0;
+  static constexpr int kSmem = (kTile + kTabC + kTabR) * 4;
+};
+
+template <int H, int W, int ARR, int MODE, int T, int MINB, bool GEN>
+__global__ void __launch_bounds__(T, MINB) k_pair_tile(TileArgs a) {
+  using Geo = PairTileGeo<H, W, ARR>;
+  constexpr int P = Geo::P, AP = Geo::AP, TR = Geo::TR;
+  extern __shared__ float smem[];
+  float* tcol = smem + Geo::kTile;
+  float* trow = H == W ? tcol : tcol + Geo::kTabC;
+  if constexpr (H >= 128) split_stage_tables<H, T>(a.tab.scol, tcol);
+  if constexpr (W >= 128 && W != H) split_stage_tables<W, T>(a.tab.srow, trow);
+  griddep_wait();
+  griddep_trigger();
+  const long long first = (long long)blockIdx.x * TR;
+  const int rows = a.rows_total - first < TR ? (int)(a.rows_total - first) : TR;
+  auto srow = [](int r) { return (r / H) * AP + (r % H) * P; };
+  constexpr int Q = W / 4;
+  // rows beyond the batch stay as they are: lines do not mix, and they are not stored
+#pragma unroll 8
+  for (int i = threadIdx.x; i < rows * Q; i += T) {
+    const int r = i / Q, c = (i % Q) * 4;
+    cp_async16(smem + srow(r) + c, GEN ? a.x + layout_row<H>(a.lx, first + r) + c : a.x + first * W + 4 * i);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  if constexpr (H >= 128) {
+    constexpr int LP = cmin(16, ARR * W / 2), G = ARR * W / (2 * LP);   // groups of LP column pairs
+    static_assert(G * 2 * LP == ARR * W, "whole groups");
+    const int p = threadIdx.x % LP;
+    auto base = [&](int g) {
+      const int c = (g * LP + p) * 2;
+      return smem + c / W * AP + c % W;
+    };
+    split_lines<H, MODE, T, G, LP, P, true>(
+        [&](int g, int i) {
+          const float2 v = *reinterpret_cast<const float2*>(base(g) + i * P);
+          return f2_make(v.x, v.y);
+        },
+        [&](int g, int i, F2 v) { *reinterpret_cast<F2*>(base(g) + i * P) = v; }, base, tcol);
+  } else {
+    for (int l = threadIdx.x; l < ARR * W / 2; l += T) {
+      float* c = smem + (l / (W / 2)) * AP + 2 * (l % (W / 2));
+      F2 v[H];
+#pragma unroll
+      for (int i = 0; i < H; ++i) v[i] = *reinterpret_cast<const F2*>(c + i * P);
+      pair_line<H, MODE>(v);
+#pragma unroll
+      for (int i = 0; i < H; ++i) *reinterpret_cast<F2*>(c + i * P) = v[i];
+    }
+  }
+  __syncthreads();
+  if constexpr (W >= 128) {
+    split_rows<W, MODE, T, TR / 16, 8>(smem, trow);
+  } else {
+    for (int l = threadIdx.x; l < TR / 2; l += T) {
+      const int r = (l / 8) * 16 + l % 8;
+      pair_rows<W, MODE>(smem + srow(r), smem + srow(r + 8));
+    }
+  }
+  if constexpr (W >= 128) {
+    fence_async();
+    __syncthreads();
+    for (int r = threadIdx.x; r < rows; r += T)
+      bulk_store(GEN ? a.y + layout_row<H>(a.ly, first + r) : a.y + (first + r) * W, smem + srow(r), W * 4);
+    bulk_commit_wait();
+  } else {
+    __syncthreads();
+#pragma unroll 8
+    for (int i = threadIdx.x; i < rows * Q; i += T) {
+      const int r = i / Q, c = (i % Q) * 4;
+      *reinterpret_cast<float4*>(GEN ? a.y + layout_row<H>(a.ly, first + r) + c : a.y + first * W + 4 * i) =
+          *reinterpret_cast<const float4*>(smem + srow(r) + c);
+    }
   }
 }
 

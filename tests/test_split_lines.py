@@ -1,4 +1,4 @@
-"""Split lines (csrc/sj_split.cuh): the generated packed programs on the CPU, and on the GPU the unit
+"""Line pairs (csrc/sj_split.cuh): the generated packed programs on the CPU, and on the GPU the
 geometries a batch size selects, at the sizes where one takes over from the other."""
 import sys
 from pathlib import Path
@@ -57,4 +57,36 @@ def test_unit_geometries_agree_bitwise_and_with_float64(shape, few, many):
         ref = O.fp64_apply(x, mode)
         # the suite's bound for float32 lines: 2e-6 of the larger of the input and output maxima
         err = np.abs(y.cpu().numpy() - ref).max() / max(np.abs(x).max(), np.abs(ref).max())
+        assert err <= 2e-6, (mode, err)
+
+
+# Whole-array tiles: one shape per configuration, a batch too small to fill the GPU (the smaller tiles)
+# and one of more than a wave of full tiles that ends in a partial one.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,many", [((8, 16), 30001), ((16, 8), 30001), ((16, 16), 15001), ((16, 32), 13001),
+                                        ((32, 32), 6501), ((64, 8), 15001), ((8, 64), 15001), ((64, 64), 1901),
+                                        ((8, 128), 5001), ((32, 128), 1601), ((64, 128), 901), ((128, 8), 6201),
+                                        ((128, 16), 2501), ((128, 32), 1601), ((8, 256), 3101), ((32, 256), 801),
+                                        ((64, 256), 451), ((256, 8), 3101), ((256, 16), 1601), ((256, 64), 451),
+                                        ((8, 512), 1601), ((32, 512), 451), ((512, 8), 1201), ((512, 32), 301),
+                                        ((8, 1024), 901), ((16, 1024), 451), ((1024, 8), 451), ((1024, 16), 451)])
+def test_tiles_agree_bitwise_and_with_float64(shape, many):
+    import torch
+
+    from bridct_b200 import torch_api
+    from oracle import oracle as O
+
+    h, w = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(h * 3 + w)
+    x = torch.randn((many, h, w), generator=g, device="cuda")
+    guard = torch.full((many + 1, h, w), 7.0, device="cuda")
+    for mode in range(3):
+        y = torch_api.apply(x, mode, out=guard[:many])
+        assert torch.equal(guard[many], torch.full_like(guard[many], 7.0)), mode
+        for n in (1, 3):
+            assert torch.equal(torch_api.apply(x[:n].contiguous(), mode), y[:n]), (mode, n)
+        tail = x[-5:].cpu().numpy()
+        ref = O.fp64_apply(tail, mode)
+        err = np.abs(y[-5:].cpu().numpy() - ref).max() / max(np.abs(tail).max(), np.abs(ref).max())
         assert err <= 2e-6, (mode, err)
