@@ -604,8 +604,8 @@ def generate() -> str:
 # ----------------------------------------------------------------------------------------
 
 PACKED_LINES = (8, 16, 32, 64)      # whole lines in registers
-PACKED_LEAVES = (16, 32)            # stage 1 of a split line: real FFT over the A samples of one residue
-PACKED_STAGE2 = (8, 16, 32)         # stage 2: complex FFT over the B residues of one column
+PACKED_LEAVES = (16, 32, 64)            # stage 1 of a split line: real FFT over the A samples of one residue
+PACKED_STAGE2 = (8, 16)             # stage 2: complex FFT over the B residues of one column
 
 
 def emit_packed(g: Graph, name: str, in_names: Sequence[str], outputs: Sequence[int],

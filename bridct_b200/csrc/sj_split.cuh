@@ -79,7 +79,9 @@ template <int N> struct Split;
 template <> struct Split<128> { static constexpr int A = 16, B = 8; };
 template <> struct Split<256> { static constexpr int A = 32, B = 8; };
 template <> struct Split<512> { static constexpr int A = 32, B = 16; };
-template <> struct Split<1024> { static constexpr int A = 32, B = 32; };
+// 64 * 16 rather than 32 * 32: the real columns' task, which one warp runs besides its own, is then
+// short (32 M elements of 1024-point columns 53.7 -> 49.9 us, rows 60.5 -> 58.2, round trips -5..8%).
+template <> struct Split<1024> { static constexpr int A = 64, B = 16; };
 
 template <int A> struct Leaf;
 template <> struct Leaf<16> {
@@ -89,6 +91,10 @@ template <> struct Leaf<16> {
 template <> struct Leaf<32> {
   static __device__ __forceinline__ void fwd(const F2 (&x)[32], F2 (&w)[32]) { sjp_rfft_32<F2>(x, w); }
   static __device__ __forceinline__ void tr(const F2 (&w)[32], F2 (&x)[32]) { sjp_rfft_32_t<F2>(w, x); }
+};
+template <> struct Leaf<64> {
+  static __device__ __forceinline__ void fwd(const F2 (&x)[64], F2 (&w)[64]) { sjp_rfft_64<F2>(x, w); }
+  static __device__ __forceinline__ void tr(const F2 (&w)[64], F2 (&x)[64]) { sjp_rfft_64_t<F2>(w, x); }
 };
 template <int B> struct Stage2;
 #define BRIDCT_STAGE2(B)                                                                       \
@@ -100,7 +106,6 @@ template <int B> struct Stage2;
   };
 BRIDCT_STAGE2(8)
 BRIDCT_STAGE2(16)
-BRIDCT_STAGE2(32)
 #undef BRIDCT_STAGE2
 
 // Rotations of one line length, A/2 * B of each kind:
@@ -395,6 +400,9 @@ constexpr int kFewPairs = 4;
 template <int N, int LP = col_pairs<N>()> struct ColGeo {
   static constexpr int TC = 2 * LP;
   static constexpr int T = 128;
+  // resident CTAs that the registers are limited for (32 M elements of 512-point columns: 45.6 us, 52.0
+  // unlimited; 1024: 49.9 and 60.2; 256-point round trips 51.7 and 61.8)
+  static constexpr int kBlocks = LP == kFewPairs ? 1 : N == 128 ? 8 : N == 256 ? 6 : N == 512 ? 5 : 3;
   static constexpr int kTile = N * TC;   // the strip, then the exchange
   static constexpr int kSmem = (kTile + SplitTab<N>::kFloats) * 4;
 };
@@ -433,7 +441,7 @@ __device__ __forceinline__ void split_col_unit(const float* x, float* y, long lo
 
 // W > 0: strips of contiguous N x W arrays; W = 0: run-time layouts, or units.
 template <int N, int W, int MODE, int LP>
-__global__ void __launch_bounds__(128) k_split_cols(SplitArgs a) {
+__global__ void __launch_bounds__(ColGeo<N, LP>::T, ColGeo<N, LP>::kBlocks) k_split_cols(SplitArgs a) {
   using Geo = ColGeo<N, LP>;
   constexpr int TC = Geo::TC;
   extern __shared__ float smem[];
@@ -460,11 +468,14 @@ __global__ void __launch_bounds__(128) k_split_cols(SplitArgs a) {
 // Rows are staged whole in shared memory in groups of 2 LP, at pitch N + 32 / LP floats: a thread holds
 // rows p and p + LP of a group, and a warp LP such pairs at 32 / LP adjacent b's (or c's), so the
 // scalar walks along the rows hit bank (32 / LP) p + b: conflict-free.
-template <int N> __host__ __device__ constexpr int row_groups() { return N <= 256 ? 2 : 1; }
-template <int N, int LP = 8, int GROUPS = LP == 8 ? row_groups<N>() : 1> struct RowGeo {
+// One group per CTA: 64 threads give 128- and 256-point lines a stage-1 task each, and ten to sixteen
+// such CTAs per SM hide one another's barriers and copies (32 M elements of 256-point rows: 49.7 us,
+// 53.7 as two groups in 128 threads, 63.1 without the register limit; 128: 48.8, 512: 52.0, 1024: 58.2).
+template <int N, int LP = 8> struct RowGeo {
   static constexpr int P = N + 32 / LP;
-  static constexpr int T = 128;
-  static constexpr int RB = 2 * LP * GROUPS;
+  static constexpr int T = LP == 8 && N <= 256 ? 64 : 128;
+  static constexpr int kBlocks = LP != 8 ? 1 : N == 128 ? 16 : N == 256 ? 10 : N == 512 ? 5 : 3;
+  static constexpr int RB = 2 * LP;
   static constexpr int kTile = RB * P;
   static constexpr int kSmem = (kTile + SplitTab<N>::kFloats) * 4;
 };
@@ -518,7 +529,7 @@ __device__ __forceinline__ void split_row_unit(const XRow& xrow, const YRow& yro
 // RB consecutive rows of a (batch * H) x N matrix per CTA.  H = 0: contiguous rows; H > 0: run-time
 // layouts of arrays of H rows, or units.
 template <int N, int H, int MODE, int LP>
-__global__ void __launch_bounds__(128) k_split_rows(SplitArgs a) {
+__global__ void __launch_bounds__(RowGeo<N, LP>::T, RowGeo<N, LP>::kBlocks) k_split_rows(SplitArgs a) {
   using Geo = RowGeo<N, LP>;
   extern __shared__ float smem[];
   float* tab = smem + Geo::kTile;
