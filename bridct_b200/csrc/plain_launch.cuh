@@ -136,7 +136,7 @@ __host__ __device__ constexpr TileCfg tile_cfg_few(int h, int w) {
     return {c.arrays, c.threads * 2, c.threads == 64 ? 5 : c.blocks == 3 ? 2 : 3};
   }
   if (m == 512) return h == 512 ? c : TileCfg{c.arrays, 256, c.blocks == 5 ? 3 : 2};
-  return c;
+  return h == 8 ? TileCfg{1, 128, 3} : c;
 }
 // Whether a batch that makes `tiles` full tiles takes the smaller ones: below one wave, unless the full
 // tiles fit in less than half of the GPU's slots and the smaller ones (twice the slots) do not: back to

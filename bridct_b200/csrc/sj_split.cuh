@@ -673,7 +673,8 @@ __global__ void __launch_bounds__(32) k_pair_rows(SplitArgs a) {
 // bytes); a split line's exchange slots are the rows of its own columns.  Rows: rows r and r + 8 of 16
 // make a pair.
 template <int H, int W, int ARR> struct PairTileGeo {
-  static constexpr int P = W + 4;
+  static constexpr int kRowPairs = ARR * H % 16 == 0 ? 8 : 4;   // split rows: pairs of a group
+  static constexpr int P = W >= 128 ? W + 32 / kRowPairs : W + 4;
   static constexpr int AP = W == 8 ? H * P + (40 - H * P % 32) % 32 : W == 16 ? H * P + (48 - H * P % 32) % 32 : H * P;
   static constexpr int TR = ARR * H;
   static constexpr int kTile = ARR * AP;
@@ -732,7 +733,7 @@ __global__ void __launch_bounds__(T, MINB) k_pair_tile(TileArgs a) {
   }
   __syncthreads();
   if constexpr (W >= 128) {
-    split_rows<W, MODE, T, TR / 16, 8>(smem, trow);
+    split_rows<W, MODE, T, TR / (2 * Geo::kRowPairs), Geo::kRowPairs>(smem, trow);
   } else {
     for (int l = threadIdx.x; l < TR / 2; l += T) {
       const int r = (l / 8) * 16 + l % 8;
