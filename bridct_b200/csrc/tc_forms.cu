@@ -142,23 +142,34 @@ std::vector<double> dct_matrix(int L) {
   return c;
 }
 
-// B image of the row pass for rows of length L: slice nb (64 output columns) at nb * kBBytes,
+// B image of the row pass for rows of length L: slice nb (64 columns of the N-block) at nb * kBBytes,
 // laid out [K-chunk][split][8 KB atom column]; B[n][k] = C_L[n][k] (forward) or C_L[k][n].  With
 // SUB > 1 the 64-float super-rows hold SUB rows of LS = 64 / SUB points, and B is block-diagonal:
-// SUB copies of C_LS (zeros elsewhere).
-template <int FORM, int L, int SUB = 1>
+// SUB copies of C_LS (zeros elsewhere).  Folded forward: row n of slice nb is coefficient
+// 2 (kNBlock (nb / 2) + n) + nb % 2, K runs over the first L / 2 samples.  Folded inverse: row n is sample
+// 64 nb + n, and within a K-chunk the even coefficients come first.
+template <int FORM, int L, int SUB, int FOLD>
 std::vector<uint8_t> pass_image(bool inverse) {
-  using PL = tc::PassLayout<FORM, L>;
+  using PL = tc::PassLayout<FORM, L, FOLD>;
   constexpr int kc_len = tc::PassForm<FORM>::kKC;
   constexpr int LS = L / SUB;
   const std::vector<double> c = dct_matrix(LS);
   std::vector<uint8_t> img((size_t)PL::kBlocks * PL::kBBytes, 0);
-  for (int n = 0; n < L; ++n)
-    for (int k = 0; k < L; ++k) {
-      if (n / LS != k / LS) continue;   // off the diagonal blocks: zero
-      const int nn = n % LS, kk0 = k % LS;
-      const double v = inverse ? c[(size_t)kk0 * LS + nn] : c[(size_t)nn * LS + kk0];
-      const int nb = n / 64, nl = n % 64, kc = k / kc_len, kk = k % kc_len;
+  constexpr int NB = PL::kNBlock;
+  for (int n = 0; n < PL::kBlocks * NB; ++n)
+    for (int k = 0; k < PL::kK; ++k) {
+      const int nb = n / NB, nl = n % NB, kc = k / kc_len, kk = k % kc_len;
+      double v;
+      if (FOLD == tc::FOLD_FWD) {
+        v = c[(size_t)(2 * (NB * (nb / 2) + nl) + nb % 2) * L + k];
+      } else if (FOLD == tc::FOLD_INV) {
+        const int coef = kc * kc_len + (kk < kc_len / 2 ? 2 * kk : 2 * (kk - kc_len / 2) + 1);
+        v = c[(size_t)coef * L + n];
+      } else {
+        if (n / LS != k / LS) continue;   // off the diagonal blocks: zero
+        const int nn = n % LS, kk0 = k % LS;
+        v = inverse ? c[(size_t)kk0 * LS + nn] : c[(size_t)nn * LS + kk0];
+      }
       uint8_t* slice = &img[(size_t)nb * PL::kBBytes];
       if (FORM == tc::BF16X3) {
         const float h = bf16_round(v);
@@ -169,7 +180,7 @@ std::vector<uint8_t> pass_image(bool inverse) {
         const uint32_t off = tc::sw128(nl, kk / 8) + (kk % 8) * 2;
         for (int sp = 0; sp < 3; ++sp) {
           const uint16_t bits = bf16_bits(parts[sp]);
-          memcpy(slice + (size_t)(kc * 3 + sp) * tc::kBAtom + off, &bits, 2);
+          memcpy(slice + (size_t)(kc * 3 + sp) * PL::kBPart + off, &bits, 2);
         }
       } else {
         const float h = tf32_round(v);
@@ -177,7 +188,7 @@ std::vector<uint8_t> pass_image(bool inverse) {
         const float parts[2] = {h, l};
         const uint32_t off = tc::sw128(nl, kk / 4) + (kk % 4) * 4;
         for (int sp = 0; sp < 2; ++sp)
-          memcpy(slice + (size_t)(kc * 2 + sp) * tc::kBAtom + off, &parts[sp], 4);
+          memcpy(slice + (size_t)(kc * 2 + sp) * PL::kBPart + off, &parts[sp], 4);
       }
     }
   return img;
@@ -286,13 +297,13 @@ bool make_rows_map(CUtensorMap* m, const float* ptr, size_t rows, int L) {
 
 constexpr int lg_points(int n) { return n <= 8 ? 0 : 1 + lg_points(n / 2); }
 
-template <int FORM, int L, int SUB = 1>
+template <int FORM, int L, int SUB = 1, int FOLD = tc::FOLD_NONE>
 const uint4* pass_image_device(TcDevice* d, bool inverse) {
   constexpr int li = lg_points(L / SUB);
   std::lock_guard<std::mutex> lock(g_tc_mutex);
   void*& slot = d->pass_images[FORM][li][inverse ? 1 : 0];
   if (!slot) {
-    const std::vector<uint8_t> img = pass_image<FORM, L, SUB>(inverse);
+    const std::vector<uint8_t> img = pass_image<FORM, L, SUB, FOLD>(inverse);
     void* ptr = nullptr;
     if (cudaMalloc(&ptr, img.size()) != cudaSuccess) return nullptr;
     if (cudaMemcpy(ptr, img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -306,14 +317,14 @@ const uint4* pass_image_device(TcDevice* d, bool inverse) {
 
 // One row pass: rows x (L / SUB) matrix at x -> transposed arrays (R = 1 << rshift rows each) at
 // out.  SUB > 1: the rows are read as rows / SUB super-rows of L = 64 floats.
-template <int FORM, int L, int SUB = 1>
-int launch_pass(const bridct_plan* p, bool inverse, const float* x, float* out, size_t rows, int rshift,
-                cudaStream_t st, TcDevice* d) {
-  using PL = tc::PassLayout<FORM, L>;
-  auto k = tc::k_tcpass<FORM, L, SUB>;
+template <int FORM, int L, int SUB, int FOLD>
+int launch_pass_fold(const bridct_plan* p, bool inverse, const float* x, float* out, size_t rows, int rshift,
+                     cudaStream_t st, TcDevice* d) {
+  using PL = tc::PassLayout<FORM, L, FOLD>;
+  auto k = tc::k_tcpass<FORM, L, SUB, FOLD>;
   if (kernel_setup(reinterpret_cast<const void*>(k), PL::kDynamic, tc::kPassThreads) <= 0)
     return cuda_fail(cudaErrorInvalidConfiguration, "k_tcpass shared memory");
-  const uint4* img = pass_image_device<FORM, L, SUB>(d, inverse);
+  const uint4* img = pass_image_device<FORM, L, SUB, FOLD>(d, inverse);
   if (!img) return cuda_fail(cudaGetLastError(), "tensor-core coefficient upload");
   const size_t srows = rows / SUB;   // SUB divides every array's row count (>= 8)
   CUtensorMap xm;
@@ -328,6 +339,17 @@ int launch_pass(const bridct_plan* p, bool inverse, const float* x, float* out, 
   cudaError_t e = launch_pdl(k, (unsigned)(slots * PL::kBlocks), tc::kPassThreads, PL::kDynamic, st, xm, out,
                              img, (long long)srows, rshift, d->err);
   return e == cudaSuccess ? BRIDCT_OK : cuda_fail(e, "k_tcpass launch");
+}
+template <int FORM, int L, int SUB = 1>
+int launch_pass(const bridct_plan* p, bool inverse, const float* x, float* out, size_t rows, int rshift,
+                cudaStream_t st, TcDevice* d) {
+  if constexpr (L >= 128) {
+    constexpr int inv = L <= 256 ? tc::FOLD_INV : tc::FOLD_NONE;
+    return inverse ? launch_pass_fold<FORM, L, SUB, inv>(p, inverse, x, out, rows, rshift, st, d)
+                   : launch_pass_fold<FORM, L, SUB, tc::FOLD_FWD>(p, inverse, x, out, rows, rshift, st, d);
+  } else {
+    return launch_pass_fold<FORM, L, SUB, tc::FOLD_NONE>(p, inverse, x, out, rows, rshift, st, d);
+  }
 }
 
 // BF16x3 on 64x64 arrays: both passes in one launch of k_tc64.

@@ -15,6 +15,14 @@
 // or arrives chunk by chunk with the ring (L = 512, 1024), and the CTA streams M-tiles through a
 // TMA ring in K-chunks (64 FP32 per row for BF16x3, 32 for TF32x3).  Rows of 8, 16 or 32 points
 // run as 64-float super-rows against a block-diagonal B (SUB).
+// Rows of 128 points and more use the symmetry of C_L (PassFold), which halves the products, and for
+// every output also the loads and splits:
+//   forward  u[j] = x[j] + x[L-1-j] and v[j] = x[j] - x[L-1-j], j < L/2, give the even and the odd
+//            coefficients as products of length L/2; an N-block is 64 even or 64 odd columns, and the
+//            split groups fold the row while they split it
+//   inverse  e[j] = sum over even k, o[j] = sum over odd k of C[k][j] X[k], j < L/2, give
+//            y[j] = e + o and y[L-1-j] = e - o; the split groups put the even elements of a K-chunk
+//            first, e and o accumulate apart, and the epilogue stores 128 columns per N-block
 // Split precision as in the 8x8 forms: BF16x3 = six products of 3-way splits, TF32x3 = three
 // products of 2-way splits, all accumulated in FP32 in TMEM.
 //
@@ -50,30 +58,39 @@ template <> struct PassForm<TF32X3> {
 };
 
 constexpr int kBAtom = 64 * 128;         // one K-major SW128 atom column of 64 B rows
-constexpr int kPassNBlock = 64;          // output columns per CTA (MMA N)
 constexpr int kPassSmemMax = 232448;     // opt-in shared memory per block
 constexpr int kPassMaxStages = 6;
 constexpr int kPassThreads = 512;
 
 constexpr int pass_min(int a, int b) { return a < b ? a : b; }
 
-// Shared-memory plan of one row pass.  The CTA's 64-column slice of C_L stays resident when it
-// fits beside a two-stage ring (L <= 256); for L = 512 and 1024 it does not (192-384 KB), and every
-// ring stage then carries the slice's K-chunk next to the A chunk (STREAM_B), brought in by a bulk
-// copy from the pre-split image in global memory (L2-resident: 0.4-1.5 MB per form and direction).
-template <int FORM, int L>
+enum PassFold { FOLD_NONE = 0, FOLD_FWD = 1, FOLD_INV = 2 };
+
+// Output columns per CTA (MMA N).  Folded forward passes of 256 points take 128, all columns of one
+// parity: with 64, every M-tile crosses from L2 four times, and that traffic (4.9 TB/s) bounds the pass.
+__host__ __device__ constexpr int pass_nblock(int L, int fold) { return fold == FOLD_FWD && L == 256 ? 128 : 64; }
+
+// Shared-memory plan of one row pass.  The CTA's slice of the coefficient matrix stays resident when it
+// fits beside a two-stage ring; otherwise every ring stage carries the slice's K-chunk next to the A
+// chunk (STREAM_B), brought in by a bulk copy from the pre-split image in global memory (L2-resident:
+// 0.2-1.5 MB per form and direction).  A folded forward stage holds both halves of the row's chunk, and
+// the split parts fill it in place, so that it needs no A buffers.
+template <int FORM, int L, int FOLD = FOLD_NONE>
 struct PassLayout {
   using F = PassForm<FORM>;
-  static constexpr int kChunks = L / F::kKC;
-  static constexpr int kBlocks = L / kPassNBlock;
-  static constexpr int kBBytes = F::kSplits * kChunks * kBAtom;   // this CTA's slice of C_L
-  static constexpr int kBChunk = F::kSplits * kBAtom;             // one K-chunk of the slice
-  static constexpr int kABufs = 2;
+  static constexpr int kK = FOLD == FOLD_FWD ? L / 2 : L;                  // products per output
+  static constexpr int kChunks = kK / F::kKC;
+  static constexpr int kNBlock = pass_nblock(L, FOLD);
+  static constexpr int kBlocks = (FOLD == FOLD_INV ? L / 2 : L) / kNBlock;
+  static constexpr int kBPart = kBAtom * kNBlock / 64;            // one split part of a K-chunk
+  static constexpr int kBBytes = F::kSplits * kChunks * kBPart;   // this CTA's slice of C_L
+  static constexpr int kBChunk = F::kSplits * kBPart;             // one K-chunk of the slice
+  static constexpr int kABufs = FOLD == FOLD_FWD ? 0 : 2;
+  static constexpr int kABytes = (FOLD == FOLD_FWD ? 2 : 1) * F::kStageBytes;   // A data of a stage
   static constexpr int kBarBytes = 1024;
-  static constexpr bool kStreamB =
-      kBBytes + kABufs * F::kABufBytes + kBarBytes + 1024 + 2 * F::kStageBytes > kPassSmemMax;
+  static constexpr bool kStreamB = kBBytes + kABufs * F::kABufBytes + kBarBytes + 1024 + 2 * kABytes > kPassSmemMax;
   static constexpr int kResident = kStreamB ? 0 : kBBytes;
-  static constexpr int kStageStride = F::kStageBytes + (kStreamB ? kBChunk : 0);
+  static constexpr int kStageStride = kABytes + (kStreamB ? kBChunk : 0);
   static constexpr int kStageTx = kStageStride;                  // bytes a stage's loads deliver
   static constexpr int kFixed = kResident + kABufs * F::kABufBytes + kBarBytes + 1024;
   static constexpr int kStages = pass_min(kPassMaxStages, (kPassSmemMax - kFixed) / kStageStride);
@@ -83,6 +100,10 @@ struct PassLayout {
   static constexpr int kBarOff = kBOff + kResident;
   static constexpr int kDynamic = kBarOff + kBarBytes + 1024;      // + 1024-byte alignment slack
   static_assert(kDynamic <= kPassSmemMax, "shared memory budget");
+  // where the split parts lie: hi at the stage, mid (BF16x3) and lo at these offsets, lo in the A buffer
+  // unless folded forward
+  static constexpr int kMidOff = FOLD == FOLD_FWD ? 49152 : 16384;
+  static constexpr int kLoOff = 16384;
 };
 
 // Bulk copy of `bytes` (a multiple of 16) from global memory into shared memory, completing on bar.
@@ -112,7 +133,121 @@ __device__ __forceinline__ void split_box_tf32(uint8_t* stage, uint8_t* abuf, ui
   }
 }
 
-// Accumulator set of one M-tile (64 TMEM columns per block).  The FP32 accumulation of an MMA
+// Folded splits: element i of the folded chunk is a[i] + sign * b[last - i], with a the chunk's row of
+// the first half of the matrix row and b that of the mirrored chunk.
+// BF16x3: boxes a0, a1, b0, b1 of 16 KB.  hi goes to a0, lo to a1, mid to b1; each half of the chunk
+// reads its two source rows completely before it writes there, and lo of the first half, which would
+// overwrite a1, waits in registers.
+__device__ __forceinline__ void split_fold_bf16(uint8_t* stage, uint32_t r, float sign) {
+  uint32_t lo0[4][4];
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    float x[32];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float4 u = *reinterpret_cast<const float4*>(stage + half * 16384u + sw128(r, c));
+      const float4 w = *reinterpret_cast<const float4*>(stage + (half ? 32768u : 49152u) + sw128(r, 7 - c));
+      x[4 * c] = fmaf(sign, w.w, u.x);
+      x[4 * c + 1] = fmaf(sign, w.z, u.y);
+      x[4 * c + 2] = fmaf(sign, w.y, u.z);
+      x[4 * c + 3] = fmaf(sign, w.x, u.w);
+    }
+#pragma unroll
+    for (int jq = 0; jq < 4; ++jq) {
+      uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split_bf16x3_pair(x[8 * jq + 2 * e], x[8 * jq + 2 * e + 1], hi[e], mid[e], lo[e]);
+      const uint32_t off = sw128(r, half * 4 + jq);
+      *reinterpret_cast<uint4*>(stage + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(stage + 49152u + off) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+      if (half) {
+        *reinterpret_cast<uint4*>(stage + 16384u + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) lo0[jq][e] = lo[e];
+      }
+    }
+  }
+#pragma unroll
+  for (int jq = 0; jq < 4; ++jq)
+    *reinterpret_cast<uint4*>(stage + 16384u + sw128(r, jq)) =
+        make_uint4(lo0[jq][0], lo0[jq][1], lo0[jq][2], lo0[jq][3]);
+}
+// TF32x3: boxes a, b; hi goes to a, lo to b.
+__device__ __forceinline__ void split_fold_tf32(uint8_t* stage, uint32_t r, float sign) {
+  float4 w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(stage + 16384u + sw128(r, j));
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t off = sw128(r, j);
+    const float4 u = *reinterpret_cast<const float4*>(stage + off);
+    uint4 h, l;
+    split_tf32x2(make_float4(fmaf(sign, w[7 - j].w, u.x), fmaf(sign, w[7 - j].z, u.y), fmaf(sign, w[7 - j].y, u.z),
+                             fmaf(sign, w[7 - j].x, u.w)),
+                 h, l);
+    *reinterpret_cast<uint4*>(stage + off) = h;
+    *reinterpret_cast<uint4*>(stage + 16384u + off) = l;
+  }
+}
+// Deinterleaving splits (inverse): the chunk's even elements go to K positions 0.., the odd ones to the
+// second half.  BF16x3: as split_tile<BF16X3>, with half `half` of the row giving 16 even elements
+// (16-byte pieces 2 half, 2 half + 1) and 16 odd ones (pieces 4 + 2 half, ...).
+__device__ __forceinline__ void split_deint_bf16(uint8_t* stage, uint8_t* abuf, uint32_t r) {
+  uint32_t mid0[4][4];
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    float x[32];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float4 u = *reinterpret_cast<const float4*>(stage + half * 16384u + sw128(r, c));
+      x[4 * c] = u.x; x[4 * c + 1] = u.y; x[4 * c + 2] = u.z; x[4 * c + 3] = u.w;
+    }
+#pragma unroll
+    for (int jq = 0; jq < 4; ++jq) {
+      const int odd = jq >> 1, piece = odd * 4 + half * 2 + (jq & 1);
+      uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = (jq & 1) * 16 + 4 * e + odd;   // elements i and i + 2 of this half
+        split_bf16x3_pair(x[i], x[i + 2], hi[e], mid[e], lo[e]);
+      }
+      const uint32_t off = sw128(r, piece);
+      *reinterpret_cast<uint4*>(stage + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(abuf + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      if (half) {
+        *reinterpret_cast<uint4*>(stage + 16384u + off) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mid0[jq][e] = mid[e];
+      }
+    }
+  }
+#pragma unroll
+  for (int jq = 0; jq < 4; ++jq)
+    *reinterpret_cast<uint4*>(stage + 16384u + sw128(r, (jq >> 1) * 4 + (jq & 1))) =
+        make_uint4(mid0[jq][0], mid0[jq][1], mid0[jq][2], mid0[jq][3]);
+}
+// TF32x3: 32 elements of a row, even ones to 16-byte pieces 0..3, odd ones to 4..7.
+__device__ __forceinline__ void split_deint_tf32(uint8_t* stage, uint8_t* abuf, uint32_t r) {
+  float x[32];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const float4 u = *reinterpret_cast<const float4*>(stage + sw128(r, c));
+    x[4 * c] = u.x; x[4 * c + 1] = u.y; x[4 * c + 2] = u.z; x[4 * c + 3] = u.w;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int i = (j & 3) * 8 + (j >> 2);
+    uint4 h, l;
+    split_tf32x2(make_float4(x[i], x[i + 2], x[i + 4], x[i + 6]), h, l);
+    const uint32_t off = sw128(r, j);
+    *reinterpret_cast<uint4*>(stage + off) = h;
+    *reinterpret_cast<uint4*>(abuf + off) = l;
+  }
+}
+
+// Accumulator set of one M-tile (N-block TMEM columns per block: NB = 64 or 128).  The FP32 accumulation of an MMA
 // into a large accumulator loses the addends' low bits toward zero, so the dominant Xh.Ch
 // product accumulates apart from the small products (whose own losses are then negligible),
 // and over long K it is spread over kBig group accumulators by K-chunk, each receiving few
@@ -127,59 +262,94 @@ __device__ __forceinline__ void split_box_tf32(uint8_t* stage, uint8_t* abuf, ui
 // MMAs of the next) for rows up to 256 points, one for 512- and 1024-point rows, whose long K
 // needs more group accumulators than two sets leave room for (TF32x3 round trips of 1024-point
 // axes exceeded 3e-6 with three groups; one set holds seven for TF32x3, six for BF16x3).
-template <int FORM, int CHUNKS, int SETS = 2>
+// PARS = 2 (folded inverse): a set holds the blocks of e, then those of o.
+template <int FORM, int CHUNKS, int SETS = 2, int PARS = 1, int NB = 64>
 struct PassAccs {
+  static constexpr int kNBlock = NB;
   static constexpr int kSmallBlocks = FORM == BF16X3 ? 2 : 1;
-  static constexpr int kMaxBig = SETS == 2 ? (FORM == BF16X3 ? 2 : 3) : 512 / kPassNBlock - kSmallBlocks;
+  static constexpr int kMaxBig = 512 / (SETS * PARS * NB) - kSmallBlocks;
   static constexpr int kBig = CHUNKS < kMaxBig ? CHUNKS : kMaxBig;
-  static constexpr int kPerTile = (1 + kSmallBlocks + (kBig - 1)) * kPassNBlock;   // columns
-  static constexpr int kExtraBig = (1 + kSmallBlocks) * kPassNBlock;               // big1 column
+  static constexpr int kPerParity = (1 + kSmallBlocks + (kBig - 1)) * NB;
+  static constexpr int kPerTile = PARS * kPerParity;                               // columns
+  static constexpr int kExtraBig = (1 + kSmallBlocks) * NB;                        // big1 column
   static constexpr int kAlloc = SETS * kPerTile <= 256 ? 256 : 512;
-  static_assert(SETS * kPerTile <= 512, "TMEM columns");
+  static_assert(kBig >= 1 && SETS * kPerTile <= 512, "TMEM columns");
   __host__ __device__ static constexpr int group(int kc) { return kc * kBig / CHUNKS; }
 };
 
-template <int L> struct PassSets { static constexpr int value = L >= 512 ? 1 : 2; };
+// Accumulator sets: one where long K needs the groups (or e and o do not fit twice).
+template <int FORM, int L, int FOLD> struct PassSets {
+  static constexpr int value = FOLD == FOLD_INV ? 1 : FOLD == FOLD_FWD ? (L >= 256 ? 1 : 2) : L >= 512 ? 1 : 2;
+};
 
-// Split products of K-chunk kc (one thread).  bchunk: shared address of the chunk's B splits,
-// laid out [split][8 KB atom column of 64 rows].  tmem: column 0 of this M-tile's set.
-template <int FORM, int CHUNKS, int SETS>
-__device__ __forceinline__ void issue_pass_mmas(uint32_t sstage, uint32_t sabuf, uint32_t bchunk, int kc,
+// Split products of K-chunk kc (one thread): hi, mid, lo: shared addresses of the A parts (mid: BF16x3
+// only).  bchunk: shared address of the chunk's B splits, laid out [split][8 KB atom column of 64 rows].
+// tmem: column 0 of this M-tile's set.  A chunk is four K steps; with PARS = 2 the first two are e's.
+template <int FORM, int CHUNKS, int SETS, int PARS, int NB>
+__device__ __forceinline__ void issue_pass_mmas(uint32_t hi, uint32_t mid, uint32_t lo, uint32_t bchunk, int kc,
                                                 uint32_t tmem) {
-  using A = PassAccs<FORM, CHUNKS, SETS>;
+  using A = PassAccs<FORM, CHUNKS, SETS, PARS, NB>;
+  constexpr uint32_t kPart = kBAtom * NB / 64;
   const int g = A::group(kc);
   const bool big_first = kc == 0 || A::group(kc - 1) != g;
-  const uint32_t big_g = tmem + A::kExtraBig + (uint32_t)(g - 1) * kPassNBlock;
-  if constexpr (FORM == BF16X3) {
-    constexpr uint32_t i192 = instr_desc(1, 192), i128 = instr_desc(1, 128), i64 = instr_desc(1, 64);
+  constexpr int kSteps = 4 / PARS;   // K steps of one parity in a chunk
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {   // 16 bf16 (32 bytes) per MMA
-      const uint64_t bd = sw128_desc(bchunk + k * 32u);
-      const uint64_t ah = sw128_desc(sstage + k * 32u);
-      if (g == 0) {
-        umma(tmem, ah, bd, i192, (kc | k) ? 1u : 0u, BF16X3);
+  for (int k = 0; k < 4; ++k) {   // 32 bytes of a row per MMA: 16 bf16 or 8 tf32
+    const uint32_t t = tmem + (uint32_t)(k / kSteps) * A::kPerParity;
+    const uint32_t big_g = t + A::kExtraBig + (uint32_t)(g - 1) * NB;
+    const bool first = k % kSteps == 0;
+    const uint64_t bd = sw128_desc(bchunk + k * 32u);
+    const uint64_t ah = sw128_desc(hi + k * 32u);
+    const uint32_t clear = (kc == 0 && first) ? 0u : 1u, clear_g = (big_first && first) ? 0u : 1u;
+    if constexpr (FORM == BF16X3) {
+      constexpr uint32_t i3 = instr_desc(1, NB == 64 ? 192 : 256), i2 = instr_desc(1, 2 * NB), i1 = instr_desc(1, NB);
+      if (g == 0 && NB == 64) {
+        umma(t, ah, bd, i3, clear, BF16X3);
+      } else if (g == 0) {   // N = 384 does not fit one MMA
+        umma(t, ah, bd, i2, clear, BF16X3);
+        umma(t + 2 * NB, ah, sw128_desc(bchunk + 2 * kPart + k * 32u), i1, clear, BF16X3);
       } else {
-        umma(big_g, ah, bd, i64, (big_first && k == 0) ? 0u : 1u, BF16X3);
-        umma(tmem + 64, ah, sw128_desc(bchunk + kBAtom + k * 32u), i128, 1u, BF16X3);
+        umma(big_g, ah, bd, i1, clear_g, BF16X3);
+        umma(t + NB, ah, sw128_desc(bchunk + kPart + k * 32u), i2, 1u, BF16X3);
       }
-      umma(tmem + 64, sw128_desc(sstage + 16384u + k * 32u), bd, i128, 1u, BF16X3);   // Xm
-      umma(tmem + 64, sw128_desc(sabuf + k * 32u), bd, i64, 1u, BF16X3);              // Xl
-    }
-  } else {
-    constexpr uint32_t i128 = instr_desc(2, 128), i64 = instr_desc(2, 64);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {   // 8 tf32 (32 bytes) per MMA
-      const uint64_t bd = sw128_desc(bchunk + k * 32u);
-      const uint64_t ah = sw128_desc(sstage + k * 32u);
+      umma(t + NB, sw128_desc(mid + k * 32u), bd, i2, 1u, BF16X3);   // Xm
+      umma(t + NB, sw128_desc(lo + k * 32u), bd, i1, 1u, BF16X3);    // Xl
+    } else {
+      constexpr uint32_t i2 = instr_desc(2, 2 * NB), i1 = instr_desc(2, NB);
       if (g == 0) {
-        umma(tmem, ah, bd, i128, (kc | k) ? 1u : 0u, TF32X3);
+        umma(t, ah, bd, i2, clear, TF32X3);
       } else {
-        umma(big_g, ah, bd, i64, (big_first && k == 0) ? 0u : 1u, TF32X3);
-        umma(tmem + 64, ah, sw128_desc(bchunk + kBAtom + k * 32u), i64, 1u, TF32X3);
+        umma(big_g, ah, bd, i1, clear_g, TF32X3);
+        umma(t + NB, ah, sw128_desc(bchunk + kPart + k * 32u), i1, 1u, TF32X3);
       }
-      umma(tmem + 64, sw128_desc(sabuf + k * 32u), bd, i64, 1u, TF32X3);   // Xl
+      umma(t + NB, sw128_desc(lo + k * 32u), bd, i1, 1u, TF32X3);   // Xl
     }
   }
+}
+
+// Columns q*16 .. q*16+15 of the sum of one parity's accumulator blocks at taddr.
+template <typename ACC>
+__device__ __forceinline__ void load_sum(uint32_t taddr, int q, float (&big)[16]) {
+  float sm[16], w[16];
+  tmem_ld16(taddr + q * 16, big);
+  tmem_ld16(taddr + ACC::kNBlock + q * 16, sm);
+  tmem_wait_ld();
+#pragma unroll
+  for (int a = 0; a < ACC::kSmallBlocks - 1; ++a) {
+    tmem_ld16(taddr + (2 + a) * ACC::kNBlock + q * 16, w);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) sm[i] += w[i];
+  }
+#pragma unroll
+  for (int a = 1; a < ACC::kBig; ++a) {
+    tmem_ld16(taddr + ACC::kExtraBig + (a - 1) * ACC::kNBlock + q * 16, w);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) big[i] += w[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) big[i] += sm[i];
 }
 
 // xmap: the (nrows x L) FP32 row matrix (box 32 x 128, SWIZZLE_128B).  out: destination of
@@ -189,18 +359,22 @@ __device__ __forceinline__ void issue_pass_mmas(uint32_t sstage, uint32_t sabuf,
 // consecutive rows of length LS (a super-row); B is block-diagonal (SUB copies of C_LS), so
 // column n = j * LS + c of super-row g is output column c of row g * SUB + j, and nrows counts
 // super-rows.
-template <int FORM, int L, int SUB = 1>
+// FOLD: see the file comment (L >= 128).  Folded forward, N-block i holds the columns
+// 2 (NB (i / 2) + n) + i % 2 (NB columns); folded inverse, the columns 64 i + n and L - 1 - (64 i + n).
+template <int FORM, int L, int SUB = 1, int FOLD = FOLD_NONE>
 __global__ void __launch_bounds__(kPassThreads, 1)
     k_tcpass(const __grid_constant__ CUtensorMap xmap, float* __restrict__ out,
              const uint4* __restrict__ bimage, long long nrows, int rshift, int* __restrict__ err) {
   static_assert(SUB == 1 || L == 64, "super-rows are 64 floats");
+  static_assert(FOLD == FOLD_NONE || (SUB == 1 && L >= 128), "folded rows");
   constexpr int LS = L / SUB;   // points per original row
-  using PL = PassLayout<FORM, L>;
+  using PL = PassLayout<FORM, L, FOLD>;
   using F = PassForm<FORM>;
   constexpr int kStages = PL::kStages;
   constexpr int kChunks = PL::kChunks;
-  constexpr int kSets = PassSets<L>::value;
-  using ACC = PassAccs<FORM, kChunks, kSets>;
+  constexpr int kSets = PassSets<FORM, L, FOLD>::value;
+  constexpr int kPars = FOLD == FOLD_INV ? 2 : 1;
+  using ACC = PassAccs<FORM, kChunks, kSets, kPars, PL::kNBlock>;
   constexpr uint32_t kTileCols = ACC::kPerTile;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -266,8 +440,14 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       tma_load_2d(dst, &xmap, kc * F::kKC, (int)(m * kRows), bars.stage_full + 8 * s);
       if constexpr (F::kKC == 64)
         tma_load_2d(dst + 16384u, &xmap, kc * F::kKC + 32, (int)(m * kRows), bars.stage_full + 8 * s);
+      if constexpr (FOLD == FOLD_FWD) {   // the mirrored chunk
+#pragma unroll
+        for (int b = 0; b < F::kKC / 32; ++b)
+          tma_load_2d(dst + F::kStageBytes + b * 16384u, &xmap, L - (kc + 1) * F::kKC + b * 32, (int)(m * kRows),
+                      bars.stage_full + 8 * s);
+      }
       if constexpr (PL::kStreamB)
-        bulk_load(dst + F::kStageBytes,
+        bulk_load(dst + PL::kABytes,
                   reinterpret_cast<const uint8_t*>(bimage) + (size_t)nblk * PL::kBBytes + (size_t)kc * PL::kBChunk,
                   PL::kBChunk, bars.stage_full + 8 * s);
     }
@@ -281,10 +461,12 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       if (!ok) break;
       tc_fence_after();
       const uint32_t sstage = sbase + s * PL::kStageStride;
-      const uint32_t bchunk = PL::kStreamB ? sstage + F::kStageBytes
-                                           : sbase + PL::kBOff + (uint32_t)(kc * F::kSplits) * kBAtom;
-      issue_pass_mmas<FORM, kChunks, kSets>(sstage, sbase + PL::kAOff + a * F::kABufBytes, bchunk, kc,
-                                     tmem_base + t * kTileCols);
+      const uint32_t bchunk = PL::kStreamB ? sstage + PL::kABytes
+                                           : sbase + PL::kBOff + (uint32_t)kc * PL::kBChunk;
+      issue_pass_mmas<FORM, kChunks, kSets, kPars, PL::kNBlock>(
+          sstage, sstage + PL::kMidOff,
+          FOLD == FOLD_FWD ? sstage + PL::kLoOff : sbase + PL::kAOff + a * F::kABufBytes, bchunk, kc,
+          tmem_base + t * kTileCols);
       umma_commit(bars.stage_free + 8 * s);
       umma_commit(bars.a_free + 8 * a);
       if (kc == kChunks - 1) umma_commit(bars.acc_full + 8 * t);
@@ -311,8 +493,17 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       }
       uint8_t* stage = base + s * PL::kStageStride;
       uint8_t* abuf = base + PL::kAOff + a * F::kABufBytes;
-      if constexpr (FORM == BF16X3) split_tile<BF16X3>(stage, abuf, r);
-      else split_box_tf32(stage, abuf, r);
+      if constexpr (FOLD == FOLD_FWD) {
+        const float sign = nblk & 1 ? -1.0f : 1.0f;
+        if constexpr (FORM == BF16X3) split_fold_bf16(stage, r, sign);
+        else split_fold_tf32(stage, r, sign);
+      } else if constexpr (FOLD == FOLD_INV) {
+        if constexpr (FORM == BF16X3) split_deint_bf16(stage, abuf, r);
+        else split_deint_tf32(stage, abuf, r);
+      } else {
+        if constexpr (FORM == BF16X3) split_tile<BF16X3>(stage, abuf, r);
+        else split_box_tf32(stage, abuf, r);
+      }
       fence_async_smem();
       named_sync(bar_id, 128);
       if (r == 0) mbar_arrive(bars.a_full + 8 * a);
@@ -338,34 +529,39 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       const bool live = g < nrows;
       const long long g0 = g * SUB;
       const long long b = g0 >> rshift, h = g0 & rmask;
-      float* dst = out + ((b * LS + (long long)nblk * kPassNBlock) << rshift) + h;
       const uint32_t taddr = tmem_base + t * kTileCols + (quarter << 16);
+      float* arr = out + ((b * LS) << rshift) + h;
+      if constexpr (FOLD == FOLD_INV) {
+        float* lo = arr + ((long long)(nblk * PL::kNBlock) << rshift);
+        float* hi = arr + ((long long)(L - 1 - nblk * PL::kNBlock) << rshift);
 #pragma unroll
-      for (int q = 0; q < kPassNBlock / 16; ++q) {
-        float big[16], sm[16], w[16];
-        tmem_ld16(taddr + q * 16, big);
-        tmem_ld16(taddr + kPassNBlock + q * 16, sm);
-        tmem_wait_ld();
+        for (int q = 0; q < PL::kNBlock / 16; ++q) {
+          float e[16], o[16];
+          load_sum<ACC>(taddr, q, e);
+          load_sum<ACC>(taddr + ACC::kPerParity, q, o);
+          if (live) {
 #pragma unroll
-        for (int a = 0; a < ACC::kSmallBlocks - 1; ++a) {
-          tmem_ld16(taddr + (2 + a) * kPassNBlock + q * 16, w);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) sm[i] += w[i];
+            for (int i = 0; i < 16; ++i) {
+              const long long c = (long long)(q * 16 + i) << rshift;
+              lo[c] = e[i] + o[i];
+              hi[-c] = e[i] - o[i];
+            }
+          }
         }
+      } else {
+        float* dst = arr + ((long long)(FOLD == FOLD_FWD ? (nblk >> 1) * 2 * PL::kNBlock + (nblk & 1)
+                                                         : nblk * PL::kNBlock) << rshift);
 #pragma unroll
-        for (int a = 1; a < ACC::kBig; ++a) {
-          tmem_ld16(taddr + ACC::kExtraBig + (a - 1) * kPassNBlock + q * 16, w);
-          tmem_wait_ld();
+        for (int q = 0; q < PL::kNBlock / 16; ++q) {
+          float v[16];
+          load_sum<ACC>(taddr, q, v);
+          if (live) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) big[i] += w[i];
-        }
-        if (live) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            constexpr int kLS = LS;
-            const int n = q * 16 + i, j = n / kLS, c = n % kLS;
-            dst[((long long)c << rshift) + j] = big[i] + sm[i];
+            for (int i = 0; i < 16; ++i) {
+              constexpr int kLS = LS;
+              const int n = q * 16 + i, j = n / kLS, c = n % kLS * (FOLD == FOLD_FWD ? 2 : 1);
+              dst[((long long)c << rshift) + j] = v[i];
+            }
           }
         }
       }
