@@ -262,11 +262,16 @@ __device__ __forceinline__ void split_deint_tf32(uint8_t* stage, uint8_t* abuf, 
 // MMAs of the next) for rows up to 256 points, one for 512- and 1024-point rows, whose long K
 // needs more group accumulators than two sets leave room for (TF32x3 round trips of 1024-point
 // axes exceeded 3e-6 with three groups; one set holds seven for TF32x3, six for BF16x3).
-// PARS = 2 (folded inverse): a set holds the blocks of e, then those of o.
+// PARS = 2 (folded inverse): a set holds the blocks of e, then those of o, half as many for each.  From 512
+// points on BF16x3 then adds all small products in one block, [big0 | small | big1 | big2], so that a big
+// group takes no more MMAs than in an unfolded pass (errors against float64 1.75e-7 -> 1.59e-7 at 512 x
+// 512, 2.77e-7 -> 2.66e-7 at 1024 x 1024; with two groups 2.01e-7 and 3.73e-7).  TF32x3 has nothing to
+// give up, and its inverse passes of 512 and 1024 points are not folded (launch_pass).
 template <int FORM, int CHUNKS, int SETS = 2, int PARS = 1, int NB = 64>
 struct PassAccs {
   static constexpr int kNBlock = NB;
-  static constexpr int kSmallBlocks = FORM == BF16X3 ? 2 : 1;
+  static constexpr bool kMerge = FORM == BF16X3 && PARS == 2 && CHUNKS >= 8;
+  static constexpr int kSmallBlocks = FORM == BF16X3 && !kMerge ? 2 : 1;
   static constexpr int kMaxBig = 512 / (SETS * PARS * NB) - kSmallBlocks;
   static constexpr int kBig = CHUNKS < kMaxBig ? CHUNKS : kMaxBig;
   static constexpr int kPerParity = (1 + kSmallBlocks + (kBig - 1)) * NB;
@@ -301,7 +306,16 @@ __device__ __forceinline__ void issue_pass_mmas(uint32_t hi, uint32_t mid, uint3
     const uint64_t bd = sw128_desc(bchunk + k * 32u);
     const uint64_t ah = sw128_desc(hi + k * 32u);
     const uint32_t clear = (kc == 0 && first) ? 0u : 1u, clear_g = (big_first && first) ? 0u : 1u;
-    if constexpr (FORM == BF16X3) {
+    if constexpr (A::kMerge) {
+      constexpr uint32_t i1 = instr_desc(1, NB);
+      const uint64_t bm = sw128_desc(bchunk + kPart + k * 32u);
+      umma(g == 0 ? t : big_g, ah, bd, i1, g == 0 ? clear : clear_g, BF16X3);
+      umma(t + NB, ah, bm, i1, clear, BF16X3);
+      umma(t + NB, ah, sw128_desc(bchunk + 2 * kPart + k * 32u), i1, 1u, BF16X3);
+      umma(t + NB, sw128_desc(mid + k * 32u), bd, i1, 1u, BF16X3);
+      umma(t + NB, sw128_desc(mid + k * 32u), bm, i1, 1u, BF16X3);
+      umma(t + NB, sw128_desc(lo + k * 32u), bd, i1, 1u, BF16X3);
+    } else if constexpr (FORM == BF16X3) {
       constexpr uint32_t i3 = instr_desc(1, NB == 64 ? 192 : 256), i2 = instr_desc(1, 2 * NB), i1 = instr_desc(1, NB);
       if (g == 0 && NB == 64) {
         umma(t, ah, bd, i3, clear, BF16X3);
