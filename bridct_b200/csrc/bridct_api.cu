@@ -8,7 +8,7 @@
 //   * a plan is not reentrant (one plan per concurrent caller), it owns its scratch and
 //     apply performs no allocation;
 //   * route strings "paper8-square" / "blocked-extension".
-// GPU specifics: every device gets one immutable context (SM count, four-step tables,
+// GPU specifics: every device gets one immutable context (SM count, split-line tables,
 // launcher table) created on first use; each plan owns a CUDA stream plus device and
 // pinned staging for host-pointer calls.
 #include <cuda_runtime.h>
@@ -56,44 +56,6 @@ double sj_scale(int n, int k) {
   return sj_scale(n / 4, k) * (k <= n / 8 ? std::cos(angle) : std::sin(angle));
 }
 
-// Four-step tables for N = 32 G (see sj_lines.cuh): twiddles w_N^{bc} s(32,c) and the
-// post-rotation coefficients with the stage-2 SJ scale of each column and the orthonormal
-// factor folded in.  Stage 2 of column c produces V(d) / scale(c, d) with
-//   scale = s(G, d)          columns 1..15 when G < 32 (SJ scaled complex FFT),
-//           s(16, d >> 1)    columns 1..15 when G = 32 (split into two radix-2 halves),
-//           1                columns 0 and 16 (cooperative shuffle DFT across the lanes).
-// Fills caller-provided arrays of G*17 float2 (tw[b*17+c]) and G*17 float4 (post at
-// post_index(G, d, c)).
-void fill_fourstep_tables(int N, float2* tw, float4* post) {
-  const int G = N / 32;
-  for (int b = 0; b < G; ++b)
-    for (int c = 0; c < 17; ++c) {
-      const double ang = -2 * M_PI * (double)b * c / N;
-      const double s = sj_scale(32, c);
-      tw[(size_t)b * 17 + c] = float2{(float)(std::cos(ang) * s), (float)(std::sin(ang) * s)};
-    }
-  auto sig = [N](int k) { return std::sqrt((k == 0 ? 1.0 : 2.0) / N); };
-  for (int c = 0; c < 17; ++c)
-    for (int d = 0; d < G; ++d) {
-      const int k = c + 32 * d;
-      const double th = M_PI * k / (2.0 * N);
-      const double sg = (c == 0 || c == 16) ? 1.0 : G == 32 ? sj_scale(16, d >> 1) : sj_scale(G, d);
-      float4 p;
-      p.x = (float)(sig(k) * sg * std::cos(th));
-      p.y = (float)(sig(k) * sg * std::sin(th));
-      p.z = k ? (float)(sig(N - k) * sg * std::sin(th)) : 0.f;
-      p.w = k ? (float)(-sig(N - k) * sg * std::cos(th)) : 0.f;
-      post[post_index(G, d, c)] = p;
-    }
-}
-
-void build_fourstep_tables(int N, std::vector<float2>& tw, std::vector<float4>& post) {
-  const int G = N / 32;
-  tw.assign((size_t)G * 17, float2{0, 0});
-  post.assign((size_t)17 * G, float4{0, 0, 0, 0});
-  fill_fourstep_tables(N, tw.data(), post.data());
-}
-
 // Rotation tables of the split lines of N points (sj_split.cuh, SplitTab): stage-1 twiddles
 // w_N^{bc} s(A, c), then the post rotations with the stage-2 scale of each output (s(B, j); s(B/2, m)
 // for column A/2) and the orthonormal factor folded in.
@@ -123,6 +85,13 @@ static std::vector<float> build_split_tables() {
       put(s * std::cos(M_PI * k / (2.0 * N)), s * std::sin(M_PI * k / (2.0 * N)));
     }
   return t;
+}
+
+std::vector<float> split_tables_host(int N) {
+  return N == 128   ? build_split_tables<128>()
+         : N == 256 ? build_split_tables<256>()
+         : N == 512 ? build_split_tables<512>()
+                    : build_split_tables<1024>();
 }
 
 #define BRIDCT_DECL_H(H)                                                            \
@@ -194,35 +163,12 @@ DeviceCtx* device_ctx(int device) {
   plain_table_h512(tab[6], d->col_units[6], d->row_units[6]);
   plain_table_h1024(tab[7], d->col_units[7], d->row_units[7]);
   for (int i = 0; i < 4; ++i) {
-    const int N = 128 << i;
-    std::vector<float2> tw;
-    std::vector<float4> post;
-    build_fourstep_tables(N, tw, post);
-    const size_t btw = tw.size() * sizeof(float2), bpo = post.size() * sizeof(float4);
+    const std::vector<float> t = split_tables_host(128 << i);
     void* mem = nullptr;
-    e = cudaMalloc(&mem, btw + bpo);
-    if (e != cudaSuccess) {
-      cuda_fail(e, "cudaMalloc(tables)");
-      return nullptr;
-    }
-    d->table_mem.push_back(mem);
-    cudaMemcpy(mem, tw.data(), btw, cudaMemcpyHostToDevice);
-    e = cudaMemcpy((char*)mem + btw, post.data(), bpo, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      cuda_fail(e, "cudaMemcpy(tables)");
-      return nullptr;
-    }
-    d->fourstep[i].tw = (const float2*)mem;
-    d->fourstep[i].post = (const float4*)((char*)mem + btw);
-  }
-  const std::vector<float> split[4] = {build_split_tables<128>(), build_split_tables<256>(), build_split_tables<512>(),
-                                       build_split_tables<1024>()};
-  for (int i = 0; i < 4; ++i) {
-    void* mem = nullptr;
-    e = cudaMalloc(&mem, split[i].size() * sizeof(float));
+    e = cudaMalloc(&mem, t.size() * sizeof(float));
     if (e == cudaSuccess) {
       d->table_mem.push_back(mem);
-      e = cudaMemcpy(mem, split[i].data(), split[i].size() * sizeof(float), cudaMemcpyHostToDevice);
+      e = cudaMemcpy(mem, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice);
     }
     if (e != cudaSuccess) {
       cuda_fail(e, "split-line tables");
@@ -235,15 +181,10 @@ DeviceCtx* device_ctx(int device) {
   return raw;
 }
 
-FourStepTables DeviceCtx::tables(int n) const {
-  if (n < 128) return FourStepTables{nullptr, nullptr};
-  return fourstep[lg2(n) - 4];
-}
-
 LineTables DeviceCtx::line_tables(int h, int w) const {
-  LineTables t{tables(h), tables(w)};
-  if (h >= 128) t.scol = split[lg2(h) - 4];
-  if (w >= 128) t.srow = split[lg2(w) - 4];
+  LineTables t;
+  if (h >= 128) t.col = split[lg2(h) - 4];
+  if (w >= 128) t.row = split[lg2(w) - 4];
   return t;
 }
 

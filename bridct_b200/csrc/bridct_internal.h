@@ -20,19 +20,16 @@ struct DeviceCtx {
   PlainLauncher plain[8][8][3] = {};
   UnitLauncher col_units[8][3] = {};    // merged column passes, by lg(column length) and mode
   UnitLauncher row_units[8][3] = {};    // merged row passes, by lg(row length) and mode
-  FourStepTables fourstep[4] = {};      // N = 128, 256, 512, 1024
-  SplitTables split[4] = {};            // the same lengths
+  SplitTables split[4] = {};            // rotation tables of N = 128, 256, 512, 1024
   std::vector<void*> table_mem;
-  FourStepTables tables(int n) const;
   LineTables line_tables(int h, int w) const;
 };
 
 void set_error(const std::string& s);
 int cuda_fail(cudaError_t e, const char* what);
 double sj_scale(int n, int k);
-// Four-step tables of line length N (twiddles, post-rotation coefficients), float64-derived.
-void build_fourstep_tables(int N, std::vector<float2>& tw, std::vector<float4>& post);
-void fill_fourstep_tables(int N, float2* tw, float4* post);
+// Rotation tables of the split lines of N = 128..1024 points (sj_split.cuh, SplitTab), float64-derived.
+std::vector<float> split_tables_host(int N);
 DeviceCtx* device_ctx(int device);
 // Opts `kernel` into `smem` bytes of dynamic shared memory on the current device and returns
 // its resident blocks per SM at `threads` threads (0 on failure); cached per device, since the

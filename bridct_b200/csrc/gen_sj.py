@@ -466,8 +466,8 @@ def emit_function(g: Graph, name: str, in_names: Sequence[str], outputs: Sequenc
 # ----------------------------------------------------------------------------------------
 
 REG_SIZES = (8, 16, 32, 64, 128)    # whole line in one thread's registers
-LEAF = 32                           # four-step leaf length for N >= 128
-STAGE2_SIZES = (4, 8, 16, 32)       # G = N / LEAF
+SCALAR_LINES = (8, 128)             # ... of which sj_generated.cuh holds the scalar programs in use
+STAGE2_SIZES = (4, 8, 16, 32)       # complex FFT lengths that the self-test covers
 
 
 def build_line_ops(n: int):
@@ -489,7 +489,7 @@ def build_line_ops(n: int):
 
 
 def build_rfft_leaf(n: int):
-    """Four-step stage 1: scaled real FFT of length n; outputs re[0..n/2], im[1..n/2-1]."""
+    """Stage 1 of a split line: scaled real FFT of length n; outputs re[0..n/2], im[1..n/2-1]."""
     g = Graph()
     xs = [g.inp(i) for i in range(n)]
     z = rfft(g, xs, "S")
@@ -505,7 +505,7 @@ def build_rfft_leaf(n: int):
 
 
 def build_cfft(n: int):
-    """Four-step stage 2: scaled complex FFT of length n (S variant) and its transpose."""
+    """Stage 2 of a split line: scaled complex FFT of length n (S variant) and its transpose."""
     g = Graph()
     zs = [(g.inp(2 * i), g.inp(2 * i + 1)) for i in range(n)]
     z = cfft(g, zs, "S")
@@ -519,30 +519,6 @@ def build_cfft(n: int):
     return (g, outs), (gt, back)
 
 
-def build_cfft_half(n: int, half: int):
-    """One radix-2 DIF half of a complex FFT of length n (G = 32 stage-2 columns split across
-    two lanes): half 0 gives V(2m), half 1 gives V(2m+1), m = 0..n/2-1, each scaled by
-    1/s(n/2, m) (an SJ scaled FFT of length n/2 on the folded inputs)."""
-    m = n // 2
-
-    def prog(g, zs):
-        if half == 0:
-            folded = [g.cadd(zs[b], zs[b + m]) for b in range(m)]
-        else:
-            folded = [g.cmulc(g.csub(zs[b], zs[b + m]),
-                              complex(math.cos(2 * math.pi * b / n), -math.sin(2 * math.pi * b / n)))
-                      for b in range(m)]
-        z = cfft(g, folded, "S")
-        return [c for k in range(m) for c in z[k]]
-    g = Graph()
-    outs = prog(g, [(g.inp(2 * i), g.inp(2 * i + 1)) for i in range(n)])
-    gt = Graph()
-    outs_t = prog(gt, [(gt.inp(n + 2 * i), gt.inp(n + 2 * i + 1)) for i in range(n)])
-    adj = [gt.inp(i) for i in range(n)]
-    back = transpose(gt, outs_t, 3 * n, adj)[n:]
-    return (g, outs), (gt, back)
-
-
 def generate() -> str:
     parts = [
         "// Generated by gen_sj.py: Shao-Johnson scaled split-radix arithmetic (straight line).",
@@ -550,7 +526,7 @@ def generate() -> str:
         "#pragma once",
         "",
     ]
-    for n in REG_SIZES:
+    for n in SCALAR_LINES:
         (g, fwd), (gi, inv), (gr, rt) = build_line_ops(n)
         ins = [f"v[{i}]" for i in range(n)]
         outs = [f"v[{i}]" for i in range(n)]
@@ -562,38 +538,6 @@ def generate() -> str:
             parts.append(emit_function(gg, nm, in_names, o, outs, "float (&v)[%d]" % n,
                                        f"{kind}, length {n}: {ops['add']} add/sub, {ops['mul']} mul"))
             parts.append("")
-    (g, outs), (gt, back) = build_rfft_leaf(LEAF)
-    m = len(outs)
-    parts.append(emit_function(g, f"sj_rfft_{LEAF}", [f"x[{i}]" for i in range(LEAF)], outs,
-                               [f"w[{i}]" for i in range(m)],
-                               f"const float (&x)[{LEAF}], float (&w)[{m}]",
-                               f"scaled real FFT, length {LEAF}: w = re[0..{LEAF//2}], im[1..{LEAF//2-1}]"))
-    parts.append("")
-    parts.append(emit_function(gt, f"sj_rfft_{LEAF}_t", [f"w[{i}]" for i in range(m)] + ["0.0f"] * LEAF,
-                               back, [f"x[{i}]" for i in range(LEAF)],
-                               f"const float (&w)[{m}], float (&x)[{LEAF}]",
-                               f"transpose of sj_rfft_{LEAF}"))
-    parts.append("")
-    for half in (0, 1):
-        (g, outs), (gt, back) = build_cfft_half(32, half)
-        parts.append(emit_function(g, f"sj_cfft_32_half{half}", [f"z[{i}]" for i in range(64)], outs,
-                                   [f"o[{i}]" for i in range(32)], "const float (&z)[64], float (&o)[32]",
-                                   f"DIF half {half} of the complex FFT of length 32"))
-        parts.append("")
-        parts.append(emit_function(gt, f"sj_cfft_32_half{half}_t", [f"o[{i}]" for i in range(32)] + ["0.0f"] * 64,
-                                   back, [f"z[{i}]" for i in range(64)], "const float (&o)[32], float (&z)[64]",
-                                   f"transpose of sj_cfft_32_half{half}"))
-        parts.append("")
-    for n in STAGE2_SIZES:
-        (g, outs), (gt, back) = build_cfft(n)
-        parts.append(emit_function(g, f"sj_cfft_{n}", [f"z[{i}]" for i in range(2 * n)], outs,
-                                   [f"z[{i}]" for i in range(2 * n)], f"float (&z)[{2 * n}]",
-                                   f"scaled complex FFT (S variant), length {n}, interleaved re/im"))
-        parts.append("")
-        parts.append(emit_function(gt, f"sj_cfft_{n}_t", [f"z[{i}]" for i in range(2 * n)] + ["0.0f"] * (2 * n),
-                                   back, [f"z[{i}]" for i in range(2 * n)], f"float (&z)[{2 * n}]",
-                                   f"transpose of sj_cfft_{n}"))
-        parts.append("")
     return "\n".join(parts)
 
 
@@ -604,7 +548,7 @@ def generate() -> str:
 # ----------------------------------------------------------------------------------------
 
 PACKED_LINES = (8, 16, 32, 64)      # whole lines in registers
-PACKED_LEAVES = (16, 32, 64)            # stage 1 of a split line: real FFT over the A samples of one residue
+PACKED_LEAVES = (16, 32, 64)        # stage 1 of a split line: real FFT over the A samples of one residue
 PACKED_STAGE2 = (8, 16)             # stage 2: complex FFT over the B residues of one column
 
 
@@ -790,27 +734,17 @@ def self_check() -> None:
         aty = gt.evaluate(back, np.concatenate([yv, np.zeros((2 * n, 1))]))
         assert abs(ax @ yv[:, 0] - flat[:, 0] @ aty[:, 0]) < 1e-9
         print(f"cfft N={n}: ops {g.count_ops(outs)}")
-    for half in (0, 1):
-        (g, outs), (gt, back) = build_cfft_half(32, half)
-        z = rng.standard_normal(32) + 1j * rng.standard_normal(32)
-        flat = np.stack([z.real, z.imag], 1).reshape(-1, 1)
-        got = g.evaluate(outs, flat).reshape(16, 2)
-        f = np.fft.fft(z)[half::2] / np.array([sj_scale(16, k) for k in range(16)])
-        assert np.abs(got[:, 0] + 1j * got[:, 1] - f).max() < 1e-10
-        yv = rng.standard_normal((32, 1))
-        aty = gt.evaluate(back, np.concatenate([yv, np.zeros((64, 1))]))
-        assert abs(got.reshape(-1) @ yv[:, 0] - flat[:, 0] @ aty[:, 0]) < 1e-9
-        print(f"cfft32 half {half}: ops {g.count_ops(outs)}")
-    (g, outs), (gt, back) = build_rfft_leaf(LEAF)
-    x = rng.standard_normal((LEAF, 1))
-    got = g.evaluate(outs, x)[:, 0]
-    f = np.fft.rfft(x[:, 0]) / np.array([sj_scale(LEAF, k) for k in range(LEAF // 2 + 1)])
-    want = np.concatenate([f.real, f.imag[1:-1]])
-    assert np.abs(got - want).max() < 1e-10
-    yv = rng.standard_normal((len(outs), 1))
-    aty = gt.evaluate(back, np.concatenate([yv, np.zeros((LEAF, 1))]))
-    assert abs(got @ yv[:, 0] - x[:, 0] @ aty[:, 0]) < 1e-9
-    print(f"rfft leaf {LEAF}: ops {g.count_ops(outs)}")
+    for n in PACKED_LEAVES:
+        (g, outs), (gt, back) = build_rfft_leaf(n)
+        x = rng.standard_normal((n, 1))
+        got = g.evaluate(outs, x)[:, 0]
+        f = np.fft.rfft(x[:, 0]) / np.array([sj_scale(n, k) for k in range(n // 2 + 1)])
+        want = np.concatenate([f.real, f.imag[1:-1]])
+        assert np.abs(got - want).max() < 1e-10
+        yv = rng.standard_normal((len(outs), 1))
+        aty = gt.evaluate(back, np.concatenate([yv, np.zeros((n, 1))]))
+        assert abs(got @ yv[:, 0] - x[:, 0] @ aty[:, 0]) < 1e-9
+        print(f"rfft leaf {n}: ops {g.count_ops(outs)}")
     print("OK")
 
 

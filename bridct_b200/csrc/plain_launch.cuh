@@ -223,7 +223,7 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
     // One column launch and one row launch over the whole batch.
     cudaError_t e;
     if constexpr (H >= 128) {
-      e = launch_split_cols<H, W, MODE, GEN>(x, y, batch, lx, ly, tab.scol, ctx, st);
+      e = launch_split_cols<H, W, MODE, GEN>(x, y, batch, lx, ly, tab.col, ctx, st);
     } else {
       using Geo = PairColGeo<H>;
       e = launch_split(k_pair_cols<H, MODE, GEN>, 0, Geo::T, batch * (W / Geo::TC), SplitArgs{x, y, {}, W, lx, ly, nullptr},
@@ -231,7 +231,7 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
     }
     if (e != cudaSuccess) return e;
     if constexpr (W >= 128) {
-      return launch_split_rows<H, W, MODE, GEN>(y, batch, ly, tab.srow, ctx, st);
+      return launch_split_rows<H, W, MODE, GEN>(y, batch, ly, tab.row, ctx, st);
     } else {
       using Geo = PairRowGeo<W>;
       return launch_split(k_pair_rows<W, GEN ? H : 0, MODE>, Geo::kSmem, Geo::T, batch * H / Geo::RB,
@@ -261,7 +261,7 @@ cudaError_t launch_col_units(const float* x, float* y, const PassUnit* units, lo
   if constexpr (H >= 128) {
     using Geo = ColGeo<H>;
     return launch_split(k_split_cols<H, 0, MODE, col_pairs<H>()>, Geo::kSmem, Geo::T, n,
-                        SplitArgs{x, y, tab.scol, 0, BatchLayout{}, BatchLayout{}, units}, st);
+                        SplitArgs{x, y, tab.col, 0, BatchLayout{}, BatchLayout{}, units}, st);
   } else {
     using Geo = PairColGeo<H>;
     return launch_split(k_pair_cols<H, MODE, true>, 0, Geo::T, n,
@@ -275,7 +275,7 @@ cudaError_t launch_row_units(const float* x, float* y, const PassUnit* units, lo
   if constexpr (W >= 128) {
     using Geo = RowGeo<W>;
     return launch_split(k_split_rows<W, W, MODE, 8>, Geo::kSmem, Geo::T, n,
-                        SplitArgs{x, y, tab.srow, 0, BatchLayout{}, BatchLayout{}, units}, st);
+                        SplitArgs{x, y, tab.row, 0, BatchLayout{}, BatchLayout{}, units}, st);
   } else {
     using Geo = PairRowGeo<W>;
     return launch_split(k_pair_rows<W, W, MODE>, Geo::kSmem, Geo::T, n,

@@ -70,8 +70,7 @@ int lg(int n) {
   return k;
 }
 
-// Four-step lines of length n are processed LPW = 1024/n at a time by one warp, so a unit must
-// hold a multiple of that many lines (1 for register lines).
+// Smallest number of lines of a unit (1 for register lines).
 int lines_per_warp(int n) { return n >= 128 ? 1024 / n : 1; }
 
 int pow2_floor(int v) {
@@ -80,17 +79,29 @@ int pow2_floor(int v) {
   return p;
 }
 
-// Columns per strip: a power of two dividing w, >= 4 (float4 rows), >= the four-step group,
+// Columns per strip: a power of two dividing w, >= 4 (float4 rows), >= lines_per_warp(h),
 // and h * columns <= budget unless the minimum forces more.
 int strip_cols(int h, int w, int budget) {
   const int want = pow2_floor(std::max(1, std::min(w, budget / h)));
   return std::min(w, std::max(want, std::max(4, lines_per_warp(h))));
 }
 
-// Rows per row block: a power of two dividing h, >= the four-step group.
+// Rows per row block: a power of two dividing h, >= lines_per_warp(w).
 int block_rows(int h, int w, int budget) {
   const int want = pow2_floor(std::max(1, std::min(h, budget / w)));
   return std::min(h, std::max(want, lines_per_warp(w)));
+}
+
+// Queue order of items a and b: large arrays first (the small ones fill the tail), arrays of one shape
+// and mode together, so that the CTAs of an SM run the same few line programs at a time (in submission
+// order the kernel spent a third of its time waiting for instructions).
+bool queue_before(const bridct_ragged_item* items, int a, int b) {
+  const bridct_ragged_item &p = items[a], &q = items[b];
+  const long long ep = (long long)p.height * p.width, eq = (long long)q.height * q.width;
+  if (ep != eq) return ep > eq;
+  if (p.height != q.height) return p.height > q.height;
+  if (p.mode != q.mode) return p.mode < q.mode;
+  return a < b;
 }
 
 void build_units(bridct_ragged* r) {
@@ -115,13 +126,9 @@ void build_units(bridct_ragged* r) {
     }
     r->arrays.push_back(a);
   }
-  auto size_desc = [&](int a, int b) {
-    const long long ea = (long long)r->items[a].height * r->items[a].width;
-    const long long eb = (long long)r->items[b].height * r->items[b].width;
-    return ea != eb ? ea > eb : a < b;
-  };
-  std::stable_sort(big.begin(), big.end(), size_desc);
-  std::stable_sort(small.begin(), small.end(), size_desc);
+  auto order = [&](int a, int b) { return queue_before(r->items.data(), a, b); };
+  std::sort(big.begin(), big.end(), order);
+  std::sort(small.begin(), small.end(), order);
   r->units.clear();
   auto cols = [&](int i) {
     const RaggedArray& a = r->arrays[i];
@@ -439,7 +446,7 @@ BRIDCT_API int bridct_ragged_apply_device(bridct_ragged* r, const float* x, floa
     args.done = r->d_counters + 1;
     args.err = r->d_err;
     args.spin_limit = r->spin_limit;
-    for (int i = 0; i < 4; ++i) args.tab[i] = r->dev->fourstep[i];
+    for (int i = 0; i < 4; ++i) args.tab[i] = r->dev->split[i];
     k_ragged<<<r->grid, kRaggedThreads, kRaggedSmem, st>>>(args);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "k_ragged launch");
@@ -574,30 +581,26 @@ BRIDCT_API int bridct_ragged_apply_loop_device(bridct_ragged* r, const float* x,
 // not acceptable, or an embedding that fixes the process's device footprint at start-up.
 // bridct_ragged_apply_noalloc serves them: the caller passes the item list and the input and
 // output buffers, and everything else the persistent kernel needs (work queue, per-array
-// counters, error word, four-step tables) lives in one statically sized __device__ array below,
+// counters, error word, split-line tables) lives in one statically sized __device__ array below,
 // which every GPU that loads this library holds until the process exits.  The host side builds
 // the queue in static buffers as well, so a successful call allocates nothing.
 namespace {
 
 constexpr int kNaMaxArrays = 4096;    // items per call
 constexpr int kNaMaxUnits = 49152;    // work units per call (default unit geometry)
-constexpr int kNaTw = 17 * (4 + 8 + 16 + 32);     // float2 twiddles, N = 128..1024
-constexpr int kNaPost = 17 * (4 + 8 + 16 + 32);   // float4 post coefficients, N = 128..1024
 
 struct NaOff {
   static constexpr size_t arrays = 0;
   static constexpr size_t units = arrays + sizeof(bridct::RaggedArray) * kNaMaxArrays;
   static constexpr size_t counters = units + sizeof(bridct::RaggedUnit) * kNaMaxUnits;
   static constexpr size_t err = counters + sizeof(unsigned int) * (kNaMaxArrays + 1);
-  static constexpr size_t tw = (err + sizeof(int) + 255) / 256 * 256;
-  static constexpr size_t post = tw + sizeof(float2) * kNaTw;
-  static constexpr size_t bytes = post + sizeof(float4) * kNaPost;
+  static constexpr size_t tabs = (err + sizeof(int) + 255) / 256 * 256;   // split-line tables, N = 128..1024
+  static constexpr size_t bytes = tabs + sizeof(float) * bridct::kRaggedTabs;
 };
-static_assert(NaOff::post % 16 == 0, "post table alignment");
 
 }  // namespace
 
-// About 0.9 MB: queue (arrays, units), counters, error word, four-step tables.  Host code must
+// About 0.9 MB: queue (arrays, units), counters, error word, split-line tables.  Host code must
 // not use this name as a device address; the entry point resolves it per device below.
 static __device__ __align__(256) unsigned char g_ragged_scratch[NaOff::bytes];
 
@@ -609,12 +612,13 @@ bridct::RaggedUnit g_na_units[kNaMaxUnits];
 int g_na_big[kNaMaxArrays];
 int g_na_small[kNaMaxArrays];
 int g_na_order[kNaMaxArrays];
-float2 g_na_tw[kNaTw];
-float4 g_na_post[kNaPost];
-bool g_na_tables = false;
+std::vector<float> g_na_tabs;
 unsigned char* g_na_addr[64] = {};                      // scratch address per device
 
-int na_segment(int i) { return 17 * ((4 << i) - 4); }  // first entry of N = 128 << i
+// First float of the tables of N = 128 << i.
+size_t na_segment(int i) {
+  return i == 0 ? 0 : i == 1 ? bridct::ragged_tab<256>() : i == 2 ? bridct::ragged_tab<512>() : bridct::ragged_tab<1024>();
+}
 
 }  // namespace
 
@@ -667,13 +671,9 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
     }
     g_na_arrays[i] = a;
   }
-  auto size_desc = [&](int a, int b) {
-    const long long ea = (long long)items[a].height * items[a].width;
-    const long long eb = (long long)items[b].height * items[b].width;
-    return ea != eb ? ea > eb : a < b;
-  };
-  std::sort(g_na_big, g_na_big + nbig, size_desc);
-  std::sort(g_na_small, g_na_small + nsmall, size_desc);
+  auto order = [&](int a, int b) { return queue_before(items, a, b); };
+  std::sort(g_na_big, g_na_big + nbig, order);
+  std::sort(g_na_small, g_na_small + nsmall, order);
   int nunits = 0;
   bool full = false;
   auto push = [&](RaggedUnit u) {
@@ -700,7 +700,7 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
   }
 
   // set-up, once per device, with that device current: resolve the scratch array's device
-  // address (the host-side name is only a stand-in) and upload the four-step tables into it
+  // address (the host-side name is only a stand-in) and upload the split-line tables into it
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
@@ -708,17 +708,17 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
     set_error("bridct_ragged_apply_noalloc: device index beyond 63");
     return BRIDCT_INVALID_ARGUMENT;
   }
-  if (!g_na_tables) {
-    for (int i = 0; i < 4; ++i) fill_fourstep_tables(128 << i, g_na_tw + na_segment(i), g_na_post + na_segment(i));
-    g_na_tables = true;
-  }
+  if (g_na_tabs.empty())
+    for (int i = 0; i < 4; ++i) {
+      const std::vector<float> t = split_tables_host(128 << i);
+      g_na_tabs.insert(g_na_tabs.end(), t.begin(), t.end());
+    }
   if (!g_na_addr[dev]) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_ragged_scratch);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_ragged_scratch)");
     unsigned char* base = static_cast<unsigned char*>(p);
-    e = cudaMemcpy(base + NaOff::tw, g_na_tw, sizeof(g_na_tw), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(base + NaOff::post, g_na_post, sizeof(g_na_post), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(base + NaOff::tabs, g_na_tabs.data(), g_na_tabs.size() * sizeof(float), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "scratch tables");
     g_na_addr[dev] = base;
   }
@@ -746,10 +746,7 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
   args.done = args.next + 1;
   args.err = reinterpret_cast<int*>(base + NaOff::err);
   args.spin_limit = kRaggedSpin;
-  for (int i = 0; i < 4; ++i) {
-    args.tab[i].tw = reinterpret_cast<const float2*>(base + NaOff::tw) + na_segment(i);
-    args.tab[i].post = reinterpret_cast<const float4*>(base + NaOff::post) + na_segment(i);
-  }
+  for (int i = 0; i < 4; ++i) args.tab[i].t = reinterpret_cast<const float*>(base + NaOff::tabs) + na_segment(i);
   const int grid = (int)std::min<long long>((long long)sms * bps, nunits);
   k_ragged<<<grid, kRaggedThreads, kRaggedSmem, st>>>(args);
   e = cudaGetLastError();

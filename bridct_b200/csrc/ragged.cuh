@@ -1,19 +1,25 @@
 // Batching form: one persistent launch over a mixed-shape, mixed-direction batch.
 //
 // The host turns the batch into a queue of work units:
-//   TILE      one array with h*w <= 16384: both passes in shared memory (as k_full)
-//   COLSTRIP  h rows x TC columns of a larger array: its column lines, x -> y
-//   ROWBLOCK  RB full rows of a larger array: its row lines, y -> y in place
+//   TILE      one array up to the tuning's tile_floats: both passes
+//   COLSTRIP  h rows x some columns of a larger array: its column lines, x -> y
+//   ROWBLOCK  some full rows of a larger array: its row lines, y -> y in place
 // CTAs are persistent (one launch, grid = SMs x resident CTAs) and take units in queue order
 // from an atomic counter.  A ROWBLOCK of array i needs every COLSTRIP of array i finished: each
 // strip adds 1 to done[i] after a __threadfence, and the row block spins on done[i] with a
 // bounded budget (nanosleep back-off).  Column strips never wait, and every unit that a waiting
 // row block depends on was dequeued earlier by a running CTA, so the wait always ends; on budget
 // expiry the unit is skipped and the error flag set instead (the host reports BRIDCT_TIMEOUT).
-// Line lengths and modes vary per unit and are dispatched at run time to the same generated
-// straight-line SJ programs and four-step lines as the fixed-shape kernels.
+//
+// Line lengths and modes vary per unit and are dispatched at run time to the line pairs of the
+// fixed-shape kernels (sj_split.cuh).  A unit is worked through in sub-blocks of at most 9216 floats of
+// shared memory, so that three CTAs of 128 threads (168 registers: 64-point leaves, two lines per thread)
+// share an SM together with the tables of all four split lengths.  An array whose tile does not fit
+// takes its two passes through y, which stays in L2.  1024 mixed arrays up to 1024 x 1024: 590 us with
+// one line per thread or line group per warp in 256-thread CTAs of 112 KB, QUEUE_US this way.
 #pragma once
 #include "sj_kernels.cuh"
+#include "sj_split.cuh"
 
 namespace bridct {
 
@@ -42,151 +48,279 @@ struct RaggedArgs {
   unsigned int* done;       // finished column strips per array (zeroed before the launch)
   int* err;
   unsigned spin_limit;      // polls of a row block's dependency wait before it gives up
-  FourStepTables tab[4];    // N = 128, 256, 512, 1024
+  SplitTables tab[4];       // N = 128, 256, 512, 1024
 };
 
-constexpr int kRaggedThreads = 256;                                 // 2 CTAs per SM at <= 128 registers
-// Exchange floats per warp, worst case over the four-step widths G = 4..32 (G = 4 and 8 need
-// most: 8 slots of 84 or 4 slots of 168 floats, re and im).
-constexpr int kXbufPerWarp = cmax(cmax(FourStepSizes<4>::FLOATS, FourStepSizes<8>::FLOATS),
-                                  cmax(FourStepSizes<16>::FLOATS, FourStepSizes<32>::FLOATS));
-constexpr int kRaggedXbuf = (kRaggedThreads / 32) * kXbufPerWarp;
-constexpr int kRaggedTile = 16384 + 1024;                           // worst-case tile floats (odd pitch)
-constexpr int kRaggedSmem = (kRaggedTile + kRaggedXbuf) * 4;
+constexpr int kRaggedThreads = 128;
+constexpr int kRaggedTile = 9216;                                   // floats of a sub-block
+constexpr int kRaggedTabs = SplitTab<128>::kFloats + SplitTab<256>::kFloats + SplitTab<512>::kFloats + SplitTab<1024>::kFloats;
+constexpr int kRaggedSmem = (kRaggedTile + kRaggedTabs) * 4;
 constexpr unsigned kRaggedSpin = 1u << 22;                          // x ~256 ns back-off
 
-// Line l of a unit starts at tile + l * s (s = 1 for columns, the pitch for rows).
-struct StrideOff {
-  int s;
-  __device__ __forceinline__ int operator()(int l) const { return l * s; }
-};
-
-__device__ __forceinline__ FourStepTables pick_tables(const RaggedArgs& a, int n) {
-  return n >= 1024 ? a.tab[3] : n >= 512 ? a.tab[2] : n >= 256 ? a.tab[1] : a.tab[0];
+// Offset (floats) of the tables of length N among the staged ones.
+template <int N> __host__ __device__ constexpr int ragged_tab() {
+  return N <= 128   ? 0
+         : N == 256 ? SplitTab<128>::kFloats
+         : N == 512 ? SplitTab<128>::kFloats + SplitTab<256>::kFloats
+                    : SplitTab<128>::kFloats + SplitTab<256>::kFloats + SplitTab<512>::kFloats;
 }
 
-// Runtime dispatch of run_lines over the line length and mode.
-__device__ __forceinline__ void lines_dyn(int n, int mode, float* tile, int nlines, int es, StrideOff off,
-                                       float* xbuf, FourStepTables t) {
-#define BRIDCT_LINES_N(N)                                                          \
-  case N:                                                                          \
-    if (mode == LM_FWD) run_lines<N, LM_FWD>(tile, nlines, es, off, xbuf, t);      \
-    else if (mode == LM_INV) run_lines<N, LM_INV>(tile, nlines, es, off, xbuf, t); \
-    else run_lines<N, LM_RT>(tile, nlines, es, off, xbuf, t);                      \
-    break;
-  switch (n) {
-    BRIDCT_LINES_N(8)
-    BRIDCT_LINES_N(16)
-    BRIDCT_LINES_N(32)
-    BRIDCT_LINES_N(64)
-    BRIDCT_LINES_N(128)
-    BRIDCT_LINES_N(256)
-    BRIDCT_LINES_N(512)
-    BRIDCT_LINES_N(1024)
-    default: break;
-  }
-#undef BRIDCT_LINES_N
-}
+// Line pairs of a group: strips of 8 columns and blocks of 8 rows for 1024-point lines.
+template <int N> __host__ __device__ constexpr int ragged_col_pairs() { return N == 1024 ? 4 : N == 512 ? 8 : 16; }
+template <int N> __host__ __device__ constexpr int ragged_row_pairs() { return N == 1024 ? 4 : 8; }
+// Row pitch in shared memory (32 / pairs modulo 32 floats for split rows).
+__host__ __device__ constexpr int ragged_pitch(int w) { return w == 1024 ? w + 8 : w + 4; }
+// Whether an array's two passes run in one shared-memory tile.
+__host__ __device__ constexpr bool ragged_fits(int h, int w) { return h <= 256 && h * ragged_pitch(w) <= kRaggedTile; }
 
-// Shared-memory pitch of a unit's block (rows x cols): aligned (cols + 4, float4 staging)
-// unless a column pass of 512- or 1024-point lines runs on it (their four-step groups put
-// every lane in one bank at an aligned pitch) or the aligned block would not fit the tile.
-__device__ __forceinline__ int ragged_pitch(int rows, int cols, bool column_pass, int h) {
-  if ((column_pass && h >= 512) || rows * (cols + 4) > kRaggedTile) return cols + 1;
-  return cols + 4;
-}
-
-// Loads rows x cols floats (row pitch gp in global) into shared memory (pitch P).  The copies are
-// asynchronous (cp.async), so a thread has all of its share of the block in flight at once; the
-// caller's __syncthreads after this call publishes the block.  An odd-pitch block copies 4-byte
-// elements (its rows are not 16-byte aligned), except when it must bypass L1 (row blocks read data
-// that other CTAs wrote in this launch; 4-byte cp.async always goes through L1), where it loads
-// through L2 synchronously.
-__device__ __forceinline__ void load_block(const float* g, long long gp, int rows, int cols, float* s, int P,
-                                           bool bypass_l1) {
-  const int q = cols >> 2;
-  const bool vec = (P & 3) == 0;
-  if (vec || !bypass_l1) {
-    for (int i = threadIdx.x; i < rows * q; i += blockDim.x) {
-      const int r = i / q, c = (i % q) * 4;
-      const float* src = g + r * gp + c;
-      float* d = s + r * P + c;
-      if (vec) {
-        cp_async16(d, src);
-      } else {
-        cp_async4(d, src);
-        cp_async4(d + 1, src + 1);
-        cp_async4(d + 2, src + 2);
-        cp_async4(d + 3, src + 3);
+// Columns of length H, x -> y, rows ld floats apart in both.
+template <int H, int MODE>
+__device__ __forceinline__ void ragged_cols(const float* x, float* y, int ld, int ncols, float* tile,
+                                            const float* tabs) {
+  if constexpr (H <= 64) {
+    for (int p = threadIdx.x; p < ncols / 2; p += kRaggedThreads) {
+      F2 v[H];
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const float2 f = __ldg(reinterpret_cast<const float2*>(x + (long long)i * ld) + p);
+        v[i] = f2_make(f.x, f.y);
+      }
+      pair_line<H, MODE>(v);
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        float2 f;
+        f2_split(v[i], f.x, f.y);
+        reinterpret_cast<float2*>(y + (long long)i * ld)[p] = f;
       }
     }
-    cp_async_wait_all();
-    return;
-  }
-  for (int i = threadIdx.x; i < rows * q; i += blockDim.x) {
-    const int r = i / q, c = (i % q) * 4;
-    const float4* p = reinterpret_cast<const float4*>(g + r * gp + c);
-    const float4 v = bypass_l1 ? __ldcg(p) : __ldg(p);
-    float* d = s + r * P + c;
-    if (vec) {
-      *reinterpret_cast<float4*>(d) = v;
-    } else {
-      d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+  } else {
+    constexpr int LP = ragged_col_pairs<H>(), TC = 2 * LP;
+    for (int c0 = 0; c0 < ncols; c0 += TC) {
+      const int nc = ncols - c0 < TC ? ncols - c0 : TC, q = nc >> 2;   // a power of two, at least 4 columns
+      const int sh = 31 - __clz(q);
+      for (int i = threadIdx.x; i < H * q; i += kRaggedThreads) {
+        const int r = i >> sh, c = (i & (q - 1)) << 2;
+        cp_async16(tile + strip_row<TC>(r) + c, x + (long long)r * ld + c0 + c);
+      }
+      cp_async_wait_all();
+      __syncthreads();
+      const int p = 2 * (threadIdx.x % LP);
+      float* yt = y + c0 + p;
+      split_lines<H, MODE, kRaggedThreads, 1, LP, false>(
+          [&](int, int i) {
+            const float2 v = *reinterpret_cast<const float2*>(tile + strip_row<TC>(i) + p);
+            return f2_make(v.x, v.y);
+          },
+          [&](int, int i, F2 v) {
+            float2 f;
+            f2_split(v, f.x, f.y);
+            *reinterpret_cast<float2*>(yt + (long long)i * ld) = f;
+          },
+          [&](int) { return tile + p; }, TC, tabs + ragged_tab<H>(), [&](int) { return p < nc; });
+      __syncthreads();
     }
   }
 }
 
-__device__ __forceinline__ void store_block(float* g, long long gp, int rows, int cols, const float* s, int P) {
-  const int q = cols >> 2;
-  const bool vec = (P & 3) == 0;
-  for (int i = threadIdx.x; i < rows * q; i += blockDim.x) {
-    const int r = i / q, c = (i % q) * 4;
-    const float* v = s + r * P + c;
-    *reinterpret_cast<float4*>(g + r * gp + c) =
-        vec ? *reinterpret_cast<const float4*>(v) : make_float4(v[0], v[1], v[2], v[3]);
+// Columns of an array that lies in shared memory whole, rows P floats apart (H <= 256).
+template <int H, int MODE>
+__device__ __forceinline__ void ragged_tile_cols(float* tile, int P, int w, const float* tabs) {
+  if constexpr (H <= 64) {
+    for (int p = threadIdx.x; p < w / 2; p += kRaggedThreads) {
+      F2 v[H];
+#pragma unroll
+      for (int i = 0; i < H; ++i) v[i] = *reinterpret_cast<const F2*>(tile + i * P + 2 * p);
+      pair_line<H, MODE>(v);
+#pragma unroll
+      for (int i = 0; i < H; ++i) *reinterpret_cast<F2*>(tile + i * P + 2 * p) = v[i];
+    }
+  } else {
+    for (int c0 = 0; c0 < w; c0 += 32) {
+      const int p = c0 + 2 * (threadIdx.x % 16);
+      split_lines<H, MODE, kRaggedThreads, 1, 16, true>(
+          [&](int, int i) { return *reinterpret_cast<const F2*>(tile + i * P + p); },
+          [&](int, int i, F2 v) { *reinterpret_cast<F2*>(tile + i * P + p) = v; }, [&](int) { return tile + p; }, P,
+          tabs + ragged_tab<H>(), [&](int) { return p < w; });
+    }
+  }
+  __syncthreads();
+}
+
+// nr rows of length W in shared memory, in place.  Split rows: up to the rows of one sub-block; the
+// second row of a pair may lie beyond nr (its values are not stored).
+template <int W, int MODE>
+__device__ __forceinline__ void ragged_rows(float* tile, int nr, const float* tabs) {
+  constexpr int P = ragged_pitch(W);
+  if constexpr (W <= 64) {
+    for (int l = threadIdx.x; l < (nr + 15) / 16 * 8; l += kRaggedThreads) {
+      const int r = (l / 8) * 16 + l % 8;
+      if (r < nr) pair_rows<W, MODE>(tile + r * P, tile + (r + 8 < nr ? r + 8 : r) * P);
+    }
+  } else {
+    constexpr int LP = ragged_row_pairs<W>(), GROUPS = W <= 256 ? 2 : 1, GP = 2 * LP * P;
+    const int p = threadIdx.x % LP;
+    float* rows = tile + p * P;
+    split_lines<W, MODE, kRaggedThreads, GROUPS, LP, true>(
+        [&](int g, int i) { return f2_make(rows[g * GP + i], rows[g * GP + i + LP * P]); },
+        [&](int g, int i, F2 v) { f2_split(v, rows[g * GP + i], rows[g * GP + i + LP * P]); },
+        [&](int g) { return tile + g * GP + 2 * p; }, 2 * LP, tabs + ragged_tab<W>(),
+        [&](int g) { return g * 2 * LP + p < nr; });
+  }
+  fence_async();
+  __syncthreads();
+}
+
+// Run-time dispatch of F<N, MODE>(...) over the line length and mode.
+#define BRIDCT_RAGGED_CASE(F, N, ...)                       \
+  case N:                                                   \
+    if (mode == LM_FWD) F<N, LM_FWD>(__VA_ARGS__);          \
+    else if (mode == LM_INV) F<N, LM_INV>(__VA_ARGS__);     \
+    else F<N, LM_RT>(__VA_ARGS__);                          \
+    break;
+
+__device__ __forceinline__ void ragged_cols_dyn(int h, int mode, const float* x, float* y, int ld, int ncols,
+                                                float* tile, const float* tabs) {
+  switch (h) {
+    BRIDCT_RAGGED_CASE(ragged_cols, 8, x, y, ld, ncols, tile, tabs)
+    BRIDCT_RAGGED_CASE(ragged_cols, 16, x, y, ld, ncols, tile, tabs)
+    BRIDCT_RAGGED_CASE(ragged_cols, 32, x, y, ld, ncols, tile, tabs)
+    BRIDCT_RAGGED_CASE(ragged_cols, 64, x, y, ld, ncols, tile, tabs)
+    BRIDCT_RAGGED_CASE(ragged_cols, 128, x, y, ld, ncols, tile, tabs)
+    BRIDCT_RAGGED_CASE(ragged_cols, 256, x, y, ld, ncols, tile, tabs)
+    BRIDCT_RAGGED_CASE(ragged_cols, 512, x, y, ld, ncols, tile, tabs)
+    BRIDCT_RAGGED_CASE(ragged_cols, 1024, x, y, ld, ncols, tile, tabs)
+    default: break;
+  }
+}
+__device__ __forceinline__ void ragged_tile_cols_dyn(int h, int mode, float* tile, int P, int w, const float* tabs) {
+  switch (h) {
+    BRIDCT_RAGGED_CASE(ragged_tile_cols, 8, tile, P, w, tabs)
+    BRIDCT_RAGGED_CASE(ragged_tile_cols, 16, tile, P, w, tabs)
+    BRIDCT_RAGGED_CASE(ragged_tile_cols, 32, tile, P, w, tabs)
+    BRIDCT_RAGGED_CASE(ragged_tile_cols, 64, tile, P, w, tabs)
+    BRIDCT_RAGGED_CASE(ragged_tile_cols, 128, tile, P, w, tabs)
+    BRIDCT_RAGGED_CASE(ragged_tile_cols, 256, tile, P, w, tabs)
+    default: break;
+  }
+}
+__device__ __forceinline__ void ragged_rows_dyn(int w, int mode, float* tile, int nr, const float* tabs) {
+  switch (w) {
+    BRIDCT_RAGGED_CASE(ragged_rows, 8, tile, nr, tabs)
+    BRIDCT_RAGGED_CASE(ragged_rows, 16, tile, nr, tabs)
+    BRIDCT_RAGGED_CASE(ragged_rows, 32, tile, nr, tabs)
+    BRIDCT_RAGGED_CASE(ragged_rows, 64, tile, nr, tabs)
+    BRIDCT_RAGGED_CASE(ragged_rows, 128, tile, nr, tabs)
+    BRIDCT_RAGGED_CASE(ragged_rows, 256, tile, nr, tabs)
+    BRIDCT_RAGGED_CASE(ragged_rows, 512, tile, nr, tabs)
+    BRIDCT_RAGGED_CASE(ragged_rows, 1024, tile, nr, tabs)
+    default: break;
+  }
+}
+#undef BRIDCT_RAGGED_CASE
+
+// Rows of one sub-block: what the threads have split-row tasks for, or 128 register rows.
+__device__ __forceinline__ int ragged_block_rows(int w) { return w <= 64 ? 128 : w <= 256 ? 32 : w == 512 ? 16 : 8; }
+
+// `rows` rows of width w to shared memory, pitch P, bypassing L1 (row blocks read data that other
+// CTAs, or other threads of this one, wrote in this launch).
+__device__ __forceinline__ void ragged_load(const float* g, int rows, int w, float* tile, int P) {
+  const int sh = 29 - __clz(w);   // log2(w / 4)
+  for (int i = threadIdx.x; i < rows << sh; i += kRaggedThreads) {
+    const int r = i >> sh, c = (i & ((1 << sh) - 1)) << 2;
+    cp_async16(tile + r * P + c, g + 4ll * i);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+}
+
+// The row lines of `rows` rows of width w at g; loaded: they already lie in the tile.
+__device__ __forceinline__ void ragged_row_pass(float* g, int rows, int w, int mode, bool loaded, float* tile,
+                                                const float* tabs) {
+  const int P = ragged_pitch(w), step = ragged_block_rows(w), sh = 29 - __clz(w);
+  for (int r0 = 0; r0 < rows; r0 += step) {
+    const int nr = rows - r0 < step ? rows - r0 : step;
+    float* t = loaded ? tile + r0 * P : tile;
+    float* gr = g + (long long)r0 * w;
+    if (!loaded) ragged_load(gr, nr, w, tile, P);
+    ragged_rows_dyn(w, mode, t, nr, tabs);
+    if (w >= 128) {
+      if (threadIdx.x < nr) {
+        bulk_store(gr + (long long)threadIdx.x * w, t + threadIdx.x * P, w * 4);
+        bulk_commit_wait();
+      }
+    } else {
+      for (int i = threadIdx.x; i < nr << sh; i += kRaggedThreads)
+        *reinterpret_cast<float4*>(gr + 4 * i) =
+            *reinterpret_cast<const float4*>(t + (i >> sh) * P + ((i & ((1 << sh) - 1)) << 2));
+    }
+    __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(kRaggedThreads, 2) k_ragged(RaggedArgs a) {
+__global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged(RaggedArgs a) {
   extern __shared__ float smem[];
   float* tile = smem;
-  float* xbuf = smem + kRaggedTile;
-  __shared__ int s_unit;
+  float* tabs = smem + kRaggedTile;
+  __shared__ int s_index;
+  __shared__ RaggedUnit s_unit;
+  __shared__ RaggedArray s_array;
   __shared__ int s_ok;
+  split_stage_tables<128, kRaggedThreads>(a.tab[0], tabs + ragged_tab<128>());
+  split_stage_tables<256, kRaggedThreads>(a.tab[1], tabs + ragged_tab<256>());
+  split_stage_tables<512, kRaggedThreads>(a.tab[2], tabs + ragged_tab<512>());
+  split_stage_tables<1024, kRaggedThreads>(a.tab[3], tabs + ragged_tab<1024>());
+  cp_async_wait_all();
+  // Thread 0 takes the next unit while the CTA works on the current one, as long as the queue is long
+  // enough that no CTA runs dry for it; a held unit comes after the current one in the queue, so what
+  // any row block waits for still makes progress.
+  int ahead = -1;
+  RaggedUnit next{};
   for (;;) {
-    if (threadIdx.x == 0) s_unit = (int)atomicAdd(a.next, 1u);
+    if (threadIdx.x == 0) {
+      int u = ahead;
+      if (u < 0) {
+        u = (int)atomicAdd(a.next, 1u);
+        if (u < a.nunits) next = a.units[u];
+      }
+      s_index = u;
+      if (u < a.nunits) {
+        s_unit = next;
+        s_array = a.arrays[next.array];
+      }
+    }
     __syncthreads();
-    const int u = s_unit;
+    const int u = s_index;
     if (u >= a.nunits) break;
-    const RaggedUnit unit = a.units[u];
-    const RaggedArray arr = a.arrays[unit.array];
+    const RaggedUnit unit = s_unit;
+    const RaggedArray arr = s_array;
+    if (threadIdx.x == 0) ahead = u + 4 * (int)gridDim.x < a.nunits ? (int)atomicAdd(a.next, 1u) : -1;
+    auto fetch = [&] {
+      if (threadIdx.x == 0 && ahead >= 0 && ahead < a.nunits) next = a.units[ahead];
+    };
     const int h = arr.h, w = arr.w, mode = arr.mode;
     const float* xa = a.x + arr.offset;
     float* ya = a.y + arr.offset;
-    if (unit.type == UNIT_TILE) {
-      const int P = ragged_pitch(h, w, true, h);
-      load_block(xa, w, h, w, tile, P, false);
-      __syncthreads();
-      lines_dyn(h, mode, tile, w, P, StrideOff{1}, xbuf, pick_tables(a, h));
-      __syncthreads();
-      lines_dyn(w, mode, tile, h, 1, StrideOff{P}, xbuf, pick_tables(a, w));
-      __syncthreads();
-      store_block(ya, w, h, w, tile, P);
-    } else if (unit.type == UNIT_COLSTRIP) {
-      const int tc = unit.count, P = ragged_pitch(h, tc, true, h);
-      load_block(xa + unit.first, w, h, tc, tile, P, false);
-      __syncthreads();
-      lines_dyn(h, mode, tile, tc, P, StrideOff{1}, xbuf, pick_tables(a, h));
-      __syncthreads();
-      store_block(ya + unit.first, w, h, tc, tile, P);
+    const bool fits = unit.type == UNIT_TILE && ragged_fits(h, w);
+    bool rows = unit.type != UNIT_COLSTRIP;
+    int first = 0, count = h;
+    if (fits) {
+      ragged_load(xa, h, w, tile, ragged_pitch(w));
+      ragged_tile_cols_dyn(h, mode, tile, ragged_pitch(w), w, tabs);
+      fetch();
+    } else if (unit.type != UNIT_ROWBLOCK) {
+      const int c0 = unit.type == UNIT_COLSTRIP ? unit.first : 0, nc = unit.type == UNIT_COLSTRIP ? unit.count : w;
+      ragged_cols_dyn(h, mode, xa + c0, ya + c0, w, nc, tile, tabs);
+      fetch();
       __threadfence();
       __syncthreads();
-      if (threadIdx.x == 0) atomicAdd(a.done + unit.array, 1u);
+      if (unit.type == UNIT_COLSTRIP && threadIdx.x == 0) atomicAdd(a.done + unit.array, 1u);
     } else {
       if (threadIdx.x == 0) {
         int ok = 0;
         for (unsigned i = 0; i < a.spin_limit; ++i) {
-          if (atomicAdd(a.done + unit.array, 0u) >= (unsigned)arr.nstrips) {
+          unsigned n;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(a.done + unit.array) : "memory");
+          if (n >= (unsigned)arr.nstrips) {
             ok = 1;
             break;
           }
@@ -196,17 +330,13 @@ __global__ void __launch_bounds__(kRaggedThreads, 2) k_ragged(RaggedArgs a) {
         __threadfence();
         s_ok = ok;
       }
+      fetch();
       __syncthreads();
-      if (s_ok) {
-        const int rb = unit.count, P = ragged_pitch(rb, w, false, 0);
-        float* ga = ya + (long long)unit.first * w;
-        load_block(ga, w, rb, w, tile, P, true);
-        __syncthreads();
-        lines_dyn(w, mode, tile, rb, 1, StrideOff{P}, xbuf, pick_tables(a, w));
-        __syncthreads();
-        store_block(ga, w, rb, w, tile, P);
-      }
+      rows = s_ok;
+      first = unit.first;
+      count = unit.count;
     }
+    if (rows) ragged_row_pass(ya + (long long)first * w, count, w, mode, fits, tile, tabs);
     __syncthreads();
   }
 }

@@ -19,9 +19,8 @@ struct SplitTables {
 };
 
 struct LineTables {
-  FourStepTables col;   // for line length h (used when h >= 128)
-  FourStepTables row;   // for line length w (used when w >= 128)
-  SplitTables scol, srow;
+  SplitTables col;   // for line length h (used when h >= 128)
+  SplitTables row;   // for line length w (used when w >= 128)
 };
 
 // Where the arrays of a launch live in a general layout (kernels instantiated with GEN): array b
@@ -64,36 +63,18 @@ __device__ __forceinline__ long long layout_row(const BatchLayout& l, long long 
 
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 __host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
-// Asynchronous global -> shared copies (cp.async; 16 bytes through L2 only, 4 bytes through L1).  The issuing thread waits with cp_async_wait_all; a barrier then publishes the data.
+// Asynchronous global -> shared copies (cp.async, 16 bytes, through L2 only).  The issuing thread waits with cp_async_wait_all; a barrier then publishes the data.
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
                "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
-               "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Runs all lines of length N in a set of `nlines` lines; line l starts at tile + off(l),
-// elements at stride es.  Register lines (one thread per line) for N <= REG_MAX, warp
-// four-step lines above.
-// PAIRS: rows (es = 1) at 8-byte aligned starts; the four-step moves them in 64-bit pairs.
-template <int N, int MODE, int REG_MAX = 64, bool PAIRS = false, typename Off>
-__device__ __forceinline__ void run_lines(float* tile, int nlines, int es, const Off& off,
-                                          float* xbuf, FourStepTables tab) {
-  if constexpr (N <= REG_MAX) {
-    for (int l = threadIdx.x; l < nlines; l += blockDim.x) reg_line<N, MODE>(tile + off(l), es);
-  } else {
-    constexpr int G = N / 32;
-    constexpr int LPW = 32 / G;
-    const int warp = threadIdx.x >> 5;
-    float* xb = xbuf + warp * FourStepSizes<G>::FLOATS;
-    for (int g = warp; g * LPW < nlines; g += blockDim.x >> 5) {
-      auto ptr = [&](int j) { return tile + off(g * LPW + j); };
-      fs_line<G, MODE, PAIRS>(ptr, es, xb, tab);
-    }
-  }
+// Runs `nlines` lines of length N, one thread per line; line l starts at tile + off(l), elements at
+// stride es.
+template <int N, int MODE, typename Off>
+__device__ __forceinline__ void run_lines(float* tile, int nlines, int es, const Off& off) {
+  for (int l = threadIdx.x; l < nlines; l += blockDim.x) reg_line<N, MODE>(tile + off(l), es);
 }
 
 // Tiles of whole arrays whose lines run in one thread's registers, scalar: ARR arrays of H x W, rows
@@ -122,9 +103,9 @@ __global__ void __launch_bounds__(T) k_reg_tile(TileArgs a) {
     }
     cp_async_wait_all();
     __syncthreads();
-    run_lines<H, MODE, H>(smem, ARR * W, P, [](int l) { return (l / W) * AP + (l % W); }, nullptr, FourStepTables{});
+    run_lines<H, MODE>(smem, ARR * W, P, [](int l) { return (l / W) * AP + (l % W); });
     __syncthreads();
-    run_lines<W, MODE, W>(smem, TR, 1, srow, nullptr, FourStepTables{});
+    run_lines<W, MODE>(smem, TR, 1, srow);
     __syncthreads();
     for (int i = threadIdx.x; i < rows * Q; i += T) {
       const int r = i / Q, c = (i % Q) * 4;

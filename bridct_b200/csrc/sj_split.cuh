@@ -249,9 +249,15 @@ __device__ __forceinline__ int split_src(int a, int b) {
 // floats apart.  The exchange may overlie what get() reads: a barrier lies between.  IN_PLACE: put()
 // may also overlie the exchange.
 // Slot (c, part, b) is number c * 2B + part * B + (b ^ (c % S)), S = 16 / LP: where a half-warp spans
-// several tasks c, their slots of one b then lie in different banks.
-template <int N, int MODE, int T, int GROUPS, int LP, int ES, bool IN_PLACE, typename Get, typename Put, typename Ex>
-__device__ __forceinline__ void split_lines(const Get& get, const Put& put, const Ex& ex, const float* tab) {
+// several tasks c, their slots of one b then lie in different banks.  Threads with on(g) false (pairs
+// that a short unit does not have) only take part in the barriers.
+struct AllPairs {
+  __device__ __forceinline__ bool operator()(int) const { return true; }
+};
+template <int N, int MODE, int T, int GROUPS, int LP, bool IN_PLACE, typename Get, typename Put, typename Ex,
+          typename On = AllPairs>
+__device__ __forceinline__ void split_lines(const Get& get, const Put& put, const Ex& ex, int ES, const float* tab,
+                                            const On& on = On()) {
   constexpr int A = Split<N>::A, B = Split<N>::B, S = LP < 16 ? 16 / LP : 1;
   auto at = [](float* e) -> F2& { return *reinterpret_cast<F2*>(e); };
   constexpr int N1 = GROUPS * B * LP, N2 = GROUPS * (A / 2) * LP;   // threads' tasks of the two stages
@@ -259,8 +265,8 @@ __device__ __forceinline__ void split_lines(const Get& get, const Put& put, cons
   static_assert(N1 % 32 == 0 && N2 % 32 == 0, "whole warps");
   const int t = threadIdx.x / LP;
   constexpr int TP = T / LP;
-  auto on1 = [&](int r) { return N1 % T == 0 || (int)threadIdx.x + r * T < N1; };
-  auto on2 = [&](int r) { return N2 % T == 0 || (int)threadIdx.x + r * T < N2; };
+  auto on1 = [&](int r) { return (N1 % T == 0 || (int)threadIdx.x + r * T < N1) && on((t + r * TP) / B); };
+  auto on2 = [&](int r) { return (N2 % T == 0 || (int)threadIdx.x + r * T < N2) && on((t + r * TP) / (A / 2)); };
   if constexpr (MODE != LM_INV) {
     F2 w[R1][A];
 #pragma unroll
@@ -426,7 +432,7 @@ __device__ __forceinline__ void split_col_unit(const float* x, float* y, long lo
   __syncthreads();
   const int p = 2 * (threadIdx.x % LP);
   float* yt = y + p;
-  split_lines<N, MODE, T, 1, LP, TC, false>(
+  split_lines<N, MODE, T, 1, LP, false>(
       [&](int, int i) {
         const float2 v = *reinterpret_cast<const float2*>(smem + strip_row<TC>(i) + p);
         return f2_make(v.x, v.y);
@@ -436,7 +442,7 @@ __device__ __forceinline__ void split_col_unit(const float* x, float* y, long lo
         f2_split(v, f.x, f.y);
         *reinterpret_cast<float2*>(yt + (W > 0 ? (long long)(i * W) : i * yp)) = f;
       },
-      [&](int) { return smem + p; }, tab);
+      [&](int) { return smem + p; }, TC, tab);
 }
 
 // W > 0: strips of contiguous N x W arrays; W = 0: run-time layouts, or units.
@@ -486,10 +492,10 @@ __device__ __forceinline__ void split_rows(float* tile, const float* tab) {
   constexpr int P = N + 32 / LP, GP = 2 * LP * P;
   const int p = threadIdx.x % LP;
   float* rows = tile + p * P;
-  split_lines<N, MODE, T, GROUPS, LP, 2 * LP, true>(
+  split_lines<N, MODE, T, GROUPS, LP, true>(
       [&](int g, int i) { return f2_make(rows[g * GP + i], rows[g * GP + i + LP * P]); },
       [&](int g, int i, F2 v) { f2_split(v, rows[g * GP + i], rows[g * GP + i + LP * P]); },
-      [&](int g) { return tile + g * GP + 2 * p; }, tab);
+      [&](int g) { return tile + g * GP + 2 * p; }, 2 * LP, tab);
 }
 
 // Stores `bytes` (a multiple of 16) of shared memory to global memory asynchronously.
@@ -690,8 +696,8 @@ __global__ void __launch_bounds__(T, MINB) k_pair_tile(TileArgs a) {
   extern __shared__ float smem[];
   float* tcol = smem + Geo::kTile;
   float* trow = H == W ? tcol : tcol + Geo::kTabC;
-  if constexpr (H >= 128) split_stage_tables<H, T>(a.tab.scol, tcol);
-  if constexpr (W >= 128 && W != H) split_stage_tables<W, T>(a.tab.srow, trow);
+  if constexpr (H >= 128) split_stage_tables<H, T>(a.tab.col, tcol);
+  if constexpr (W >= 128 && W != H) split_stage_tables<W, T>(a.tab.row, trow);
   griddep_wait();
   griddep_trigger();
   const long long first = (long long)blockIdx.x * TR;
@@ -714,12 +720,12 @@ __global__ void __launch_bounds__(T, MINB) k_pair_tile(TileArgs a) {
       const int c = (g * LP + p) * 2;
       return smem + c / W * AP + c % W;
     };
-    split_lines<H, MODE, T, G, LP, P, true>(
+    split_lines<H, MODE, T, G, LP, true>(
         [&](int g, int i) {
           const float2 v = *reinterpret_cast<const float2*>(base(g) + i * P);
           return f2_make(v.x, v.y);
         },
-        [&](int g, int i, F2 v) { *reinterpret_cast<F2*>(base(g) + i * P) = v; }, base, tcol);
+        [&](int g, int i, F2 v) { *reinterpret_cast<F2*>(base(g) + i * P) = v; }, base, P, tcol);
   } else {
     for (int l = threadIdx.x; l < ARR * W / 2; l += T) {
       float* c = smem + (l / (W / 2)) * AP + 2 * (l % (W / 2));
