@@ -157,9 +157,9 @@ def tune_classes(items, x, tuning: Optional[Dict[str, int]] = None, steps: int =
     # together, the whole-array (tile) classes share one persistent launch beside the two-pass
     # classes' own launches.
     hybrid = {r["class"]: ("queue" if "launch_small" not in r["ms"] else every_launch[r["class"]]) for r in rows}
-    # merged: the two-pass classes share one column-pass launch per column length and mode and one
-    # row-pass launch per row length and mode (far fewer launches and tails); whole 32768-float
-    # arrays keep their own launch, the rest the queue
+    # merged: the two-pass classes share a few column-pass launches and a few row-pass launches (one
+    # per group of line lengths; far fewer launches and tails); the classes that cannot merge keep
+    # their own launch, the rest the queue
     from .ragged import two_pass
 
     def merged_choice(r):

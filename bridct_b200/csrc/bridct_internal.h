@@ -18,8 +18,6 @@ struct DeviceCtx {
   long long l2_bytes = 0;
   LaunchCtx launch{};
   PlainLauncher plain[8][8][3] = {};
-  UnitLauncher col_units[8][3] = {};    // merged column passes, by lg(column length) and mode
-  UnitLauncher row_units[8][3] = {};    // merged row passes, by lg(row length) and mode
   SplitTables split[4] = {};            // rotation tables of N = 128, 256, 512, 1024
   std::vector<void*> table_mem;
   LineTables line_tables(int h, int w) const;
@@ -31,6 +29,22 @@ double sj_scale(int n, int k);
 // Rotation tables of the split lines of N = 128..1024 points (sj_split.cuh, SplitTab), float64-derived.
 std::vector<float> split_tables_host(int N);
 DeviceCtx* device_ctx(int device);
+
+// One unit of a merged pass (merged.cu): a column strip or a row block, starting `off` floats into both
+// x and y, rows ld floats apart, of lines of n points in the given mode.
+struct MergedUnit {
+  long long off;
+  int ld;
+  short n, mode;
+};
+// Which kernel takes the units of line length n (columns 0..2, rows 0..3), the strip width of column
+// length h, the row-block height of row length w, and one such launch (columns x -> y, rows in place;
+// mode -1: every unit in its own mode).
+int merged_class(bool col, int n);
+int merged_strip_cols(int h);
+int merged_block_rows(int w);
+cudaError_t launch_merged_pass(const DeviceCtx* d, bool col, int cls, int mode, const MergedUnit* units, long long n,
+                               const float* x, float* y, cudaStream_t st);
 // Opts `kernel` into `smem` bytes of dynamic shared memory on the current device and returns
 // its resident blocks per SM at `threads` threads (0 on failure); cached per device, since the
 // attribute belongs to the device's copy of the kernel.

@@ -67,7 +67,7 @@ cudaError_t launch_split_cols(const float* x, float* y, long long batch, const B
                               SplitTables tab, const LaunchCtx& ctx, cudaStream_t st) {
   using Wide = ColGeo<H>;
   using Few = ColGeo<H, kFewPairs>;
-  const SplitArgs a{x, y, tab, W, lx, ly, nullptr};
+  const SplitArgs a{x, y, tab, W, lx, ly};
   const long long units = batch * (W / Wide::TC);
   if ((units <= 64 && (W < 128 || few_rows<cmax(W, 128)>(batch * H, ctx))) || (GEN && lx.small_units))
     return launch_split(k_split_cols<H, GEN ? 0 : W, MODE, kFewPairs>, Few::kSmem, Few::T, batch * (W / Few::TC), a, st);
@@ -80,7 +80,7 @@ cudaError_t launch_split_rows(float* y, long long batch, const BatchLayout& ly, 
                               cudaStream_t st) {
   using Wide = RowGeo<W>;
   using Few = RowGeo<W, kFewPairs>;
-  const SplitArgs a{y, y, tab, W, ly, ly, nullptr};
+  const SplitArgs a{y, y, tab, W, ly, ly};
   if (few_rows<W>(batch * H, ctx) || (GEN && ly.small_units))
     return launch_split(k_split_rows<W, GEN ? H : 0, MODE, kFewPairs>, Few::kSmem, Few::T, batch * H / Few::RB, a, st);
   return launch_split(k_split_rows<W, GEN ? H : 0, MODE, 8>, Wide::kSmem, Wide::T, batch * H / Wide::RB, a, st);
@@ -226,7 +226,7 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
       e = launch_split_cols<H, W, MODE, GEN>(x, y, batch, lx, ly, tab.col, ctx, st);
     } else {
       using Geo = PairColGeo<H>;
-      e = launch_split(k_pair_cols<H, MODE, GEN>, 0, Geo::T, batch * (W / Geo::TC), SplitArgs{x, y, {}, W, lx, ly, nullptr},
+      e = launch_split(k_pair_cols<H, MODE, GEN>, 0, Geo::T, batch * (W / Geo::TC), SplitArgs{x, y, {}, W, lx, ly},
                        st);
     }
     if (e != cudaSuccess) return e;
@@ -235,7 +235,7 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
     } else {
       using Geo = PairRowGeo<W>;
       return launch_split(k_pair_rows<W, GEN ? H : 0, MODE>, Geo::kSmem, Geo::T, batch * H / Geo::RB,
-                          SplitArgs{y, y, {}, W, ly, ly, nullptr}, st);
+                          SplitArgs{y, y, {}, W, ly, ly}, st);
     }
   }
 }
@@ -246,46 +246,6 @@ cudaError_t launch_plain(const float* x, float* y, long long batch, cudaStream_t
   if (lx && ly) return launch_plain_impl<H, W, MODE, true>(x, y, batch, st, tab, ctx, *lx, *ly);
   return launch_plain_impl<H, W, MODE, false>(x, y, batch, st, tab, ctx, BatchLayout{}, BatchLayout{});
 }
-
-// Merged passes of a ragged batch (UNITS kernels): one launch over the column strips of arrays of
-// column length H and any width (launch_col_units), or over the row blocks of arrays of row length
-// W and any height (launch_row_units), with the geometry the two-pass route uses for them (the
-// strip width depends only on H and the row-block height only on W for two-pass shapes; the
-// templates take 1024 for the other axis).  `units` lists the strips (or blocks), n of them.
-using UnitLauncher = cudaError_t (*)(const float*, float*, const PassUnit*, long long, cudaStream_t,
-                                     LineTables, const LaunchCtx&);
-
-template <int H, int MODE>
-cudaError_t launch_col_units(const float* x, float* y, const PassUnit* units, long long n, cudaStream_t st,
-                             LineTables tab, const LaunchCtx& ctx) {
-  if constexpr (H >= 128) {
-    using Geo = ColGeo<H>;
-    return launch_split(k_split_cols<H, 0, MODE, col_pairs<H>()>, Geo::kSmem, Geo::T, n,
-                        SplitArgs{x, y, tab.col, 0, BatchLayout{}, BatchLayout{}, units}, st);
-  } else {
-    using Geo = PairColGeo<H>;
-    return launch_split(k_pair_cols<H, MODE, true>, 0, Geo::T, n,
-                        SplitArgs{x, y, {}, 0, BatchLayout{}, BatchLayout{}, units}, st);
-  }
-}
-
-template <int W, int MODE>
-cudaError_t launch_row_units(const float* x, float* y, const PassUnit* units, long long n, cudaStream_t st,
-                             LineTables tab, const LaunchCtx& ctx) {
-  if constexpr (W >= 128) {
-    using Geo = RowGeo<W>;
-    return launch_split(k_split_rows<W, W, MODE, 8>, Geo::kSmem, Geo::T, n,
-                        SplitArgs{x, y, tab.row, 0, BatchLayout{}, BatchLayout{}, units}, st);
-  } else {
-    using Geo = PairRowGeo<W>;
-    return launch_split(k_pair_rows<W, W, MODE>, Geo::kSmem, Geo::T, n,
-                        SplitArgs{x, y, {}, 0, BatchLayout{}, BatchLayout{}, units}, st);
-  }
-}
-
-// Strip width of two-pass arrays of column length h, and row-block height of row length w.
-int merged_strip_cols(int h);
-int merged_block_rows(int w);
 
 // Per-H instantiation units (plain_inst.cu compiled once per H) export this table row.
 void plain_table_row(int h, PlainLauncher (*row)[3]);

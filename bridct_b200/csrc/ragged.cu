@@ -26,12 +26,12 @@ struct RaggedClass {
 
 constexpr int kRaggedMaxStreams = 8;
 
-// A merged pass: every column strip (col) or row block of the MERGED classes that share one column
-// length (or row length) and mode, as one launch over a device table of units.
+// A merged pass: every column strip (col) or row block of the MERGED classes whose line lengths share a
+// kernel (merged.cu), as one launch over a device table of units.
 struct MergedPass {
-  int len = 0, mode = 0;
+  int cls = 0, mode = 0;              // mode -1: every unit its own
   bool col = true;
-  bridct::PassUnit* d_units = nullptr;
+  bridct::MergedUnit* d_units = nullptr;
   long long n = 0;
   size_t floats = 0;
 };
@@ -189,42 +189,49 @@ int build_classes(bridct_ragged* r) {
   return e == cudaSuccess ? BRIDCT_OK : cuda_fail(e, "ragged streams");
 }
 
+// Merged batches up to this many elements take all modes in one launch: the launches bound them (81
+// against 88 us a call at 12 M elements, 192 against 182 at 37 M; merged.cu).
+constexpr size_t kMergedAllModes = (size_t)1 << 24;
+
 void free_merged(bridct_ragged* r) {
   for (MergedPass& m : r->merged) cudaFree(m.d_units);
   r->merged.clear();
 }
 
-// Unit tables of the merged passes: column strips of the MERGED classes grouped by (column length,
-// mode), row blocks grouped by (row length, mode), each group largest first.
+// Unit tables of the merged passes: column strips of the MERGED classes grouped by the kernel of their
+// column length, row blocks by that of their row length, each group largest first.  Within a group the
+// units go by line length and mode, so that the CTAs of an SM run few line programs at a time.
 int build_merged(bridct_ragged* r) {
   free_merged(r);
-  std::map<std::pair<int, int>, std::vector<PassUnit>> cols, rows;
-  std::map<std::pair<int, int>, size_t> cfl, rfl;
-  for (const RaggedClass& c : r->classes) {
-    if (c.schedule != BRIDCT_RAGGED_MERGED) continue;
-    const int tc = merged_strip_cols(c.h), rb = merged_block_rows(c.w);
-    for (int i : c.arrays) {
-      const long long off = (long long)r->items[i].offset;
-      for (int s0 = 0; s0 < c.w; s0 += tc) cols[{c.h, c.mode}].push_back(PassUnit{off + s0, c.w});
-      for (int r0 = 0; r0 < c.h; r0 += rb) rows[{c.w, c.mode}].push_back(PassUnit{off + (long long)r0 * c.w, c.w});
-      cfl[{c.h, c.mode}] += (size_t)c.h * c.w;
-      rfl[{c.w, c.mode}] += (size_t)c.h * c.w;
-    }
-  }
+  size_t floats = 0;
+  for (const RaggedClass& c : r->classes) floats += c.schedule == BRIDCT_RAGGED_MERGED ? c.floats : 0;
+  const bool all_modes = floats <= kMergedAllModes;
   for (int pass = 0; pass < 2; ++pass) {
-    auto& groups = pass == 0 ? cols : rows;
-    auto& fl = pass == 0 ? cfl : rfl;
+    const bool col = pass == 0;
+    std::map<std::pair<int, int>, std::vector<MergedUnit>> groups;
+    for (const RaggedClass& c : r->classes) {
+      if (c.schedule != BRIDCT_RAGGED_MERGED) continue;
+      std::vector<MergedUnit>& g = groups[{merged_class(col, col ? c.h : c.w), all_modes ? -1 : c.mode}];
+      const int step = col ? merged_strip_cols(c.h) : merged_block_rows(c.w), end = col ? c.w : c.h;
+      for (int i : c.arrays)
+        for (int k = 0; k < end; k += step)
+          g.push_back(MergedUnit{(long long)r->items[i].offset + (long long)k * (col ? 1 : c.w), c.w,
+                                 (short)(col ? c.h : c.w), (short)c.mode});
+    }
     std::vector<MergedPass> list;
     for (auto& kv : groups) {
+      std::vector<MergedUnit>& g = kv.second;
+      std::stable_sort(g.begin(), g.end(), [](const MergedUnit& a, const MergedUnit& b) {
+        return a.n != b.n ? a.n > b.n : a.mode < b.mode;
+      });
       MergedPass m;
-      m.len = kv.first.first;
+      m.cls = kv.first.first;
       m.mode = kv.first.second;
-      m.col = pass == 0;
-      m.n = (long long)kv.second.size();
-      m.floats = fl[kv.first];
-      cudaError_t e = cudaMalloc((void**)&m.d_units, kv.second.size() * sizeof(PassUnit));
-      if (e == cudaSuccess)
-        e = cudaMemcpy(m.d_units, kv.second.data(), kv.second.size() * sizeof(PassUnit), cudaMemcpyHostToDevice);
+      m.col = col;
+      m.n = (long long)g.size();
+      for (const MergedUnit& u : g) m.floats += (size_t)u.n * (col ? merged_strip_cols(u.n) : merged_block_rows(u.n));
+      cudaError_t e = cudaMalloc((void**)&m.d_units, g.size() * sizeof(MergedUnit));
+      if (e == cudaSuccess) e = cudaMemcpy(m.d_units, g.data(), g.size() * sizeof(MergedUnit), cudaMemcpyHostToDevice);
       if (e != cudaSuccess) {
         cudaFree(m.d_units);
         free_merged(r);
@@ -239,16 +246,8 @@ int build_merged(bridct_ragged* r) {
 }
 
 int launch_merged(bridct_ragged* r, const MergedPass& m, const float* x, float* y, cudaStream_t st) {
-  const int li = lg(m.len);
-  UnitLauncher fn = m.col ? r->dev->col_units[li][m.mode] : r->dev->row_units[li][m.mode];
-  if (!fn) {
-    set_error("ragged: no merged pass for this length");
-    return BRIDCT_INVALID_ARGUMENT;
-  }
-  // the line tables of the pass's own axis (the other axis's are not read)
-  const LineTables tab = r->dev->line_tables(m.len, m.len);
   // column passes read x and write y; row passes transform y in place
-  cudaError_t e = fn(m.col ? x : y, y, m.d_units, m.n, st, tab, r->dev->launch);
+  cudaError_t e = launch_merged_pass(r->dev, m.col, m.cls, m.mode, m.d_units, m.n, m.col ? x : y, y, st);
   return e == cudaSuccess ? BRIDCT_OK : cuda_fail(e, "merged pass launch");
 }
 

@@ -35,15 +35,6 @@ struct BatchLayout {
   int small_units = 0;   // two-pass shapes: force the narrow strips and row blocks
 };
 
-// One unit of a merged launch: a column strip or a row block of some array of a
-// ragged batch, starting `off` floats into both x and y, rows `ld` floats apart.  A merged column
-// launch covers strips of arrays that share the column length but not the width; a merged row
-// launch covers row blocks of arrays that share the row length but not the height.
-struct PassUnit {
-  long long off;
-  long long ld;
-};
-
 struct TileArgs {
   const float* x;
   float* y;

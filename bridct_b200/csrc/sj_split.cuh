@@ -392,7 +392,6 @@ struct SplitArgs {
   SplitTables tab;
   int width;              // run-time layouts: columns of an array
   BatchLayout lx, ly;     // run-time layouts
-  const PassUnit* units;  // one strip or row block per unit, where set
 };
 
 // A strip of TC columns is copied to shared memory (cp.async: loads into registers would be limited
@@ -445,7 +444,7 @@ __device__ __forceinline__ void split_col_unit(const float* x, float* y, long lo
       [&](int) { return smem + p; }, TC, tab);
 }
 
-// W > 0: strips of contiguous N x W arrays; W = 0: run-time layouts, or units.
+// W > 0: strips of contiguous N x W arrays; W = 0: run-time layouts.
 template <int N, int W, int MODE, int LP>
 __global__ void __launch_bounds__(ColGeo<N, LP>::T, ColGeo<N, LP>::kBlocks) k_split_cols(SplitArgs a) {
   using Geo = ColGeo<N, LP>;
@@ -460,9 +459,6 @@ __global__ void __launch_bounds__(ColGeo<N, LP>::T, ColGeo<N, LP>::kBlocks) k_sp
     const unsigned arr = blockIdx.x / S, s = blockIdx.x % S;
     const long long off = (long long)arr * N * W + s * TC;
     split_col_unit<N, W, MODE, LP>(a.x + off, a.y + off, W, W, smem, tab);
-  } else if (a.units) {
-    const PassUnit u = a.units[blockIdx.x];
-    split_col_unit<N, 0, MODE, LP>(a.x + u.off, a.y + u.off, u.ld, u.ld, smem, tab);
   } else {
     const unsigned S = a.width / TC, arr = blockIdx.x / S, s = blockIdx.x % S;
     split_col_unit<N, 0, MODE, LP>(a.x + layout_row<N>(a.lx, (long long)arr * N) + s * TC,
@@ -533,7 +529,7 @@ __device__ __forceinline__ void split_row_unit(const XRow& xrow, const YRow& yro
 }
 
 // RB consecutive rows of a (batch * H) x N matrix per CTA.  H = 0: contiguous rows; H > 0: run-time
-// layouts of arrays of H rows, or units.
+// layouts of arrays of H rows.
 template <int N, int H, int MODE, int LP>
 __global__ void __launch_bounds__(RowGeo<N, LP>::T, RowGeo<N, LP>::kBlocks) k_split_rows(SplitArgs a) {
   using Geo = RowGeo<N, LP>;
@@ -546,10 +542,6 @@ __global__ void __launch_bounds__(RowGeo<N, LP>::T, RowGeo<N, LP>::kBlocks) k_sp
   if constexpr (H == 0) {
     split_row_unit<N, MODE, LP>([&](int r) { return a.x + (first + r) * N; },
                                 [&](int r) { return a.y + (first + r) * N; }, smem, tab);
-  } else if (a.units) {
-    const PassUnit u = a.units[blockIdx.x];
-    split_row_unit<N, MODE, LP>([&](int r) { return a.x + u.off + r * u.ld; },
-                                [&](int r) { return a.y + u.off + r * u.ld; }, smem, tab);
   } else {
     split_row_unit<N, MODE, LP>([&](int r) { return a.x + layout_row<H>(a.lx, first + r); },
                                 [&](int r) { return a.y + layout_row<H>(a.ly, first + r); }, smem, tab);
@@ -597,32 +589,8 @@ template <int N> struct PairColGeo {
   static constexpr int T = 32;
   static constexpr int TC = 2 * T;
 };
-template <int N, int MODE, bool GEN>
-__global__ void __launch_bounds__(32) k_pair_cols(SplitArgs a) {
-  constexpr int TC = PairColGeo<N>::TC;
-  griddep_wait();
-  griddep_trigger();
-  const float* x;
-  float* y;
-  long long xp = a.width, yp = a.width;
-  if (GEN && a.units) {
-    const PassUnit u = a.units[blockIdx.x];
-    x = a.x + u.off;
-    y = a.y + u.off;
-    xp = yp = u.ld;
-  } else {
-    const unsigned S = a.width / TC, arr = blockIdx.x / S, s = blockIdx.x % S;
-    if (GEN) {
-      x = a.x + layout_row<N>(a.lx, (long long)arr * N) + s * TC;
-      y = a.y + layout_row<N>(a.ly, (long long)arr * N) + s * TC;
-      xp = a.lx.ld;
-      yp = a.ly.ld;
-    } else {
-      const long long off = (long long)arr * N * a.width + s * TC;
-      x = a.x + off;
-      y = a.y + off;
-    }
-  }
+template <int N, int MODE>
+__device__ __forceinline__ void pair_col_unit(const float* x, float* y, long long xp, long long yp) {
   x += 2 * threadIdx.x;
   y += 2 * threadIdx.x;
   F2 v[N];
@@ -639,6 +607,20 @@ __global__ void __launch_bounds__(32) k_pair_cols(SplitArgs a) {
     *reinterpret_cast<float2*>(y + i * yp) = f;
   }
 }
+template <int N, int MODE, bool GEN>
+__global__ void __launch_bounds__(32) k_pair_cols(SplitArgs a) {
+  constexpr int TC = PairColGeo<N>::TC;
+  griddep_wait();
+  griddep_trigger();
+  const unsigned S = a.width / TC, arr = blockIdx.x / S, s = blockIdx.x % S;
+  if constexpr (GEN) {
+    pair_col_unit<N, MODE>(a.x + layout_row<N>(a.lx, (long long)arr * N) + s * TC,
+                           a.y + layout_row<N>(a.ly, (long long)arr * N) + s * TC, a.lx.ld, a.ly.ld);
+  } else {
+    const long long off = (long long)arr * N * a.width + s * TC;
+    pair_col_unit<N, MODE>(a.x + off, a.y + off, a.width, a.width);
+  }
+}
 
 // Row pass of 32- and 64-point rows in place: 64 rows per warp, staged in shared memory.
 template <int N> struct PairRowGeo {
@@ -647,19 +629,10 @@ template <int N> struct PairRowGeo {
   static constexpr int P = N + 4;
   static constexpr int kSmem = RB * P * 4;
 };
-template <int N, int H, int MODE>
-__global__ void __launch_bounds__(32) k_pair_rows(SplitArgs a) {
+template <int N, int MODE, typename Row>
+__device__ __forceinline__ void pair_row_unit(const Row& row, float* smem) {
   using Geo = PairRowGeo<N>;
   constexpr int P = Geo::P, Q = N / 4;
-  extern __shared__ float smem[];
-  griddep_wait();
-  griddep_trigger();
-  const long long first = (long long)blockIdx.x * Geo::RB;
-  auto row = [&](int r) -> float* {
-    if (H == 0) return a.y + (first + r) * N;
-    if (a.units) return a.y + a.units[blockIdx.x].off + r * a.units[blockIdx.x].ld;
-    return a.y + layout_row<cmax(H, 1)>(a.ly, first + r);
-  };
 #pragma unroll 8
   for (int i = threadIdx.x; i < Geo::RB * Q; i += 32) cp_async16(smem + i / Q * P + i % Q * 4, row(i / Q) + i % Q * 4);
   cp_async_wait_all();
@@ -670,6 +643,16 @@ __global__ void __launch_bounds__(32) k_pair_rows(SplitArgs a) {
 #pragma unroll 8
   for (int i = threadIdx.x; i < Geo::RB * Q; i += 32)
     *reinterpret_cast<float4*>(row(i / Q) + i % Q * 4) = *reinterpret_cast<const float4*>(smem + i / Q * P + i % Q * 4);
+}
+template <int N, int H, int MODE>
+__global__ void __launch_bounds__(32) k_pair_rows(SplitArgs a) {
+  extern __shared__ float smem[];
+  griddep_wait();
+  griddep_trigger();
+  const long long first = (long long)blockIdx.x * PairRowGeo<N>::RB;
+  pair_row_unit<N, MODE>(
+      [&](int r) -> float* { return H == 0 ? a.y + (first + r) * N : a.y + layout_row<cmax(H, 1)>(a.ly, first + r); },
+      smem);
 }
 
 // ---- whole arrays in one tile ------------------------------------------------------------------

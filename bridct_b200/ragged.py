@@ -34,9 +34,9 @@ SCHEDULES = {"queue": 0, "launch": 1, "launch_small": 2, "merged": 3}
 
 
 def two_pass(h: int, w: int, mode: int) -> bool:
-    """Whether the plain form runs (h, w, mode) as a column pass then a row pass (the classes that
-    may take the "merged" schedule): every shape above 16384 floats except whole 32768-float
-    arrays in the modes where one tile measured faster (plain_launch.cuh, whole_array_route)."""
+    """Whether the class (h, w, mode) may take the "merged" schedule (plain_launch.cuh, merged_route):
+    every shape above 16384 floats, which the plain form runs as a column pass then a row pass,
+    without some 32768-float classes."""
     whole = h * w == 32768 and (mode == 1 or h in (1024, 64) or (h == 32 and mode == 0))
     return h * w > 16384 and not whole
 

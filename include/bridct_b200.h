@@ -153,7 +153,7 @@ BRIDCT_API int bridct_ragged_apply_device(bridct_ragged *batch, const float *inp
  * The batch's arrays fall into shape classes (height, width, mode), numbered largest first (by
  * elements).  Each class runs either in the shared persistent queue, or as its own launch of the
  * fixed-shape kernels of that shape over the class's offset table, with the tile shapes measured
- * best for that shape, or with the few-array geometry (one four-step line group per warp).  The
+ * best for that shape, or with the few-array geometry (narrow strips and row blocks).  The
  * autotuner (bridct_b200.autotune) measures the choices per class.  No reference counterpart: the
  * reference picks a per-(h, w, mode) policy from a table (src/generated/rect_policy.inc,
  * src/plan.c:140-148). */
@@ -161,9 +161,9 @@ enum bridct_ragged_schedule {
     BRIDCT_RAGGED_QUEUE = 0,               /* units in the persistent kernel's queue           */
     BRIDCT_RAGGED_CLASS_LAUNCH = 1,        /* the class's own fixed-shape launch               */
     BRIDCT_RAGGED_CLASS_LAUNCH_SMALL = 2,  /* the same with the few-array geometry (two-pass)  */
-    BRIDCT_RAGGED_MERGED = 3               /* two-pass classes only: one column-pass launch per
-                                              (column length, mode) and one row-pass launch per
-                                              (row length, mode) over all MERGED classes      */
+    BRIDCT_RAGGED_MERGED = 3               /* two-pass classes only: column passes, then row
+                                              passes, one launch per group of line lengths
+                                              over all MERGED classes                         */
 };
 BRIDCT_API size_t bridct_ragged_class_count(const bridct_ragged *batch);
 /* Kernel launches of one bridct_ragged_apply_device call with the current schedule: the merged

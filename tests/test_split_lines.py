@@ -90,3 +90,33 @@ def test_tiles_agree_bitwise_and_with_float64(shape, many):
         ref = O.fp64_apply(tail, mode)
         err = np.abs(y[-5:].cpu().numpy() - ref).max() / max(np.abs(tail).max(), np.abs(ref).max())
         assert err <= 2e-6, (mode, err)
+
+
+# The ragged batch's kernels over every shape and mode once: the queue with its default and its
+# smallest units, the merged passes with all modes in one launch, and (two arrays of each class, more
+# than 2^24 elements) a launch per mode.
+@pytest.mark.gpu
+@pytest.mark.parametrize("schedule,copies,unit", [("queue", 1, 16384), ("queue", 1, 1024), ("merged", 1, 16384),
+                                                  ("merged", 2, 16384)])
+def test_ragged_kernels_on_every_shape_and_mode(schedule, copies, unit):
+    import torch
+
+    from bridct_b200.ragged import RaggedBatch, two_pass
+    from oracle import oracle as O
+
+    sizes = (8, 16, 32, 64, 128, 256, 512, 1024)
+    items = [(h, w, m) for h in sizes for w in sizes for m in range(3) for _ in range(copies)]
+    total = sum(h * w for h, w, m in items if two_pass(h, w, m))
+    assert (total > 1 << 24) == (copies == 2)
+    classes = {f"{h}x{w}/{m}": "merged" for h, w, m in items if two_pass(h, w, m)}
+    batch = RaggedBatch(items, tuning=dict(tile_floats=unit, strip_floats=unit, row_floats=unit),
+                        schedule={"classes": classes, "streams": 2} if schedule == "merged" else None)
+    rng = np.random.default_rng(copies)
+    x = torch.from_numpy(rng.standard_normal(batch.span).astype(np.float32)).cuda()
+    y = batch.apply(x)
+    torch.cuda.synchronize()
+    assert not batch.timed_out()
+    for (h, w, m), xi, yi in zip(items, batch.unpack(x.cpu()), batch.unpack(y.cpu())):
+        xi, ref = xi.numpy(), O.fp64_apply(xi.numpy(), m)
+        err = np.abs(yi.numpy() - ref).max() / max(np.abs(xi).max(), np.abs(ref).max())
+        assert err <= 2e-6, (h, w, m, err)
