@@ -13,7 +13,7 @@
 // 64 output columns: its slice of C_L (64 x L, split into bf16 or tf32 parts, in the K-major
 // 128-byte-swizzled image the UMMA B operand reads) is loaded into shared memory once (L <= 256)
 // or arrives chunk by chunk with the ring (L = 512, 1024), and the CTA streams M-tiles through a
-// TMA ring in K-chunks (64 FP32 per row for BF16x3, 32 for TF32x3).  Rows of 8, 16 or 32 points
+// TMA ring in K-chunks (64 FP32 per row for BF16x3, 32 for TF32x3 and for short folded rows).  Rows of 8, 16 or 32 points
 // run as 64-float super-rows against a block-diagonal B (SUB).
 // Rows of 128 points and more use the symmetry of C_L (PassFold), which halves the products, and for
 // every output also the loads and splits:
@@ -70,6 +70,13 @@ enum PassFold { FOLD_NONE = 0, FOLD_FWD = 1, FOLD_INV = 2 };
 // parity: with 64, every M-tile crosses from L2 four times, and that traffic (4.9 TB/s) bounds the pass.
 __host__ __device__ constexpr int pass_nblock(int L, int fold) { return fold == FOLD_FWD && L == 256 ? 128 : 64; }
 
+// Folded BF16x3 forward passes of 128 and 256 points run K-chunks of 32: the same ring then holds twice
+// the stages, and loads, splits and products of one M-tile overlap more finely (16 M elements at 256 x 256:
+// 96.4 -> 91.9 us).  512 points measured 221 us that way, 210 with chunks of 64.
+__host__ __device__ constexpr bool pass_half(int form, int L, int fold) {
+  return form == BF16X3 && fold == FOLD_FWD && L <= 256;
+}
+
 // Shared-memory plan of one row pass.  The CTA's slice of the coefficient matrix stays resident when it
 // fits beside a two-stage ring; otherwise every ring stage carries the slice's K-chunk next to the A
 // chunk (STREAM_B), brought in by a bulk copy from the pre-split image in global memory (L2-resident:
@@ -78,15 +85,18 @@ __host__ __device__ constexpr int pass_nblock(int L, int fold) { return fold == 
 template <int FORM, int L, int FOLD = FOLD_NONE>
 struct PassLayout {
   using F = PassForm<FORM>;
+  static constexpr bool kHalf = pass_half(FORM, L, FOLD);
+  static constexpr int kKC = kHalf ? 32 : F::kKC;                          // products per K-chunk
   static constexpr int kK = FOLD == FOLD_FWD ? L / 2 : L;                  // products per output
-  static constexpr int kChunks = kK / F::kKC;
+  static constexpr int kChunks = kK / kKC;
+  static constexpr int kStageBytes = kRows * kKC * 4;
   static constexpr int kNBlock = pass_nblock(L, FOLD);
   static constexpr int kBlocks = (FOLD == FOLD_INV ? L / 2 : L) / kNBlock;
   static constexpr int kBPart = kBAtom * kNBlock / 64;            // one split part of a K-chunk
-  static constexpr int kBBytes = F::kSplits * kChunks * kBPart;   // this CTA's slice of C_L
-  static constexpr int kBChunk = F::kSplits * kBPart;             // one K-chunk of the slice
+  static constexpr int kBBytes = F::kSplits * (kK / F::kKC) * kBPart;   // this CTA's slice of C_L
+  static constexpr int kBChunk = F::kSplits * kBPart;             // F::kKC products' part of the slice
   static constexpr int kABufs = FOLD == FOLD_FWD ? 0 : 2;
-  static constexpr int kABytes = (FOLD == FOLD_FWD ? 2 : 1) * F::kStageBytes;   // A data of a stage
+  static constexpr int kABytes = (FOLD == FOLD_FWD ? 2 : 1) * kStageBytes;   // A data of a stage
   static constexpr int kBarBytes = 1024;
   static constexpr bool kStreamB = kBBytes + kABufs * F::kABufBytes + kBarBytes + 1024 + 2 * kABytes > kPassSmemMax;
   static constexpr int kResident = kStreamB ? 0 : kBBytes;
@@ -102,7 +112,8 @@ struct PassLayout {
   static_assert(kDynamic <= kPassSmemMax, "shared memory budget");
   // where the split parts lie: hi at the stage, mid (BF16x3) and lo at these offsets, lo in the A buffer
   // unless folded forward
-  static constexpr int kMidOff = FOLD == FOLD_FWD ? 49152 : 16384;
+  static constexpr int kMidOff = kHalf ? 64 : FOLD == FOLD_FWD ? 49152 : 16384;
+  static_assert(!kHalf || !kStreamB, "half chunks: resident coefficients");
   static constexpr int kLoOff = 16384;
 };
 
@@ -113,12 +124,14 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
+// a_full: one per A buffer, or folded forward (no A buffers) one per stage.
+constexpr int kPassTmemSlot = 24 * kPassMaxStages + 48;
 struct PassBars {
-  uint32_t stage_full, stage_free, a_full, a_free, acc_full, acc_free, tmem_slot;
+  uint32_t stage_full, stage_free, a_full, a_free, acc_full, acc_free;
   __device__ explicit PassBars(uint32_t b)
       : stage_full(b), stage_free(b + 8 * kPassMaxStages), a_full(b + 16 * kPassMaxStages),
-        a_free(b + 16 * kPassMaxStages + 16), acc_full(b + 16 * kPassMaxStages + 32),
-        acc_free(b + 16 * kPassMaxStages + 48), tmem_slot(b + 16 * kPassMaxStages + 64) {}
+        a_free(b + 24 * kPassMaxStages), acc_full(b + 24 * kPassMaxStages + 16),
+        acc_free(b + 24 * kPassMaxStages + 32) {}
 };
 
 // TF32 split of a one-box stage (128 rows x 32 FP32): Xh in place, Xl into the A buffer.
@@ -172,6 +185,29 @@ __device__ __forceinline__ void split_fold_bf16(uint8_t* stage, uint32_t r, floa
   for (int jq = 0; jq < 4; ++jq)
     *reinterpret_cast<uint4*>(stage + 16384u + sw128(r, jq)) =
         make_uint4(lo0[jq][0], lo0[jq][1], lo0[jq][2], lo0[jq][3]);
+}
+// BF16x3, K-chunks of 32: boxes a, b; a row of box a becomes hi (64 bytes) and mid, that of box b lo.
+__device__ __forceinline__ void split_fold_bf16_half(uint8_t* stage, uint32_t r, float sign) {
+  float4 w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(stage + 16384u + sw128(r, j));
+  uint32_t mid[4][4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {   // elements 8q .. 8q + 7
+    const float4 u0 = *reinterpret_cast<const float4*>(stage + sw128(r, 2 * q));
+    const float4 u1 = *reinterpret_cast<const float4*>(stage + sw128(r, 2 * q + 1));
+    const float4 w0 = w[7 - 2 * q], w1 = w[6 - 2 * q];
+    uint32_t hi[4], lo[4];
+    split_bf16x3_pair(fmaf(sign, w0.w, u0.x), fmaf(sign, w0.z, u0.y), hi[0], mid[q][0], lo[0]);
+    split_bf16x3_pair(fmaf(sign, w0.y, u0.z), fmaf(sign, w0.x, u0.w), hi[1], mid[q][1], lo[1]);
+    split_bf16x3_pair(fmaf(sign, w1.w, u1.x), fmaf(sign, w1.z, u1.y), hi[2], mid[q][2], lo[2]);
+    split_bf16x3_pair(fmaf(sign, w1.y, u1.z), fmaf(sign, w1.x, u1.w), hi[3], mid[q][3], lo[3]);
+    *reinterpret_cast<uint4*>(stage + sw128(r, q)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(stage + 16384u + sw128(r, q)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    *reinterpret_cast<uint4*>(stage + sw128(r, 4 + q)) = make_uint4(mid[q][0], mid[q][1], mid[q][2], mid[q][3]);
 }
 // TF32x3: boxes a, b; hi goes to a, lo to b.
 __device__ __forceinline__ void split_fold_tf32(uint8_t* stage, uint32_t r, float sign) {
@@ -258,20 +294,24 @@ __device__ __forceinline__ void split_deint_tf32(uint8_t* stage, uint8_t* abuf, 
 //   TF32x3 blocks [big0 | small | big1 | big2]:
 //     Xh.[Ch|Cl] -> [big0|small] (group 0) or Xh.Ch -> big_g, Xh.Cl -> small;  Xl.Ch -> small
 // The epilogue adds the blocks in FP32.
-// SETS accumulator sets share the 512 TMEM columns: two (the epilogue of one M-tile overlaps the
-// MMAs of the next) for rows up to 256 points, one for 512- and 1024-point rows, whose long K
+// SETS accumulator sets share the 512 TMEM columns (PassSets): two, so that the epilogue of one M-tile
+// overlaps the MMAs of the next, for rows up to 256 points; one for 512- and 1024-point rows, whose long K
 // needs more group accumulators than two sets leave room for (TF32x3 round trips of 1024-point
 // axes exceeded 3e-6 with three groups; one set holds seven for TF32x3, six for BF16x3).
-// PARS = 2 (folded inverse): a set holds the blocks of e, then those of o, half as many for each.  From 512
-// points on BF16x3 then adds all small products in one block, [big0 | small | big1 | big2], so that a big
-// group takes no more MMAs than in an unfolded pass (errors against float64 1.75e-7 -> 1.59e-7 at 512 x
-// 512, 2.77e-7 -> 2.66e-7 at 1024 x 1024; with two groups 2.01e-7 and 3.73e-7).  TF32x3 has nothing to
-// give up, and its inverse passes of 512 and 1024 points are not folded (launch_pass).
-template <int FORM, int CHUNKS, int SETS = 2, int PARS = 1, int NB = 64>
+// PARS = 2 (folded inverse): a set holds the blocks of e, then those of o, half as many for each.
+// MERGE: BF16x3 adds all small products in one block, [big0 | small | big1 ..].  This makes room for the
+// second set of a 128-column N-block (forward, 256 points: 91.9 -> 67 us per call on 16 M elements, with
+// the errors of one K = 128 group per output, as in the unfolded pass) and of the inverses up to 256
+// points (104 -> 95 us; 128 points 73 -> 59), and at 512 and 1024 points keeps a big group to no more MMAs
+// than in an unfolded pass (errors against float64 1.75e-7 -> 1.57e-7 at 512 x 512, 2.77e-7 -> 2.65e-7 at
+// 1024 x 1024; with two groups 2.01e-7 and 3.73e-7).  TF32x3 has nothing to give up: its folded passes of
+// 256 points forward and 128 and 256 inverse keep one set, and its inverses of 512 and 1024 points are not
+// folded (launch_pass).
+template <int FORM, int CHUNKS, int SETS, int PARS, int NB, bool MERGE>
 struct PassAccs {
   static constexpr int kNBlock = NB;
-  static constexpr bool kMerge = FORM == BF16X3 && PARS == 2 && CHUNKS >= 8;
-  static constexpr int kSmallBlocks = FORM == BF16X3 && !kMerge ? 2 : 1;
+  static constexpr bool kMerge = MERGE;
+  static constexpr int kSmallBlocks = FORM == BF16X3 && !MERGE ? 2 : 1;
   static constexpr int kMaxBig = 512 / (SETS * PARS * NB) - kSmallBlocks;
   static constexpr int kBig = CHUNKS < kMaxBig ? CHUNKS : kMaxBig;
   static constexpr int kPerParity = (1 + kSmallBlocks + (kBig - 1)) * NB;
@@ -282,24 +322,28 @@ struct PassAccs {
   __host__ __device__ static constexpr int group(int kc) { return kc * kBig / CHUNKS; }
 };
 
-// Accumulator sets: one where long K needs the groups (or e and o do not fit twice).
+// Accumulator sets, and whether the small products share a block (see PassAccs).
 template <int FORM, int L, int FOLD> struct PassSets {
-  static constexpr int value = FOLD == FOLD_INV ? 1 : FOLD == FOLD_FWD ? (L >= 256 ? 1 : 2) : L >= 512 ? 1 : 2;
+  static constexpr bool kMerge = FORM == BF16X3 && ((FOLD == FOLD_FWD && L == 256) || FOLD == FOLD_INV);
+  static constexpr int value = L >= 512                                   ? 1
+                               : FORM == BF16X3 || FOLD == FOLD_NONE      ? 2
+                               : FOLD == FOLD_FWD && L == 128             ? 2
+                                                                          : 1;
 };
 
 // Split products of K-chunk kc (one thread): hi, mid, lo: shared addresses of the A parts (mid: BF16x3
 // only).  bchunk: shared address of the chunk's B splits, laid out [split][8 KB atom column of 64 rows].
-// tmem: column 0 of this M-tile's set.  A chunk is four K steps; with PARS = 2 the first two are e's.
-template <int FORM, int CHUNKS, int SETS, int PARS, int NB>
+// tmem: column 0 of this M-tile's set.  With PARS = 2 the first half of a chunk's steps are e's.
+// STEPS: K steps of a chunk (two in half chunks).
+template <int FORM, typename A, int PARS, int NB, int STEPS>
 __device__ __forceinline__ void issue_pass_mmas(uint32_t hi, uint32_t mid, uint32_t lo, uint32_t bchunk, int kc,
                                                 uint32_t tmem) {
-  using A = PassAccs<FORM, CHUNKS, SETS, PARS, NB>;
   constexpr uint32_t kPart = kBAtom * NB / 64;
   const int g = A::group(kc);
   const bool big_first = kc == 0 || A::group(kc - 1) != g;
-  constexpr int kSteps = 4 / PARS;   // K steps of one parity in a chunk
+  constexpr int kSteps = STEPS / PARS;   // K steps of one parity in a chunk
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {   // 32 bytes of a row per MMA: 16 bf16 or 8 tf32
+  for (int k = 0; k < STEPS; ++k) {   // 32 bytes of a row per MMA: 16 bf16 or 8 tf32
     const uint32_t t = tmem + (uint32_t)(k / kSteps) * A::kPerParity;
     const uint32_t big_g = t + A::kExtraBig + (uint32_t)(g - 1) * NB;
     const bool first = k % kSteps == 0;
@@ -309,8 +353,13 @@ __device__ __forceinline__ void issue_pass_mmas(uint32_t hi, uint32_t mid, uint3
     if constexpr (A::kMerge) {
       constexpr uint32_t i1 = instr_desc(1, NB);
       const uint64_t bm = sw128_desc(bchunk + kPart + k * 32u);
-      umma(g == 0 ? t : big_g, ah, bd, i1, g == 0 ? clear : clear_g, BF16X3);
-      umma(t + NB, ah, bm, i1, clear, BF16X3);
+      if constexpr (NB == 128) {
+        static_assert(NB != 128 || A::kBig == 1, "big and small side by side");
+        umma(t, ah, bd, instr_desc(1, 2 * NB), clear, BF16X3);
+      } else {
+        umma(g == 0 ? t : big_g, ah, bd, i1, g == 0 ? clear : clear_g, BF16X3);
+        umma(t + NB, ah, bm, i1, clear, BF16X3);
+      }
       umma(t + NB, ah, sw128_desc(bchunk + 2 * kPart + k * 32u), i1, 1u, BF16X3);
       umma(t + NB, sw128_desc(mid + k * 32u), bd, i1, 1u, BF16X3);
       umma(t + NB, sw128_desc(mid + k * 32u), bm, i1, 1u, BF16X3);
@@ -341,10 +390,11 @@ __device__ __forceinline__ void issue_pass_mmas(uint32_t hi, uint32_t mid, uint3
   }
 }
 
-// Columns q*16 .. q*16+15 of the sum of one parity's accumulator blocks at taddr.
+// Columns q*16 .. q*16+15 of one parity's accumulator blocks at taddr: the sum of the big groups and that
+// of the small products.
 template <typename ACC>
-__device__ __forceinline__ void load_sum(uint32_t taddr, int q, float (&big)[16]) {
-  float sm[16], w[16];
+__device__ __forceinline__ void load_parts(uint32_t taddr, int q, float (&big)[16], float (&sm)[16]) {
+  float w[16];
   tmem_ld16(taddr + q * 16, big);
   tmem_ld16(taddr + ACC::kNBlock + q * 16, sm);
   tmem_wait_ld();
@@ -362,8 +412,6 @@ __device__ __forceinline__ void load_sum(uint32_t taddr, int q, float (&big)[16]
 #pragma unroll
     for (int i = 0; i < 16; ++i) big[i] += w[i];
   }
-#pragma unroll
-  for (int i = 0; i < 16; ++i) big[i] += sm[i];
 }
 
 // xmap: the (nrows x L) FP32 row matrix (box 32 x 128, SWIZZLE_128B).  out: destination of
@@ -388,13 +436,13 @@ __global__ void __launch_bounds__(kPassThreads, 1)
   constexpr int kChunks = PL::kChunks;
   constexpr int kSets = PassSets<FORM, L, FOLD>::value;
   constexpr int kPars = FOLD == FOLD_INV ? 2 : 1;
-  using ACC = PassAccs<FORM, kChunks, kSets, kPars, PL::kNBlock>;
+  using ACC = PassAccs<FORM, kChunks, kSets, kPars, PL::kNBlock, PassSets<FORM, L, FOLD>::kMerge>;
   constexpr uint32_t kTileCols = ACC::kPerTile;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(base);
   const PassBars bars(sbase + PL::kBarOff);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + PL::kBarOff + 16 * kPassMaxStages + 64);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + PL::kBarOff + kPassTmemSlot);
   __shared__ volatile int s_abort;
   __shared__ volatile int s_group_ok[3];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -411,9 +459,9 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     for (int i = 0; i < kStages; ++i) {
       mbar_init(bars.stage_full + 8 * i, 1);
       mbar_init(bars.stage_free + 8 * i, 1);
+      mbar_init(bars.a_full + 8 * i, 1);
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bars.a_full + 8 * i, 1);
       mbar_init(bars.a_free + 8 * i, 1);
       mbar_init(bars.acc_full + 8 * i, 1);
       mbar_init(bars.acc_free + 8 * i, 1);
@@ -451,13 +499,13 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       const int kc = (int)(j % kChunks);
       const uint32_t dst = sbase + s * PL::kStageStride;
       mbar_expect_tx(bars.stage_full + 8 * s, PL::kStageTx);
-      tma_load_2d(dst, &xmap, kc * F::kKC, (int)(m * kRows), bars.stage_full + 8 * s);
-      if constexpr (F::kKC == 64)
-        tma_load_2d(dst + 16384u, &xmap, kc * F::kKC + 32, (int)(m * kRows), bars.stage_full + 8 * s);
+      tma_load_2d(dst, &xmap, kc * PL::kKC, (int)(m * kRows), bars.stage_full + 8 * s);
+      if constexpr (PL::kKC == 64)
+        tma_load_2d(dst + 16384u, &xmap, kc * PL::kKC + 32, (int)(m * kRows), bars.stage_full + 8 * s);
       if constexpr (FOLD == FOLD_FWD) {   // the mirrored chunk
 #pragma unroll
-        for (int b = 0; b < F::kKC / 32; ++b)
-          tma_load_2d(dst + F::kStageBytes + b * 16384u, &xmap, L - (kc + 1) * F::kKC + b * 32, (int)(m * kRows),
+        for (int b = 0; b < PL::kKC / 32; ++b)
+          tma_load_2d(dst + PL::kStageBytes + b * 16384u, &xmap, L - (kc + 1) * PL::kKC + b * 32, (int)(m * kRows),
                       bars.stage_full + 8 * s);
       }
       if constexpr (PL::kStreamB)
@@ -470,24 +518,26 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       const int s = (int)(j % kStages), a = (int)(j & 1);
       const long long jt = j / kChunks;
       const int kc = (int)(j % kChunks), t = (int)(jt % kSets);
-      ok = mbar_wait(bars.a_full + 8 * a, (uint32_t)(j >> 1) & 1u);
+      ok = FOLD == FOLD_FWD ? mbar_wait(bars.a_full + 8 * s, (uint32_t)(j / kStages) & 1u)
+                            : mbar_wait(bars.a_full + 8 * a, (uint32_t)(j >> 1) & 1u);
       if (ok && kc == 0) ok = mbar_wait(bars.acc_free + 8 * t, ((uint32_t)(jt / kSets) & 1u) ^ 1u);
       if (!ok) break;
       tc_fence_after();
       const uint32_t sstage = sbase + s * PL::kStageStride;
       const uint32_t bchunk = PL::kStreamB ? sstage + PL::kABytes
+                              : PL::kHalf  ? sbase + PL::kBOff + (uint32_t)(kc >> 1) * PL::kBChunk + (uint32_t)(kc & 1) * 64u
                                            : sbase + PL::kBOff + (uint32_t)kc * PL::kBChunk;
-      issue_pass_mmas<FORM, kChunks, kSets, kPars, PL::kNBlock>(
+      issue_pass_mmas<FORM, ACC, kPars, PL::kNBlock, PL::kHalf ? 2 : 4>(
           sstage, sstage + PL::kMidOff,
           FOLD == FOLD_FWD ? sstage + PL::kLoOff : sbase + PL::kAOff + a * F::kABufBytes, bchunk, kc,
           tmem_base + t * kTileCols);
       umma_commit(bars.stage_free + 8 * s);
-      umma_commit(bars.a_free + 8 * a);
+      if (FOLD != FOLD_FWD) umma_commit(bars.a_free + 8 * a);
       if (kc == kChunks - 1) umma_commit(bars.acc_full + 8 * t);
     }
     if (ok && nchunk_local > 0) {   // the last MMAs must finish before TMEM is freed
       const long long j = nchunk_local - 1;
-      ok = mbar_wait(bars.a_free + 8 * (int)(j & 1), (uint32_t)(j >> 1) & 1u);
+      ok = mbar_wait(bars.stage_free + 8 * (int)(j % kStages), (uint32_t)(j / kStages) & 1u);
     }
   } else if (warp >= 4 && warp < 12) {
     const int grp = (warp - 4) >> 2;              // 0: even K-chunks, 1: odd K-chunks
@@ -497,7 +547,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       const int s = (int)(j % kStages), a = (int)(j & 1);
       if (r == 0) {
         bool g = !s_abort && mbar_wait(bars.stage_full + 8 * s, (uint32_t)(j / kStages) & 1u);
-        if (g) g = mbar_wait(bars.a_free + 8 * a, ((uint32_t)(j >> 1) & 1u) ^ 1u);
+        if (FOLD != FOLD_FWD && g) g = mbar_wait(bars.a_free + 8 * a, ((uint32_t)(j >> 1) & 1u) ^ 1u);
         s_group_ok[ok_slot] = g ? 1 : 0;
       }
       named_sync(bar_id, 128);
@@ -509,7 +559,8 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       uint8_t* abuf = base + PL::kAOff + a * F::kABufBytes;
       if constexpr (FOLD == FOLD_FWD) {
         const float sign = nblk & 1 ? -1.0f : 1.0f;
-        if constexpr (FORM == BF16X3) split_fold_bf16(stage, r, sign);
+        if constexpr (PL::kHalf) split_fold_bf16_half(stage, r, sign);
+        else if constexpr (FORM == BF16X3) split_fold_bf16(stage, r, sign);
         else split_fold_tf32(stage, r, sign);
       } else if constexpr (FOLD == FOLD_INV) {
         if constexpr (FORM == BF16X3) split_deint_bf16(stage, abuf, r);
@@ -520,7 +571,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       }
       fence_async_smem();
       named_sync(bar_id, 128);
-      if (r == 0) mbar_arrive(bars.a_full + 8 * a);
+      if (r == 0) mbar_arrive(bars.a_full + 8 * (FOLD == FOLD_FWD ? s : a));
     }
   } else if (warp >= 12) {
     const uint32_t r = tid - 384;                 // tile row = TMEM lane
@@ -550,15 +601,16 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         float* hi = arr + ((long long)(L - 1 - nblk * PL::kNBlock) << rshift);
 #pragma unroll
         for (int q = 0; q < PL::kNBlock / 16; ++q) {
-          float e[16], o[16];
-          load_sum<ACC>(taddr, q, e);
-          load_sum<ACC>(taddr + ACC::kPerParity, q, o);
+          float e[16], o[16], es[16], os[16];
+          load_parts<ACC>(taddr, q, e, es);
+          load_parts<ACC>(taddr + ACC::kPerParity, q, o, os);
           if (live) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const long long c = (long long)(q * 16 + i) << rshift;
-              lo[c] = e[i] + o[i];
-              hi[-c] = e[i] - o[i];
+              // the small sums join the smaller addend first: one rounding less at the size of the result
+              lo[c] = e[i] + (o[i] + (os[i] + es[i]));
+              hi[-c] = e[i] - (o[i] + (os[i] - es[i]));
             }
           }
         }
@@ -567,14 +619,14 @@ __global__ void __launch_bounds__(kPassThreads, 1)
                                                          : nblk * PL::kNBlock) << rshift);
 #pragma unroll
         for (int q = 0; q < PL::kNBlock / 16; ++q) {
-          float v[16];
-          load_sum<ACC>(taddr, q, v);
+          float v[16], sm[16];
+          load_parts<ACC>(taddr, q, v, sm);
           if (live) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               constexpr int kLS = LS;
               const int n = q * 16 + i, j = n / kLS, c = n % kLS * (FOLD == FOLD_FWD ? 2 : 1);
-              dst[((long long)c << rshift) + j] = v[i];
+              dst[((long long)c << rshift) + j] = v[i] + sm[i];
             }
           }
         }
