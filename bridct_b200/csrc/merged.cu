@@ -1,7 +1,7 @@
 // Merged passes of a ragged batch: one launch over the column strips (or row blocks) of arrays of many
 // shapes.  Each CTA takes the unit of its block index and runs the pass of that unit's line length, so a
 // launch holds every length that needs about the same registers and shared memory: columns of 32 and 64
-// points, of 128 to 512, and of 1024; rows of 64, of 128 and 256, of 512, and of 1024.  Batches whose
+// points, of 128 to 512, and of 1024; rows of 32 and 64, of 128 and 256, of 512, and of 1024.  Batches whose
 // launches cost the host more than the device take all modes in one launch too (3 + 4 launches at most
 // instead of up to 21); larger ones a launch per mode, whose kernels are faster (fewer line programs in
 // the instruction cache).  Batches of mixed arrays, merged, with one launch per length and mode / per
@@ -97,7 +97,7 @@ cudaError_t launch_merged_pass(const DeviceCtx* d, bool col, int cls, int mode, 
     if (cls == 1) return launch_merged_kernel<true, 128, 5, 512, 256, 128>(mode, n, a, st);
     return launch_merged_kernel<true, 128, 3, 1024>(mode, n, a, st);
   }
-  if (cls == 0) return launch_merged_kernel<false, 32, 12, 64>(mode, n, a, st);
+  if (cls == 0) return launch_merged_kernel<false, 32, 12, 64, 32>(mode, n, a, st);
   if (cls == 1) return launch_merged_kernel<false, 64, 10, 256, 128>(mode, n, a, st);
   if (cls == 2) return launch_merged_kernel<false, 128, 5, 512>(mode, n, a, st);
   return launch_merged_kernel<false, 128, 3, 1024>(mode, n, a, st);

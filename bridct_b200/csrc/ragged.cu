@@ -22,6 +22,7 @@ struct RaggedClass {
   long long* d_offs = nullptr;        // offsets (floats) of those arrays
   size_t floats = 0;                  // elements of the class
   int schedule = BRIDCT_RAGGED_QUEUE;
+  bool merged = false;                // its arrays are in the merged passes
 };
 
 constexpr int kRaggedMaxStreams = 8;
@@ -92,6 +93,16 @@ int block_rows(int h, int w, int budget) {
   return std::min(h, std::max(want, lines_per_warp(w)));
 }
 
+// Queued arrays that run in the merged passes where a batch has them: those that the queue takes through
+// its two passes because no sub-block holds them, with lines that the merged kernels know.  The
+// queue takes about three times as long for them: batches of mixed arrays, queued / joined, us a call:
+// 640 up to 256 x 256 42 / 34, 200 up to 1024 x 1024 81 / 74, 1024 of them 296 / 280.  Below kJoinFloats
+// elements the launches they add cost more (200 up to 256 x 256 27.8 / 29.7, 64 of them 26.9 / 30.9).
+constexpr size_t kJoinFloats = (size_t)1 << 21;
+bool may_join(const RaggedClass& c) {
+  return c.schedule == BRIDCT_RAGGED_QUEUE && !ragged_fits(c.h, c.w) && c.h >= 32 && c.w >= 32;
+}
+
 // Queue order of items a and b: large arrays first (the small ones fill the tail), arrays of one shape
 // and mode together, so that the CTAs of an SM run the same few line programs at a time (in submission
 // order the kernel spent a third of its time waiting for instructions).
@@ -109,7 +120,7 @@ void build_units(bridct_ragged* r) {
   std::vector<int> big, small;
   std::vector<char> queued(r->items.size(), 1);
   for (const RaggedClass& c : r->classes)
-    if (c.schedule != BRIDCT_RAGGED_QUEUE)
+    if (c.schedule != BRIDCT_RAGGED_QUEUE || c.merged)
       for (int i : c.arrays) queued[i] = 0;
   r->arrays.clear();
   for (size_t i = 0; i < r->items.size(); ++i) {
@@ -204,13 +215,13 @@ void free_merged(bridct_ragged* r) {
 int build_merged(bridct_ragged* r) {
   free_merged(r);
   size_t floats = 0;
-  for (const RaggedClass& c : r->classes) floats += c.schedule == BRIDCT_RAGGED_MERGED ? c.floats : 0;
+  for (const RaggedClass& c : r->classes) floats += c.merged ? c.floats : 0;
   const bool all_modes = floats <= kMergedAllModes;
   for (int pass = 0; pass < 2; ++pass) {
     const bool col = pass == 0;
     std::map<std::pair<int, int>, std::vector<MergedUnit>> groups;
     for (const RaggedClass& c : r->classes) {
-      if (c.schedule != BRIDCT_RAGGED_MERGED) continue;
+      if (!c.merged) continue;
       std::vector<MergedUnit>& g = groups[{merged_class(col, col ? c.h : c.w), all_modes ? -1 : c.mode}];
       const int step = col ? merged_strip_cols(c.h) : merged_block_rows(c.w), end = col ? c.w : c.h;
       for (int i : c.arrays)
@@ -499,7 +510,16 @@ BRIDCT_API int bridct_ragged_set_schedule(bridct_ragged* r, const int* schedules
   if (guard.status != cudaSuccess) return cuda_fail(guard.status, "cudaSetDevice(batch device)");
   cudaError_t e = cudaDeviceSynchronize();   // the old queue may still be in use
   if (e != cudaSuccess) return cuda_fail(e, "bridct_ragged_set_schedule");
-  for (size_t i = 0; i < count; ++i) r->classes[i].schedule = schedules[i];
+  bool any_merged = false;
+  size_t merged_floats = 0;   // with the queued classes that may join
+  for (size_t i = 0; i < count; ++i) {
+    RaggedClass& c = r->classes[i];
+    c.schedule = schedules[i];
+    any_merged |= c.schedule == BRIDCT_RAGGED_MERGED;
+    if (c.schedule == BRIDCT_RAGGED_MERGED || may_join(c)) merged_floats += c.floats;
+  }
+  const bool join = any_merged && merged_floats >= kJoinFloats;
+  for (RaggedClass& c : r->classes) c.merged = c.schedule == BRIDCT_RAGGED_MERGED || (join && may_join(c));
   r->streams = streams;
   build_units(r);
   int s = upload(r);
