@@ -87,6 +87,9 @@ int strip_cols(int h, int w, int budget) {
   return std::min(w, std::max(want, std::max(4, lines_per_warp(h))));
 }
 
+// Whether an array is one unit.
+bool one_unit(int h, int w, const bridct_ragged_tuning& t) { return h * w <= t.tile_floats && ragged_fits(h, w); }
+
 // Rows per row block: a power of two dividing h, >= lines_per_warp(w).
 int block_rows(int h, int w, int budget) {
   const int want = pow2_floor(std::max(1, std::min(h, budget / w)));
@@ -116,7 +119,9 @@ bool queue_before(const bridct_ragged_item* items, int a, int b) {
 }
 
 void build_units(bridct_ragged* r) {
-  const bridct_ragged_tuning& t = r->tuning;
+  bridct_ragged_tuning t = r->tuning;
+  t.strip_floats = std::min(t.strip_floats, kRaggedUnit);
+  t.row_floats = std::min(t.row_floats, kRaggedUnit);
   std::vector<int> big, small;
   std::vector<char> queued(r->items.size(), 1);
   for (const RaggedClass& c : r->classes)
@@ -126,10 +131,9 @@ void build_units(bridct_ragged* r) {
   for (size_t i = 0; i < r->items.size(); ++i) {
     const bridct_ragged_item& it = r->items[i];
     RaggedArray a{(long long)it.offset, it.height, it.width, it.mode, 0};
-    const long long e = (long long)it.height * it.width;
     if (!queued[i]) {
       // run by its class's own launch: not in the queue
-    } else if (e <= t.tile_floats) {
+    } else if (one_unit(it.height, it.width, t)) {
       small.push_back((int)i);
     } else {
       a.nstrips = it.width / strip_cols(it.height, it.width, t.strip_floats);
@@ -606,12 +610,15 @@ BRIDCT_API int bridct_ragged_apply_loop_device(bridct_ragged* r, const float* x,
 namespace {
 
 constexpr int kNaMaxArrays = 4096;    // items per call
-constexpr int kNaMaxUnits = 49152;    // work units per call (default unit geometry)
+constexpr int kNaMaxUnits = 49152;    // work units per call, counted in units of the default tuning's sizes
+// The units queued are smaller: strips and row blocks by half, and a whole array that no sub-block
+// holds becomes up to four of them.
+constexpr int kNaQueue = 2 * kNaMaxUnits + 2 * kNaMaxArrays;
 
 struct NaOff {
   static constexpr size_t arrays = 0;
   static constexpr size_t units = arrays + sizeof(bridct::RaggedArray) * kNaMaxArrays;
-  static constexpr size_t counters = units + sizeof(bridct::RaggedUnit) * kNaMaxUnits;
+  static constexpr size_t counters = units + sizeof(bridct::RaggedUnit) * kNaQueue;
   static constexpr size_t err = counters + sizeof(unsigned int) * (kNaMaxArrays + 1);
   static constexpr size_t tabs = (err + sizeof(int) + 255) / 256 * 256;   // split-line tables, N = 128..1024
   static constexpr size_t bytes = tabs + sizeof(float) * bridct::kRaggedTabs;
@@ -619,7 +626,7 @@ struct NaOff {
 
 }  // namespace
 
-// About 0.9 MB: queue (arrays, units), counters, error word, split-line tables.  Host code must
+// About 1.8 MB: queue (arrays, units), counters, error word, split-line tables.  Host code must
 // not use this name as a device address; the entry point resolves it per device below.
 static __device__ __align__(256) unsigned char g_ragged_scratch[NaOff::bytes];
 
@@ -627,7 +634,7 @@ namespace {
 
 std::mutex g_na_mutex;                                  // one call at a time (shared scratch)
 bridct::RaggedArray g_na_arrays[kNaMaxArrays];
-bridct::RaggedUnit g_na_units[kNaMaxUnits];
+bridct::RaggedUnit g_na_units[kNaQueue];
 int g_na_big[kNaMaxArrays];
 int g_na_small[kNaMaxArrays];
 int g_na_order[kNaMaxArrays];
@@ -679,13 +686,17 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
   bridct_ragged_tuning t;
   bridct_ragged_default_tuning(&t);
   int nbig = 0, nsmall = 0;
+  long long limit = 0;   // units of the tuning's sizes
   for (size_t i = 0; i < count; ++i) {
     const bridct_ragged_item& it = items[i];
     RaggedArray a{(long long)it.offset, it.height, it.width, it.mode, 0};
-    if ((long long)it.height * it.width <= t.tile_floats) {
+    const bool tile = (long long)it.height * it.width <= t.tile_floats;
+    limit += tile ? 1 : it.width / strip_cols(it.height, it.width, t.strip_floats) +
+                            it.height / block_rows(it.height, it.width, t.row_floats);
+    if (one_unit(it.height, it.width, t)) {
       g_na_small[nsmall++] = (int)i;
     } else {
-      a.nstrips = it.width / strip_cols(it.height, it.width, t.strip_floats);
+      a.nstrips = it.width / strip_cols(it.height, it.width, std::min(t.strip_floats, kRaggedUnit));
       g_na_big[nbig++] = (int)i;
     }
     g_na_arrays[i] = a;
@@ -694,9 +705,9 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
   std::sort(g_na_big, g_na_big + nbig, order);
   std::sort(g_na_small, g_na_small + nsmall, order);
   int nunits = 0;
-  bool full = false;
+  bool full = limit > kNaMaxUnits;
   auto push = [&](RaggedUnit u) {
-    if (nunits == kNaMaxUnits) full = true;
+    if (nunits == kNaQueue) full = true;
     else g_na_units[nunits++] = u;
   };
   for (int k = 0; k < nbig + t.lookahead; ++k) {
@@ -708,7 +719,7 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
     if (k >= t.lookahead) {
       const int i = g_na_big[k - t.lookahead];
       const RaggedArray& a = g_na_arrays[i];
-      const int rb = block_rows(a.h, a.w, t.row_floats);
+      const int rb = block_rows(a.h, a.w, std::min(t.row_floats, kRaggedUnit));
       for (int r0 = 0; r0 < a.h; r0 += rb) push(RaggedUnit{i, UNIT_ROWBLOCK, r0, rb});
     }
   }

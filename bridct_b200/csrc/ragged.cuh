@@ -1,7 +1,7 @@
 // Batching form: one persistent launch over a mixed-shape, mixed-direction batch.
 //
 // The host turns the batch into a queue of work units:
-//   TILE      one array up to the tuning's tile_floats: both passes
+//   TILE      one array up to the tuning's tile_floats that lies in a sub-block whole: both passes
 //   COLSTRIP  h rows x some columns of a larger array: its column lines, x -> y
 //   ROWBLOCK  some full rows of a larger array: its row lines, y -> y in place
 // CTAs are persistent (one launch, grid = SMs x resident CTAs) and take units in queue order
@@ -14,8 +14,7 @@
 // Line lengths and modes vary per unit and are dispatched at run time to the line pairs of the
 // fixed-shape kernels (sj_split.cuh).  A unit is worked through in sub-blocks of at most 9216 floats of
 // shared memory, so that three CTAs of 128 threads (168 registers: 64-point leaves, two lines per thread)
-// share an SM together with the tables of all four split lengths.  An array whose tile does not fit
-// takes its two passes through y, which stays in L2.  1024 mixed arrays up to 1024 x 1024: 590 us with
+// share an SM together with the tables of all four split lengths.  1024 mixed arrays up to 1024 x 1024: 590 us with
 // one line per thread or line group per warp in 256-thread CTAs of 112 KB, 408 us this way.
 #pragma once
 #include "sj_kernels.cuh"
@@ -53,6 +52,11 @@ struct RaggedArgs {
 
 constexpr int kRaggedThreads = 128;
 constexpr int kRaggedTile = 9216;                                   // floats of a sub-block
+// Floats of a strip or row block at most: one sub-block's.  Units of 16384 floats, and whole arrays of
+// that size as one unit, measured (before / after, us a call of mixed arrays): 16 up to 256 x 256 23 / 17,
+// 200 up to 256 x 256 30 / 24, 64 up to 1024 x 1024 48 / 39, 640 up to 1024 x 1024 237 / 230.  Units of
+// 4096: 15.5, 27, 51 and 353.
+constexpr int kRaggedUnit = 8192;
 constexpr int kRaggedTabs = SplitTab<128>::kFloats + SplitTab<256>::kFloats + SplitTab<512>::kFloats + SplitTab<1024>::kFloats;
 constexpr int kRaggedSmem = (kRaggedTile + kRaggedTabs) * 4;
 constexpr unsigned kRaggedSpin = 1u << 22;                          // x ~256 ns back-off
@@ -300,20 +304,19 @@ __global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged(RaggedArgs a) {
     const int h = arr.h, w = arr.w, mode = arr.mode;
     const float* xa = a.x + arr.offset;
     float* ya = a.y + arr.offset;
-    const bool fits = unit.type == UNIT_TILE && ragged_fits(h, w);
+    const bool whole = unit.type == UNIT_TILE;
     bool rows = unit.type != UNIT_COLSTRIP;
     int first = 0, count = h;
-    if (fits) {
+    if (whole) {
       ragged_load(xa, h, w, tile, ragged_pitch(w));
       ragged_tile_cols_dyn(h, mode, tile, ragged_pitch(w), w, tabs);
       fetch();
-    } else if (unit.type != UNIT_ROWBLOCK) {
-      const int c0 = unit.type == UNIT_COLSTRIP ? unit.first : 0, nc = unit.type == UNIT_COLSTRIP ? unit.count : w;
-      ragged_cols_dyn(h, mode, xa + c0, ya + c0, w, nc, tile, tabs);
+    } else if (unit.type == UNIT_COLSTRIP) {
+      ragged_cols_dyn(h, mode, xa + unit.first, ya + unit.first, w, unit.count, tile, tabs);
       fetch();
       __threadfence();
       __syncthreads();
-      if (unit.type == UNIT_COLSTRIP && threadIdx.x == 0) atomicAdd(a.done + unit.array, 1u);
+      if (threadIdx.x == 0) atomicAdd(a.done + unit.array, 1u);
     } else {
       if (threadIdx.x == 0) {
         int ok = 0;
@@ -336,7 +339,7 @@ __global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged(RaggedArgs a) {
       first = unit.first;
       count = unit.count;
     }
-    if (rows) ragged_row_pass(ya + (long long)first * w, count, w, mode, fits, tile, tabs);
+    if (rows) ragged_row_pass(ya + (long long)first * w, count, w, mode, whole, tile, tabs);
     __syncthreads();
   }
 }

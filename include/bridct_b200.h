@@ -123,9 +123,10 @@ typedef struct {
 
 /* Work-unit geometry of a ragged batch (chosen per shape class by the autotuner). */
 typedef struct {
-    int tile_floats;   /* arrays up to this many floats run both passes in one unit (<= 16384) */
-    int strip_floats;  /* floats per column-strip unit of a larger array (<= 16384)            */
-    int row_floats;    /* floats per row-block unit of a larger array (<= 16384)               */
+    int tile_floats;   /* arrays up to this many floats run both passes in one unit, if its    */
+                       /* shared memory holds them (<= 16384)                                  */
+    int strip_floats;  /* floats per column-strip unit of a larger array (<= 16384; 8192 used) */
+    int row_floats;    /* floats per row-block unit of a larger array (<= 16384; 8192 used)    */
     int lookahead;     /* larger arrays whose strips are queued ahead of a row pass (1..64)   */
 } bridct_ragged_tuning;
 
@@ -196,7 +197,7 @@ BRIDCT_API int bridct_ragged_set_wait_limit(bridct_ragged *batch, unsigned polls
  * allocate device memory (a framework whose caching allocator owns the whole GPU, a loop that
  * cannot afford cudaMalloc's implicit synchronisation, a fixed device footprint): the items and
  * the input/output buffers are passed in, and the work queue, counters and tables live in one
- * static device array of about 0.9 MB that every GPU loading this library holds until exit.
+ * static device array of about 1.8 MB that every GPU loading this library holds until exit.
  * Limits: at most 4096 arrays and 49152 work units per call (default unit geometry), else
  * BRIDCT_INVALID_ARGUMENT with a message.  A successful call allocates nothing.  The first call
  * on a device resolves that array's address and uploads the four-step tables into it.  Every
