@@ -230,13 +230,15 @@ def cpu_single_thread(x: np.ndarray, mode: int, budget_s: float = 0.5):
 
 def tensor_rate(form: str, h: int, w: int, elems_per_s: float, pk: dict):
     """Tensor-core FLOP rate of a form: 2*h*w*P flop per element for the 8x8 Kronecker GEMM,
-    2*(h+w)*P for the two separable passes (P = products: 6 BF16x3, 3 TF32x3, 1 FP8 plus its
+    2*(h+w)*P for the two separable passes, where a split-precision axis of 128 points and more counts
+    half (forward passes fold the row's symmetric halves) (P = products: 6 BF16x3, 3 TF32x3, 1 FP8 plus its
     refinement's second FP8 transform), against the measured bf16 peak (TF32 runs at half the
     bf16 rate and FP8 at twice, nominally)."""
     prods = {"tc_bf16x3": 6, "tc_tf32x3": 3, "tc_fp8": 2}.get(form)
     if prods is None:
         return None
-    per_elem = 2.0 * h * w * prods if (h, w) == (8, 8) else 2.0 * (h + w) * prods
+    length = lambda n: n / 2 if n >= 128 and form != "tc_fp8" else n
+    per_elem = 2.0 * h * w * prods if (h, w) == (8, 8) else 2.0 * (length(h) + length(w)) * prods
     tflops = per_elem * elems_per_s / 1e12
     scale = {"tc_bf16x3": 1.0, "tc_tf32x3": 0.5, "tc_fp8": 2.0}[form]
     peak = pk["bf16_tflops"] * scale

@@ -200,7 +200,7 @@ BRIDCT_API int bridct_ragged_set_wait_limit(bridct_ragged *batch, unsigned polls
  * static device array of about 1.8 MB that every GPU loading this library holds until exit.
  * Limits: at most 4096 arrays and 49152 work units per call (default unit geometry), else
  * BRIDCT_INVALID_ARGUMENT with a message.  A successful call allocates nothing.  The first call
- * on a device resolves that array's address and uploads the four-step tables into it.  Every
+ * on a device resolves that array's address and uploads the split-line tables into it.  Every
  * call shares the array and overwrites the previous call's queue; calls are serialized and
  * synchronous (they return after their kernel finished), because two calls overlapping on the
  * GPU would race on it.  Returns BRIDCT_TIMEOUT if a bounded dependency wait expired. */
