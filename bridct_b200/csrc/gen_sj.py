@@ -543,8 +543,7 @@ def generate() -> str:
 
 # ----------------------------------------------------------------------------------------
 # Programs over a value type T (sj_packed.cuh): T = F2 runs two lines at once with the packed
-# f32x2 instructions, T = float one line.  Both round every operation alike: a multiplication whose
-# only use is an addition is fused here, explicitly, and nothing else is contracted.
+# f32x2 instructions.  A multiplication whose only use is an addition is fused here, explicitly.
 # ----------------------------------------------------------------------------------------
 
 PACKED_LINES = (8, 16, 32, 64)      # whole lines in registers
@@ -649,7 +648,7 @@ def build_special(n: int):
 def generate_packed() -> str:
     parts = [
         "// Generated by gen_sj.py --packed: Shao-Johnson programs over a value type T (F2: two lines at",
-        "// once in packed f32x2 instructions; float: one line, rounded alike).",
+        "// once in packed f32x2 instructions).",
         "// Do not edit by hand; rerun `python gen_sj.py --packed > sj_packed.cuh`.",
         "#pragma once",
         "",
