@@ -45,10 +45,11 @@ __device__ __forceinline__ void b8_transform(float (&v)[64]) {
   }
 }
 
-// x, y: `batch` contiguous 8x8 arrays (16-byte aligned).
+// x, y: `batch` contiguous 8x8 arrays (16-byte aligned).  x is neither __restrict__ nor read with __ldg:
+// it is not read-only for the kernel's lifetime, since the previous kernel of the stream may write it
+// until griddep_wait() returns.
 template <int MODE>
-__global__ void __launch_bounds__(kB8Threads) k_blocks8(const float* __restrict__ x,
-                                                        float* __restrict__ y, long long batch) {
+__global__ void __launch_bounds__(kB8Threads) k_blocks8(const float* x, float* __restrict__ y, long long batch) {
   extern __shared__ float4 s8[];
   // Full rounds: tile r*grid + blockIdx of 256 arrays (all CTAs stream one contiguous region
   // together).  The arrays left after the full rounds are split evenly over all CTAs (fewer
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(kB8Threads) k_blocks8(const float* __restrict_
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
       const int q = t + k * kB8Threads;
-      buf[k] = q < chunks ? __ldg(src + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      buf[k] = q < chunks ? src[q] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int k = 0; k < 16; ++k) s8[b8_slot(t + k * kB8Threads)] = buf[k];
@@ -117,7 +118,7 @@ __device__ __forceinline__ void b8_cp_async16(float4* dst, const float4* src) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kB8dbThreads) k_blocks8_db(const float* __restrict__ x, float* __restrict__ y,
+__global__ void __launch_bounds__(kB8dbThreads) k_blocks8_db(const float* x, float* __restrict__ y,
                                                              long long batch) {
   extern __shared__ float4 s8[];
   const long long round_arrays = (long long)gridDim.x * kB8dbThreads;

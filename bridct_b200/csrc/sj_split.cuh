@@ -596,7 +596,8 @@ __device__ __forceinline__ void pair_col_unit(const float* x, float* y, long lon
   F2 v[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const float2 f = __ldg(reinterpret_cast<const float2*>(x + i * xp));
+    // not __ldg: the previous kernel of the stream may still be writing x until griddep_wait() returns
+    const float2 f = *reinterpret_cast<const float2*>(x + i * xp);
     v[i] = f2_make(f.x, f.y);
   }
   pair_line<N, MODE>(v);

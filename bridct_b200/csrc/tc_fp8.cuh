@@ -140,7 +140,7 @@ constexpr uint32_t kFp8Idesc = (1u << 4) | ((64u >> 3) << 17) | ((uint32_t)(kRow
 // transposed (R = 1 << rshift rows of length L in, L rows of length R out).
 template <int LS, int SUB, int UKT>
 __global__ void __launch_bounds__(256, 1)
-    k_fp8pass(const __grid_constant__ CUtensorMap xmap, const float* __restrict__ sx, float* __restrict__ out,
+    k_fp8pass(const __grid_constant__ CUtensorMap xmap, const float* sx, float* __restrict__ out,
               const uint4* __restrict__ bimage, const float* __restrict__ sc, long long nrows, int rshift,
               int* __restrict__ err) {
   using F = Fp8Layout<LS, SUB, UKT>;
@@ -257,13 +257,14 @@ __global__ void __launch_bounds__(256, 1)
       }
       tc_fence_after();
       const long long gs = (slot + (j / F::kUnits) * nslots) * kRows + r;   // this thread's super-row
-      // data scale of each of the unit's K-tiles: its first row and column band
+      // data scale of each of the unit's K-tiles: its first row and column band (not __ldg: the kernel
+      // before this one writes them, until griddepcontrol.wait returns)
       float rs[UKT];
 #pragma unroll
       for (int kt = 0; kt < UKT; ++kt) {
         const int kg = u * UKT + kt;
         const long long g = gs * SUB + (kg * 32) / L;
-        rs[kt] = g < nrows ? __ldg(sx + (g >> tr_shift) * kBandsPerRow + kg % kBandsPerRow) : 0.0f;
+        rs[kt] = g < nrows ? sx[(g >> tr_shift) * kBandsPerRow + kg % kBandsPerRow] : 0.0f;
       }
       const uint32_t taddr = tmem_base + (uint32_t)(t * UKT * 64) + (quarter << 16);
 #pragma unroll
