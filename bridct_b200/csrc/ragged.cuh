@@ -335,6 +335,9 @@ __global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged(RaggedArgs a) {
       }
       fetch();
       __syncthreads();
+      // The strips of this launch stored y through the generic proxy; the bulk stores below write the same
+      // rows through the async proxy.  No grid boundary lies between, so order the two here.
+      asm volatile("fence.proxy.async.global;" ::: "memory");
       rows = s_ok;
       first = unit.first;
       count = unit.count;

@@ -504,6 +504,9 @@ __device__ __forceinline__ void bulk_commit_wait() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
+// Orders this thread's shared-memory writes before bulk stores that read them.  The global side needs
+// no fence where a grid boundary lies between the ordinary stores to the rows and the bulk stores to
+// them (the two passes, whole-array tiles); the queue of a ragged batch adds its own (ragged.cuh).
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // RB rows, row r at xrow(r) and yrow(r), in place or x -> y.
