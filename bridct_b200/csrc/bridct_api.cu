@@ -60,13 +60,11 @@ double sj_scale(int n, int k) {
 // w_N^{bc} s(A, c), then the post rotations with the stage-2 scale of each output (s(B, j); s(B/2, m)
 // for column A/2) and the orthonormal factor folded in.
 template <int N>
-static std::vector<float> build_split_tables() {
+static void fill_split_tables_n(float* t) {
   constexpr int A = Split<N>::A, B = Split<N>::B, copies = SplitTab<N>::kWords / 2;
-  std::vector<float> t;
-  t.reserve(SplitTab<N>::kFloats);
   auto put = [&t](double x, double y) {
-    t.insert(t.end(), copies, (float)x);
-    t.insert(t.end(), copies, (float)y);
+    for (int i = 0; i < copies; ++i) *t++ = (float)x;
+    for (int i = 0; i < copies; ++i) *t++ = (float)y;
   };
   for (int c = 0; c < A / 2; ++c)
     for (int b = 0; b < B; ++b) {
@@ -84,14 +82,20 @@ static std::vector<float> build_split_tables() {
       const double s = std::sqrt(2.0 / N) * (second ? sj_scale(B / 2, j - B / 2) : sj_scale(B, j));
       put(s * std::cos(M_PI * k / (2.0 * N)), s * std::sin(M_PI * k / (2.0 * N)));
     }
-  return t;
 }
 
-std::vector<float> split_tables_host(int N) {
-  return N == 128   ? build_split_tables<128>()
-         : N == 256 ? build_split_tables<256>()
-         : N == 512 ? build_split_tables<512>()
-                    : build_split_tables<1024>();
+int split_table_floats(int N) {
+  return N == 128   ? SplitTab<128>::kFloats
+         : N == 256 ? SplitTab<256>::kFloats
+         : N == 512 ? SplitTab<512>::kFloats
+                    : SplitTab<1024>::kFloats;
+}
+
+void fill_split_tables(int N, float* t) {
+  if (N == 128) fill_split_tables_n<128>(t);
+  else if (N == 256) fill_split_tables_n<256>(t);
+  else if (N == 512) fill_split_tables_n<512>(t);
+  else fill_split_tables_n<1024>(t);
 }
 
 #define BRIDCT_DECL_H(H) void plain_table_h##H(PlainLauncher (*row)[3]);
@@ -136,7 +140,8 @@ DeviceCtx* device_ctx(int device) {
   plain_table_h512(tab[6]);
   plain_table_h1024(tab[7]);
   for (int i = 0; i < 4; ++i) {
-    const std::vector<float> t = split_tables_host(128 << i);
+    std::vector<float> t(split_table_floats(128 << i));
+    fill_split_tables(128 << i, t.data());
     void* mem = nullptr;
     e = cudaMalloc(&mem, t.size() * sizeof(float));
     if (e == cudaSuccess) {

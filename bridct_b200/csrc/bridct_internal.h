@@ -26,8 +26,10 @@ struct DeviceCtx {
 void set_error(const std::string& s);
 int cuda_fail(cudaError_t e, const char* what);
 double sj_scale(int n, int k);
-// Rotation tables of the split lines of N = 128..1024 points (sj_split.cuh, SplitTab), float64-derived.
-std::vector<float> split_tables_host(int N);
+// Rotation tables of the split lines of N = 128..1024 points (sj_split.cuh, SplitTab), float64-derived:
+// their size, and their values to t.
+int split_table_floats(int N);
+void fill_split_tables(int N, float* t);
 DeviceCtx* device_ctx(int device);
 
 // One unit of a merged pass (merged.cu): a column strip or a row block, starting `off` floats into both

@@ -638,7 +638,8 @@ bridct::RaggedUnit g_na_units[kNaQueue];
 int g_na_big[kNaMaxArrays];
 int g_na_small[kNaMaxArrays];
 int g_na_order[kNaMaxArrays];
-std::vector<float> g_na_tabs;
+float g_na_tabs[bridct::kRaggedTabs];                  // split-line tables, N = 128..1024
+bool g_na_filled = false;
 unsigned char* g_na_addr[64] = {};                      // scratch address per device
 
 // First float of the tables of N = 128 << i.
@@ -738,17 +739,16 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
     set_error("bridct_ragged_apply_noalloc: device index beyond 63");
     return BRIDCT_INVALID_ARGUMENT;
   }
-  if (g_na_tabs.empty())
-    for (int i = 0; i < 4; ++i) {
-      const std::vector<float> t = split_tables_host(128 << i);
-      g_na_tabs.insert(g_na_tabs.end(), t.begin(), t.end());
-    }
+  if (!g_na_filled) {
+    for (int i = 0; i < 4; ++i) fill_split_tables(128 << i, g_na_tabs + na_segment(i));
+    g_na_filled = true;
+  }
   if (!g_na_addr[dev]) {
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_ragged_scratch);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_ragged_scratch)");
     unsigned char* base = static_cast<unsigned char*>(p);
-    e = cudaMemcpy(base + NaOff::tabs, g_na_tabs.data(), g_na_tabs.size() * sizeof(float), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(base + NaOff::tabs, g_na_tabs, sizeof(g_na_tabs), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "scratch tables");
     g_na_addr[dev] = base;
   }
