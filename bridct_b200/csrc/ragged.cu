@@ -37,14 +37,20 @@ struct MergedPass {
   size_t floats = 0;
 };
 
-struct bridct_ragged {
-  int device = 0;
-  bridct::DeviceCtx* dev = nullptr;
-  std::vector<bridct_ragged_item> items;
+// What a batch's schedule runs: the queue and the merged passes, on the host and on the device.
+struct RaggedTables {
   std::vector<bridct::RaggedArray> arrays;
   std::vector<bridct::RaggedUnit> units;
   bridct::RaggedArray* d_arrays = nullptr;
   bridct::RaggedUnit* d_units = nullptr;
+  std::vector<MergedPass> merged;       // column passes first, then row passes
+};
+
+struct bridct_ragged {
+  int device = 0;
+  bridct::DeviceCtx* dev = nullptr;
+  std::vector<bridct_ragged_item> items;
+  RaggedTables tables;
   unsigned int* d_counters = nullptr;   // [0] queue head, [1..n] strips done per array
   int* d_err = nullptr;
   size_t span = 0;                      // floats covered by the batch (max offset + size)
@@ -55,7 +61,6 @@ struct bridct_ragged {
   // shape classes, in decreasing size; classes scheduled as their own launches run on `streams`
   // side streams forked from and joined back into the caller's stream
   std::vector<RaggedClass> classes;
-  std::vector<MergedPass> merged;       // column passes first, then row passes
   int streams = 4;
   cudaStream_t aux[kRaggedMaxStreams] = {};
   cudaEvent_t fork_ev = nullptr, join_ev[kRaggedMaxStreams] = {};
@@ -118,7 +123,8 @@ bool queue_before(const bridct_ragged_item* items, int a, int b) {
   return a < b;
 }
 
-void build_units(bridct_ragged* r) {
+// The queue of the classes' present schedules.
+void build_units(const bridct_ragged* r, RaggedTables& tables) {
   bridct_ragged_tuning t = r->tuning;
   t.strip_floats = std::min(t.strip_floats, kRaggedUnit);
   t.row_floats = std::min(t.row_floats, kRaggedUnit);
@@ -127,7 +133,6 @@ void build_units(bridct_ragged* r) {
   for (const RaggedClass& c : r->classes)
     if (c.schedule != BRIDCT_RAGGED_QUEUE || c.merged)
       for (int i : c.arrays) queued[i] = 0;
-  r->arrays.clear();
   for (size_t i = 0; i < r->items.size(); ++i) {
     const bridct_ragged_item& it = r->items[i];
     RaggedArray a{(long long)it.offset, it.height, it.width, it.mode, 0};
@@ -139,21 +144,20 @@ void build_units(bridct_ragged* r) {
       a.nstrips = it.width / strip_cols(it.height, it.width, t.strip_floats);
       big.push_back((int)i);
     }
-    r->arrays.push_back(a);
+    tables.arrays.push_back(a);
   }
   auto order = [&](int a, int b) { return queue_before(r->items.data(), a, b); };
   std::sort(big.begin(), big.end(), order);
   std::sort(small.begin(), small.end(), order);
-  r->units.clear();
   auto cols = [&](int i) {
-    const RaggedArray& a = r->arrays[i];
+    const RaggedArray& a = tables.arrays[i];
     const int tc = a.w / a.nstrips;
-    for (int s = 0; s < a.nstrips; ++s) r->units.push_back(RaggedUnit{i, UNIT_COLSTRIP, s * tc, tc});
+    for (int s = 0; s < a.nstrips; ++s) tables.units.push_back(RaggedUnit{i, UNIT_COLSTRIP, s * tc, tc});
   };
   auto rows = [&](int i) {
-    const RaggedArray& a = r->arrays[i];
+    const RaggedArray& a = tables.arrays[i];
     const int rb = block_rows(a.h, a.w, t.row_floats);
-    for (int r0 = 0; r0 < a.h; r0 += rb) r->units.push_back(RaggedUnit{i, UNIT_ROWBLOCK, r0, rb});
+    for (int r0 = 0; r0 < a.h; r0 += rb) tables.units.push_back(RaggedUnit{i, UNIT_ROWBLOCK, r0, rb});
   };
   // Column strips of array k+lookahead are queued ahead of the row blocks of array k, so a
   // row block usually finds its strips finished; small arrays fill the tail.
@@ -162,7 +166,7 @@ void build_units(bridct_ragged* r) {
     if (k < big.size()) cols(big[k]);
     if (k >= (size_t)la) rows(big[k - la]);
   }
-  for (int i : small) r->units.push_back(RaggedUnit{i, UNIT_TILE, 0, 0});
+  for (int i : small) tables.units.push_back(RaggedUnit{i, UNIT_TILE, 0, 0});
 }
 
 // Groups the items into shape classes (height, width, mode), largest first, and uploads each
@@ -208,16 +212,17 @@ int build_classes(bridct_ragged* r) {
 // against 88 us a call at 12 M elements, 192 against 182 at 37 M; merged.cu).
 constexpr size_t kMergedAllModes = (size_t)1 << 24;
 
-void free_merged(bridct_ragged* r) {
-  for (MergedPass& m : r->merged) cudaFree(m.d_units);
-  r->merged.clear();
+void free_tables(RaggedTables& tables) {
+  cudaFree(tables.d_arrays);
+  cudaFree(tables.d_units);
+  for (MergedPass& m : tables.merged) cudaFree(m.d_units);
+  tables = RaggedTables{};
 }
 
 // Unit tables of the merged passes: column strips of the MERGED classes grouped by the kernel of their
 // column length, row blocks by that of their row length, each group largest first.  Within a group the
 // units go by line length and mode, so that the CTAs of an SM run few line programs at a time.
-int build_merged(bridct_ragged* r) {
-  free_merged(r);
+int build_merged(const bridct_ragged* r, RaggedTables& tables) {
   size_t floats = 0;
   for (const RaggedClass& c : r->classes) floats += c.merged ? c.floats : 0;
   const bool all_modes = floats <= kMergedAllModes;
@@ -233,7 +238,7 @@ int build_merged(bridct_ragged* r) {
           g.push_back(MergedUnit{(long long)r->items[i].offset + (long long)k * (col ? 1 : c.w), c.w,
                                  (short)(col ? c.h : c.w), (short)c.mode});
     }
-    std::vector<MergedPass> list;
+    const size_t first = tables.merged.size();
     for (auto& kv : groups) {
       std::vector<MergedUnit>& g = kv.second;
       std::stable_sort(g.begin(), g.end(), [](const MergedUnit& a, const MergedUnit& b) {
@@ -249,13 +254,12 @@ int build_merged(bridct_ragged* r) {
       if (e == cudaSuccess) e = cudaMemcpy(m.d_units, g.data(), g.size() * sizeof(MergedUnit), cudaMemcpyHostToDevice);
       if (e != cudaSuccess) {
         cudaFree(m.d_units);
-        free_merged(r);
         return cuda_fail(e, "merged pass tables");
       }
-      list.push_back(m);
+      tables.merged.push_back(m);
     }
-    std::stable_sort(list.begin(), list.end(), [](const MergedPass& a, const MergedPass& b) { return a.floats > b.floats; });
-    r->merged.insert(r->merged.end(), list.begin(), list.end());
+    std::stable_sort(tables.merged.begin() + first, tables.merged.end(),
+                     [](const MergedPass& a, const MergedPass& b) { return a.floats > b.floats; });
   }
   return BRIDCT_OK;
 }
@@ -275,18 +279,30 @@ int launch_class(bridct_ragged* r, const RaggedClass& c, int schedule, const flo
   return launch_plain_layout(r->dev, c.h, c.w, c.mode, x, y, (long long)c.arrays.size(), &l, &l, st);
 }
 
-int upload(bridct_ragged* r) {
-  cudaFree(r->d_arrays);
-  cudaFree(r->d_units);
-  r->d_arrays = nullptr;
-  r->d_units = nullptr;
-  cudaError_t e = cudaMalloc((void**)&r->d_arrays, r->arrays.size() * sizeof(RaggedArray));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&r->d_units, std::max<size_t>(1, r->units.size()) * sizeof(RaggedUnit));
+int upload(RaggedTables& t) {
+  cudaError_t e = cudaMalloc((void**)&t.d_arrays, t.arrays.size() * sizeof(RaggedArray));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&t.d_units, std::max<size_t>(1, t.units.size()) * sizeof(RaggedUnit));
   if (e == cudaSuccess)
-    e = cudaMemcpy(r->d_arrays, r->arrays.data(), r->arrays.size() * sizeof(RaggedArray), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !r->units.empty())
-    e = cudaMemcpy(r->d_units, r->units.data(), r->units.size() * sizeof(RaggedUnit), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(t.d_arrays, t.arrays.data(), t.arrays.size() * sizeof(RaggedArray), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !t.units.empty())
+    e = cudaMemcpy(t.d_units, t.units.data(), t.units.size() * sizeof(RaggedUnit), cudaMemcpyHostToDevice);
   return e == cudaSuccess ? BRIDCT_OK : cuda_fail(e, "ragged upload");
+}
+
+// The tables of the classes' present schedules, in place of the batch's: all of them, or on failure none (the batch
+// keeps the old ones).
+int replace_tables(bridct_ragged* r) {
+  RaggedTables t;
+  build_units(r, t);
+  int s = upload(t);
+  if (!s) s = build_merged(r, t);
+  if (s) {
+    free_tables(t);
+    return s;
+  }
+  std::swap(r->tables, t);
+  free_tables(t);
+  return BRIDCT_OK;
 }
 
 }  // namespace
@@ -355,11 +371,10 @@ BRIDCT_API bridct_ragged* bridct_ragged_create_tuned(const bridct_ragged_item* i
     bridct_ragged_destroy(r);
     return nullptr;
   }
-  build_units(r);
   cudaError_t e = cudaMalloc((void**)&r->d_counters, (count + 1) * sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMalloc((void**)&r->d_err, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(r->d_err, 0, sizeof(int));
-  if (e != cudaSuccess || upload(r) != BRIDCT_OK) {
+  if (e != cudaSuccess || replace_tables(r) != BRIDCT_OK) {
     if (e != cudaSuccess) cuda_fail(e, "bridct_ragged_create");
     bridct_ragged_destroy(r);
     return nullptr;
@@ -370,19 +385,17 @@ BRIDCT_API bridct_ragged* bridct_ragged_create_tuned(const bridct_ragged_item* i
     bridct_ragged_destroy(r);
     return nullptr;
   }
-  r->grid = std::min<long long>((long long)d->sm_count * bps, std::max<size_t>(1, r->units.size()));
+  r->grid = std::min<long long>((long long)d->sm_count * bps, std::max<size_t>(1, r->tables.units.size()));
   return r;
 }
 
 BRIDCT_API void bridct_ragged_destroy(bridct_ragged* r) {
   if (!r) return;
-  cudaFree(r->d_arrays);
-  cudaFree(r->d_units);
+  free_tables(r->tables);
   cudaFree(r->d_counters);
   cudaFree(r->d_err);
   for (auto& kv : r->plans) bridct_plan_destroy(kv.second);
   for (RaggedClass& c : r->classes) cudaFree(c.d_offs);
-  free_merged(r);
   for (int i = 0; i < kRaggedMaxStreams; ++i) {
     if (r->aux[i]) cudaStreamDestroy(r->aux[i]);
     if (r->join_ev[i]) cudaEventDestroy(r->join_ev[i]);
@@ -393,7 +406,7 @@ BRIDCT_API void bridct_ragged_destroy(bridct_ragged* r) {
   delete r;
 }
 
-BRIDCT_API size_t bridct_ragged_units(const bridct_ragged* r) { return r ? r->units.size() : 0; }
+BRIDCT_API size_t bridct_ragged_units(const bridct_ragged* r) { return r ? r->tables.units.size() : 0; }
 
 BRIDCT_API int bridct_ragged_apply_device(bridct_ragged* r, const float* x, float* y, void* stream) {
   if (!r || !x || !y) return BRIDCT_INVALID_ARGUMENT;
@@ -414,20 +427,20 @@ BRIDCT_API int bridct_ragged_apply_device(bridct_ragged* r, const float* x, floa
   for (const RaggedClass& c : r->classes)
     if (c.schedule == BRIDCT_RAGGED_CLASS_LAUNCH || c.schedule == BRIDCT_RAGGED_CLASS_LAUNCH_SMALL) own.push_back(&c);
   size_t ncol = 0;
-  for (const MergedPass& m : r->merged) ncol += m.col ? 1 : 0;
-  const size_t nrow = r->merged.size() - ncol;
+  for (const MergedPass& m : r->tables.merged) ncol += m.col ? 1 : 0;
+  const size_t nrow = r->tables.merged.size() - ncol;
   const size_t widest = std::max(own.size(), std::max(ncol, nrow));
   cudaError_t e = cudaSuccess;
   const int nst = std::max(1, std::min(r->streams, (int)widest));
-  const bool fork = !own.empty() || !r->merged.empty();
+  const bool fork = !own.empty() || !r->tables.merged.empty();
   if (fork) {
     e = cudaEventRecord(r->fork_ev, st);
     for (int i = 0; e == cudaSuccess && i < nst; ++i) e = cudaStreamWaitEvent(r->aux[i], r->fork_ev, 0);
     if (e != cudaSuccess) return cuda_fail(e, "ragged fork");
   }
-  if (!r->merged.empty()) {
+  if (!r->tables.merged.empty()) {
     for (size_t k = 0; k < ncol; ++k) {
-      const int s = launch_merged(r, r->merged[k], x, y, r->aux[k % nst]);
+      const int s = launch_merged(r, r->tables.merged[k], x, y, r->aux[k % nst]);
       if (s) return s;
     }
     // every row block needs its array's column strips: all side streams meet here
@@ -439,7 +452,7 @@ BRIDCT_API int bridct_ragged_apply_device(bridct_ragged* r, const float* x, floa
     for (int i = 1; e == cudaSuccess && i < nst; ++i) e = cudaStreamWaitEvent(r->aux[i], r->mid_fork, 0);
     if (e != cudaSuccess) return cuda_fail(e, "ragged merged barrier");
     for (size_t k = 0; k < nrow; ++k) {
-      const int s = launch_merged(r, r->merged[ncol + k], x, y, r->aux[k % nst]);
+      const int s = launch_merged(r, r->tables.merged[ncol + k], x, y, r->aux[k % nst]);
       if (s) return s;
     }
   }
@@ -447,15 +460,15 @@ BRIDCT_API int bridct_ragged_apply_device(bridct_ragged* r, const float* x, floa
     const int s = launch_class(r, *own[k], own[k]->schedule, x, y, r->aux[k % nst]);
     if (s) return s;
   }
-  if (!r->units.empty()) {
+  if (!r->tables.units.empty()) {
     e = cudaMemsetAsync(r->d_counters, 0, (r->items.size() + 1) * sizeof(unsigned int), st);
     if (e != cudaSuccess) return cuda_fail(e, "ragged reset");
     RaggedArgs args;
     args.x = x;
     args.y = y;
-    args.arrays = r->d_arrays;
-    args.units = r->d_units;
-    args.nunits = (int)r->units.size();
+    args.arrays = r->tables.d_arrays;
+    args.units = r->tables.d_units;
+    args.nunits = (int)r->tables.units.size();
     args.next = r->d_counters;
     args.done = r->d_counters + 1;
     args.err = r->d_err;
@@ -477,7 +490,7 @@ BRIDCT_API size_t bridct_ragged_class_count(const bridct_ragged* r) { return r ?
 
 BRIDCT_API size_t bridct_ragged_launch_count(const bridct_ragged* r) {
   if (!r) return 0;
-  size_t n = r->merged.size() + (r->units.empty() ? 0 : 1);
+  size_t n = r->tables.merged.size() + (r->tables.units.empty() ? 0 : 1);
   for (const RaggedClass& c : r->classes)
     if (c.schedule == BRIDCT_RAGGED_CLASS_LAUNCH || c.schedule == BRIDCT_RAGGED_CLASS_LAUNCH_SMALL)
       n += c.h * c.w <= 16384 ? 1 : 2;
@@ -514,6 +527,8 @@ BRIDCT_API int bridct_ragged_set_schedule(bridct_ragged* r, const int* schedules
   if (guard.status != cudaSuccess) return cuda_fail(guard.status, "cudaSetDevice(batch device)");
   cudaError_t e = cudaDeviceSynchronize();   // the old queue may still be in use
   if (e != cudaSuccess) return cuda_fail(e, "bridct_ragged_set_schedule");
+  std::vector<std::pair<int, bool>> before;   // schedules and merged flags, kept if the tables cannot be made
+  for (const RaggedClass& c : r->classes) before.push_back({c.schedule, c.merged});
   bool any_merged = false;
   size_t merged_floats = 0;   // with the queued classes that may join
   for (size_t i = 0; i < count; ++i) {
@@ -524,14 +539,18 @@ BRIDCT_API int bridct_ragged_set_schedule(bridct_ragged* r, const int* schedules
   }
   const bool join = any_merged && merged_floats >= kJoinFloats;
   for (RaggedClass& c : r->classes) c.merged = c.schedule == BRIDCT_RAGGED_MERGED || (join && may_join(c));
+  const int s = replace_tables(r);
+  if (s) {
+    for (size_t i = 0; i < count; ++i) {
+      r->classes[i].schedule = before[i].first;
+      r->classes[i].merged = before[i].second;
+    }
+    return s;
+  }
   r->streams = streams;
-  build_units(r);
-  int s = upload(r);
-  if (!s) s = build_merged(r);
-  if (s) return s;
   const int bps = kernel_setup(reinterpret_cast<const void*>(k_ragged), kRaggedSmem, kRaggedThreads);
   r->grid = (int)std::min<long long>((long long)r->dev->sm_count * std::max(1, bps),
-                                     std::max<size_t>(1, r->units.size()));
+                                     std::max<size_t>(1, r->tables.units.size()));
   return BRIDCT_OK;
 }
 
