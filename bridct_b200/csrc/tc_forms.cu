@@ -146,7 +146,8 @@ std::vector<double> dct_matrix(int L) {
 // laid out [K-chunk][split][8 KB atom column]; B[n][k] = C_L[n][k] (forward) or C_L[k][n].  With
 // SUB > 1 the 64-float super-rows hold SUB rows of LS = 64 / SUB points, and B is block-diagonal:
 // SUB copies of C_LS (zeros elsewhere).  Folded forward: row n of slice nb is coefficient
-// 2 (kNBlock (nb / 2) + n) + nb % 2, K runs over the first L / 2 samples.  Folded inverse: row n is sample
+// 2 (kNBlock (nb / 2) + n) + nb % 2, K runs over the first L / 2 samples, and the values are doubled (the
+// kernel halves the folded samples).  Folded inverse: row n is sample
 // 64 nb + n, and within a K-chunk the even coefficients come first.
 template <int FORM, int L, int SUB, int FOLD>
 std::vector<uint8_t> pass_image(bool inverse) {
@@ -161,7 +162,7 @@ std::vector<uint8_t> pass_image(bool inverse) {
       const int nb = n / NB, nl = n % NB, kc = k / kc_len, kk = k % kc_len;
       double v;
       if (FOLD == tc::FOLD_FWD) {
-        v = c[(size_t)(2 * (NB * (nb / 2) + nl) + nb % 2) * L + k];
+        v = 2 * c[(size_t)(2 * (NB * (nb / 2) + nl) + nb % 2) * L + k];
       } else if (FOLD == tc::FOLD_INV) {
         const int coef = kc * kc_len + (kk < kc_len / 2 ? 2 * kk : 2 * (kk - kc_len / 2) + 1);
         v = c[(size_t)coef * L + n];

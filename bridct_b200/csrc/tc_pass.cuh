@@ -17,8 +17,8 @@
 // run as 64-float super-rows against a block-diagonal B (SUB).
 // Rows of 128 points and more use the symmetry of C_L (PassFold), which halves the products, and for
 // every output also the loads and splits:
-//   forward  u[j] = x[j] + x[L-1-j] and v[j] = x[j] - x[L-1-j], j < L/2, give the even and the odd
-//            coefficients as products of length L/2; an N-block is 64 even or 64 odd columns, and the
+//   forward  u[j] = (x[j] + x[L-1-j]) / 2 and v[j] = (x[j] - x[L-1-j]) / 2, j < L/2, give the even and the
+//            odd coefficients as products of length L/2 with 2 C_L; an N-block is 64 even or 64 odd columns, and the
 //            split groups fold the row while they split it
 //   inverse  e[j] = sum over even k, o[j] = sum over odd k of C[k][j] X[k], j < L/2, give
 //            y[j] = e + o and y[L-1-j] = e - o; the split groups put the even elements of a K-chunk
@@ -146,12 +146,15 @@ __device__ __forceinline__ void split_box_tf32(uint8_t* stage, uint8_t* abuf, ui
   }
 }
 
-// Folded splits: element i of the folded chunk is a[i] + sign * b[last - i], with a the chunk's row of
-// the first half of the matrix row and b that of the mirrored chunk.
+// Folded splits: element i of the folded chunk is (a[i] + sign * b[last - i]) / 2, with a the chunk's row of
+// the first half of the matrix row and b that of the mirrored chunk.  Halved, because the sum itself leaves
+// FP32's range for inputs above half of it, whose transform does not; the coefficient images hold
+// twice the matrix, and both scalings are exact.
+__device__ __forceinline__ float fold_half(float a, float b, float half_sign) { return fmaf(half_sign, b, 0.5f * a); }
 // BF16x3: boxes a0, a1, b0, b1 of 16 KB.  hi goes to a0, lo to a1, mid to b1; each half of the chunk
 // reads its two source rows completely before it writes there, and lo of the first half, which would
 // overwrite a1, waits in registers.
-__device__ __forceinline__ void split_fold_bf16(uint8_t* stage, uint32_t r, float sign) {
+__device__ __forceinline__ void split_fold_bf16(uint8_t* stage, uint32_t r, float hs) {
   uint32_t lo0[4][4];
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
@@ -160,10 +163,10 @@ __device__ __forceinline__ void split_fold_bf16(uint8_t* stage, uint32_t r, floa
     for (int c = 0; c < 8; ++c) {
       const float4 u = *reinterpret_cast<const float4*>(stage + half * 16384u + sw128(r, c));
       const float4 w = *reinterpret_cast<const float4*>(stage + (half ? 32768u : 49152u) + sw128(r, 7 - c));
-      x[4 * c] = fmaf(sign, w.w, u.x);
-      x[4 * c + 1] = fmaf(sign, w.z, u.y);
-      x[4 * c + 2] = fmaf(sign, w.y, u.z);
-      x[4 * c + 3] = fmaf(sign, w.x, u.w);
+      x[4 * c] = fold_half(u.x, w.w, hs);
+      x[4 * c + 1] = fold_half(u.y, w.z, hs);
+      x[4 * c + 2] = fold_half(u.z, w.y, hs);
+      x[4 * c + 3] = fold_half(u.w, w.x, hs);
     }
 #pragma unroll
     for (int jq = 0; jq < 4; ++jq) {
@@ -187,7 +190,7 @@ __device__ __forceinline__ void split_fold_bf16(uint8_t* stage, uint32_t r, floa
         make_uint4(lo0[jq][0], lo0[jq][1], lo0[jq][2], lo0[jq][3]);
 }
 // BF16x3, K-chunks of 32: boxes a, b; a row of box a becomes hi (64 bytes) and mid, that of box b lo.
-__device__ __forceinline__ void split_fold_bf16_half(uint8_t* stage, uint32_t r, float sign) {
+__device__ __forceinline__ void split_fold_bf16_half(uint8_t* stage, uint32_t r, float hs) {
   float4 w[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(stage + 16384u + sw128(r, j));
@@ -198,10 +201,10 @@ __device__ __forceinline__ void split_fold_bf16_half(uint8_t* stage, uint32_t r,
     const float4 u1 = *reinterpret_cast<const float4*>(stage + sw128(r, 2 * q + 1));
     const float4 w0 = w[7 - 2 * q], w1 = w[6 - 2 * q];
     uint32_t hi[4], lo[4];
-    split_bf16x3_pair(fmaf(sign, w0.w, u0.x), fmaf(sign, w0.z, u0.y), hi[0], mid[q][0], lo[0]);
-    split_bf16x3_pair(fmaf(sign, w0.y, u0.z), fmaf(sign, w0.x, u0.w), hi[1], mid[q][1], lo[1]);
-    split_bf16x3_pair(fmaf(sign, w1.w, u1.x), fmaf(sign, w1.z, u1.y), hi[2], mid[q][2], lo[2]);
-    split_bf16x3_pair(fmaf(sign, w1.y, u1.z), fmaf(sign, w1.x, u1.w), hi[3], mid[q][3], lo[3]);
+    split_bf16x3_pair(fold_half(u0.x, w0.w, hs), fold_half(u0.y, w0.z, hs), hi[0], mid[q][0], lo[0]);
+    split_bf16x3_pair(fold_half(u0.z, w0.y, hs), fold_half(u0.w, w0.x, hs), hi[1], mid[q][1], lo[1]);
+    split_bf16x3_pair(fold_half(u1.x, w1.w, hs), fold_half(u1.y, w1.z, hs), hi[2], mid[q][2], lo[2]);
+    split_bf16x3_pair(fold_half(u1.z, w1.y, hs), fold_half(u1.w, w1.x, hs), hi[3], mid[q][3], lo[3]);
     *reinterpret_cast<uint4*>(stage + sw128(r, q)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(stage + 16384u + sw128(r, q)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
@@ -210,7 +213,7 @@ __device__ __forceinline__ void split_fold_bf16_half(uint8_t* stage, uint32_t r,
     *reinterpret_cast<uint4*>(stage + sw128(r, 4 + q)) = make_uint4(mid[q][0], mid[q][1], mid[q][2], mid[q][3]);
 }
 // TF32x3: boxes a, b; hi goes to a, lo to b.
-__device__ __forceinline__ void split_fold_tf32(uint8_t* stage, uint32_t r, float sign) {
+__device__ __forceinline__ void split_fold_tf32(uint8_t* stage, uint32_t r, float hs) {
   float4 w[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const float4*>(stage + 16384u + sw128(r, j));
@@ -219,8 +222,8 @@ __device__ __forceinline__ void split_fold_tf32(uint8_t* stage, uint32_t r, floa
     const uint32_t off = sw128(r, j);
     const float4 u = *reinterpret_cast<const float4*>(stage + off);
     uint4 h, l;
-    split_tf32x2(make_float4(fmaf(sign, w[7 - j].w, u.x), fmaf(sign, w[7 - j].z, u.y), fmaf(sign, w[7 - j].y, u.z),
-                             fmaf(sign, w[7 - j].x, u.w)),
+    split_tf32x2(make_float4(fold_half(u.x, w[7 - j].w, hs), fold_half(u.y, w[7 - j].z, hs), fold_half(u.z, w[7 - j].y, hs),
+                             fold_half(u.w, w[7 - j].x, hs)),
                  h, l);
     *reinterpret_cast<uint4*>(stage + off) = h;
     *reinterpret_cast<uint4*>(stage + 16384u + off) = l;
@@ -558,10 +561,10 @@ __global__ void __launch_bounds__(kPassThreads, 1)
       uint8_t* stage = base + s * PL::kStageStride;
       uint8_t* abuf = base + PL::kAOff + a * F::kABufBytes;
       if constexpr (FOLD == FOLD_FWD) {
-        const float sign = nblk & 1 ? -1.0f : 1.0f;
-        if constexpr (PL::kHalf) split_fold_bf16_half(stage, r, sign);
-        else if constexpr (FORM == BF16X3) split_fold_bf16(stage, r, sign);
-        else split_fold_tf32(stage, r, sign);
+        const float hs = nblk & 1 ? -0.5f : 0.5f;
+        if constexpr (PL::kHalf) split_fold_bf16_half(stage, r, hs);
+        else if constexpr (FORM == BF16X3) split_fold_bf16(stage, r, hs);
+        else split_fold_tf32(stage, r, hs);
       } else if constexpr (FOLD == FOLD_INV) {
         if constexpr (FORM == BF16X3) split_deint_bf16(stage, abuf, r);
         else split_deint_tf32(stage, abuf, r);
