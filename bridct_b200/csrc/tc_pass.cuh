@@ -150,7 +150,15 @@ __device__ __forceinline__ void split_box_tf32(uint8_t* stage, uint8_t* abuf, ui
 // the first half of the matrix row and b that of the mirrored chunk.  Halved, because the sum itself leaves
 // FP32's range for inputs above half of it, whose transform does not; the coefficient images hold
 // twice the matrix, and both scalings are exact.
-__device__ __forceinline__ float fold_half(float a, float b, float half_sign) { return fmaf(half_sign, b, 0.5f * a); }
+// The halving is packed: one instruction for two values.
+__device__ __forceinline__ float4 half4(float4 v) {
+  asm("{\n .reg .b64 a, h;\n mov.b64 h, {%4, %4};\n"
+      " mov.b64 a, {%0, %1};\n mul.rn.f32x2 a, a, h;\n mov.b64 {%0, %1}, a;\n"
+      " mov.b64 a, {%2, %3};\n mul.rn.f32x2 a, a, h;\n mov.b64 {%2, %3}, a;\n}\n"
+      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+      : "f"(0.5f));
+  return v;
+}
 // BF16x3: boxes a0, a1, b0, b1 of 16 KB.  hi goes to a0, lo to a1, mid to b1; each half of the chunk
 // reads its two source rows completely before it writes there, and lo of the first half, which would
 // overwrite a1, waits in registers.
@@ -161,12 +169,12 @@ __device__ __forceinline__ void split_fold_bf16(uint8_t* stage, uint32_t r, floa
     float x[32];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const float4 u = *reinterpret_cast<const float4*>(stage + half * 16384u + sw128(r, c));
+      const float4 u = half4(*reinterpret_cast<const float4*>(stage + half * 16384u + sw128(r, c)));
       const float4 w = *reinterpret_cast<const float4*>(stage + (half ? 32768u : 49152u) + sw128(r, 7 - c));
-      x[4 * c] = fold_half(u.x, w.w, hs);
-      x[4 * c + 1] = fold_half(u.y, w.z, hs);
-      x[4 * c + 2] = fold_half(u.z, w.y, hs);
-      x[4 * c + 3] = fold_half(u.w, w.x, hs);
+      x[4 * c] = fmaf(hs, w.w, u.x);
+      x[4 * c + 1] = fmaf(hs, w.z, u.y);
+      x[4 * c + 2] = fmaf(hs, w.y, u.z);
+      x[4 * c + 3] = fmaf(hs, w.x, u.w);
     }
 #pragma unroll
     for (int jq = 0; jq < 4; ++jq) {
@@ -197,14 +205,14 @@ __device__ __forceinline__ void split_fold_bf16_half(uint8_t* stage, uint32_t r,
   uint32_t mid[4][4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {   // elements 8q .. 8q + 7
-    const float4 u0 = *reinterpret_cast<const float4*>(stage + sw128(r, 2 * q));
-    const float4 u1 = *reinterpret_cast<const float4*>(stage + sw128(r, 2 * q + 1));
+    const float4 u0 = half4(*reinterpret_cast<const float4*>(stage + sw128(r, 2 * q)));
+    const float4 u1 = half4(*reinterpret_cast<const float4*>(stage + sw128(r, 2 * q + 1)));
     const float4 w0 = w[7 - 2 * q], w1 = w[6 - 2 * q];
     uint32_t hi[4], lo[4];
-    split_bf16x3_pair(fold_half(u0.x, w0.w, hs), fold_half(u0.y, w0.z, hs), hi[0], mid[q][0], lo[0]);
-    split_bf16x3_pair(fold_half(u0.z, w0.y, hs), fold_half(u0.w, w0.x, hs), hi[1], mid[q][1], lo[1]);
-    split_bf16x3_pair(fold_half(u1.x, w1.w, hs), fold_half(u1.y, w1.z, hs), hi[2], mid[q][2], lo[2]);
-    split_bf16x3_pair(fold_half(u1.z, w1.y, hs), fold_half(u1.w, w1.x, hs), hi[3], mid[q][3], lo[3]);
+    split_bf16x3_pair(fmaf(hs, w0.w, u0.x), fmaf(hs, w0.z, u0.y), hi[0], mid[q][0], lo[0]);
+    split_bf16x3_pair(fmaf(hs, w0.y, u0.z), fmaf(hs, w0.x, u0.w), hi[1], mid[q][1], lo[1]);
+    split_bf16x3_pair(fmaf(hs, w1.w, u1.x), fmaf(hs, w1.z, u1.y), hi[2], mid[q][2], lo[2]);
+    split_bf16x3_pair(fmaf(hs, w1.y, u1.z), fmaf(hs, w1.x, u1.w), hi[3], mid[q][3], lo[3]);
     *reinterpret_cast<uint4*>(stage + sw128(r, q)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     *reinterpret_cast<uint4*>(stage + 16384u + sw128(r, q)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
@@ -220,10 +228,10 @@ __device__ __forceinline__ void split_fold_tf32(uint8_t* stage, uint32_t r, floa
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const uint32_t off = sw128(r, j);
-    const float4 u = *reinterpret_cast<const float4*>(stage + off);
+    const float4 u = half4(*reinterpret_cast<const float4*>(stage + off));
     uint4 h, l;
-    split_tf32x2(make_float4(fold_half(u.x, w[7 - j].w, hs), fold_half(u.y, w[7 - j].z, hs), fold_half(u.z, w[7 - j].y, hs),
-                             fold_half(u.w, w[7 - j].x, hs)),
+    split_tf32x2(make_float4(fmaf(hs, w[7 - j].w, u.x), fmaf(hs, w[7 - j].z, u.y), fmaf(hs, w[7 - j].y, u.z),
+                             fmaf(hs, w[7 - j].x, u.w)),
                  h, l);
     *reinterpret_cast<uint4*>(stage + off) = h;
     *reinterpret_cast<uint4*>(stage + 16384u + off) = l;
