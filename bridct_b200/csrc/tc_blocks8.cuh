@@ -128,6 +128,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
+// Waits until use u of a ring stage is full, for the leader of one of two groups that take the ring's uses in
+// turn.  A parity wait tells a phase from the one before it only.  With an odd number of stages a
+// stage's uses go to the groups alternately, so a leader has not seen use u - 1 complete, and loads may
+// land out of order: the wait for use u would end at once while use u - 1 is still on its way, and the group
+// would split what is not there.  It first waits until use u - 1 has been freed, which the load of use
+// u waits for anyway.
+template <int STAGES>
+__device__ __forceinline__ bool ring_wait(uint32_t stage_full, uint32_t stage_free, uint32_t u) {
+  if (STAGES % 2 && !mbar_wait(stage_free, (u & 1u) ^ 1u)) return false;
+  return mbar_wait(stage_full, u & 1u);
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y,
                                             uint32_t bar) {
   asm volatile(
@@ -448,7 +460,7 @@ __global__ void __launch_bounds__(kTc8Threads, 1) k_tc8(const __grid_constant__ 
     for (int j = grp; j < ntile_local; j += 2) {
       const int s = j % kStages, a = j % kABufs;
       if (r == 0) {
-        bool g = !s_abort && mbar_wait(bars.stage_full + 8 * s, (uint32_t)(j / kStages) & 1u);
+        bool g = !s_abort && ring_wait<kStages>(bars.stage_full + 8 * s, bars.stage_free + 8 * s, (uint32_t)(j / kStages));
         if (g) g = mbar_wait(bars.a_free + 8 * a, ((uint32_t)(j / kABufs) & 1u) ^ 1u);
         s_group_ok[ok_slot] = g ? 1 : 0;
       }

@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     for (long long j = grp; j < nchunk_local; j += 2) {
       const int s = (int)(j % kStages), a = (int)(j & 1);
       if (r == 0) {
-        bool g = !s_abort && mbar_wait(bars.stage_full + 8 * s, (uint32_t)(j / kStages) & 1u);
+        bool g = !s_abort && ring_wait<kStages>(bars.stage_full + 8 * s, bars.stage_free + 8 * s, (uint32_t)(j / kStages));
         if (FOLD != FOLD_FWD && g) g = mbar_wait(bars.a_free + 8 * a, ((uint32_t)(j >> 1) & 1u) ^ 1u);
         s_group_ok[ok_slot] = g ? 1 : 0;
       }
