@@ -127,7 +127,7 @@ std::vector<uint8_t> b_image(int form, bool inverse) {
 
 struct TcDevice {
   void* images[3][2] = {};   // [form][inverse]
-  void* pass_images[3][8][3] = {};   // [form][log2(points per row) - 3][forward, inverse, folded inverse], on first use
+  void* pass_images[3][8][2][2] = {};   // [form][log2(points per row) - 3][inverse][narrow], on first use
   void* fp8_images[8][2] = {};       // [log2(L) - 3][inverse]: E4M3 codes of C or C^T (block-diagonal below 128)
   float* fp8_scales[8][2] = {};      // their 32x32 tile scales
   int* err = nullptr;
@@ -148,10 +148,10 @@ std::vector<double> dct_matrix(int L) {
 // SUB copies of C_LS (zeros elsewhere).  Folded forward: row n of slice nb is coefficient
 // 2 (kNBlock (nb / 2) + n) + nb % 2, K runs over the first L / 2 samples, and the values are doubled (the
 // kernel halves the folded samples).  Folded inverse: row n is sample
-// 64 nb + n, and within a K-chunk the even coefficients come first.
-template <int FORM, int L, int SUB, int FOLD>
+// kNBlock nb + n, and within a K-chunk the even coefficients come first.
+template <int FORM, int L, int SUB, int FOLD, bool NARROW>
 std::vector<uint8_t> pass_image(bool inverse) {
-  using PL = tc::PassLayout<FORM, L, FOLD>;
+  using PL = tc::PassLayout<FORM, L, FOLD, NARROW>;
   constexpr int kc_len = tc::PassForm<FORM>::kKC;
   constexpr int LS = L / SUB;
   const std::vector<double> c = dct_matrix(LS);
@@ -298,13 +298,13 @@ bool make_rows_map(CUtensorMap* m, const float* ptr, size_t rows, int L) {
 
 constexpr int lg_points(int n) { return n <= 8 ? 0 : 1 + lg_points(n / 2); }
 
-template <int FORM, int L, int SUB = 1, int FOLD = tc::FOLD_NONE>
+template <int FORM, int L, int SUB, int FOLD, bool NARROW>
 const uint4* pass_image_device(TcDevice* d, bool inverse) {
   constexpr int li = lg_points(L / SUB);
   std::lock_guard<std::mutex> lock(g_tc_mutex);
-  void*& slot = d->pass_images[FORM][li][!inverse ? 0 : FOLD == tc::FOLD_NONE ? 1 : 2];
+  void*& slot = d->pass_images[FORM][li][inverse ? 1 : 0][NARROW ? 1 : 0];
   if (!slot) {
-    const std::vector<uint8_t> img = pass_image<FORM, L, SUB, FOLD>(inverse);
+    const std::vector<uint8_t> img = pass_image<FORM, L, SUB, FOLD, NARROW>(inverse);
     void* ptr = nullptr;
     if (cudaMalloc(&ptr, img.size()) != cudaSuccess) return nullptr;
     if (cudaMemcpy(ptr, img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -318,14 +318,14 @@ const uint4* pass_image_device(TcDevice* d, bool inverse) {
 
 // One row pass: rows x (L / SUB) matrix at x -> transposed arrays (R = 1 << rshift rows each) at
 // out.  SUB > 1: the rows are read as rows / SUB super-rows of L = 64 floats.
-template <int FORM, int L, int SUB, int FOLD>
-int launch_pass_fold(const bridct_plan* p, bool inverse, const float* x, float* out, size_t rows, int rshift,
-                     cudaStream_t st, TcDevice* d) {
-  using PL = tc::PassLayout<FORM, L, FOLD>;
-  auto k = tc::k_tcpass<FORM, L, SUB, FOLD>;
+template <int FORM, int L, int SUB, int FOLD, bool NARROW>
+int launch_pass_width(const bridct_plan* p, bool inverse, const float* x, float* out, size_t rows, int rshift,
+                      cudaStream_t st, TcDevice* d) {
+  using PL = tc::PassLayout<FORM, L, FOLD, NARROW>;
+  auto k = tc::k_tcpass<FORM, L, SUB, FOLD, NARROW>;
   if (kernel_setup(reinterpret_cast<const void*>(k), PL::kDynamic, tc::kPassThreads) <= 0)
     return cuda_fail(cudaErrorInvalidConfiguration, "k_tcpass shared memory");
-  const uint4* img = pass_image_device<FORM, L, SUB, FOLD>(d, inverse);
+  const uint4* img = pass_image_device<FORM, L, SUB, FOLD, NARROW>(d, inverse);
   if (!img) return cuda_fail(cudaGetLastError(), "tensor-core coefficient upload");
   const size_t srows = rows / SUB;   // SUB divides every array's row count (>= 8)
   CUtensorMap xm;
@@ -341,24 +341,30 @@ int launch_pass_fold(const bridct_plan* p, bool inverse, const float* x, float* 
                              img, (long long)srows, rshift, d->err);
   return e == cudaSuccess ? BRIDCT_OK : cuda_fail(e, "k_tcpass launch");
 }
+template <int FORM, int L, int SUB, int FOLD>
+int launch_pass_fold(const bridct_plan* p, bool inverse, const float* x, float* out, size_t rows, int rshift,
+                     cudaStream_t st, TcDevice* d) {
+  if constexpr (tc::pass_has_narrow(L, FOLD)) {
+    // Narrow N-blocks where the wide ones would leave half of the SMs idle: us a call on 2^18 elements, wide /
+    // narrow, BF16x3: 256x256 forward 15.6 / 13.0, inverse 18.7 / 16.1; 128x128 inverse 13.9 / 11.6; 512x512 inverse
+    // 29.4 / 26.7; 1024x1024 inverse on 2^20 48.8 / 45.7.  Both images are uploaded by the first call, whichever
+    // pass it takes, so that a later one can be captured.
+    if (!pass_image_device<FORM, L, SUB, FOLD, false>(d, inverse) || !pass_image_device<FORM, L, SUB, FOLD, true>(d, inverse))
+      return cuda_fail(cudaGetLastError(), "tensor-core coefficient upload");
+    const size_t mtiles = (rows + tc::kRows - 1) / tc::kRows;
+    if (mtiles * tc::PassLayout<FORM, L, FOLD>::kBlocks * 2 <= (size_t)p->dev->sm_count)
+      return launch_pass_width<FORM, L, SUB, FOLD, true>(p, inverse, x, out, rows, rshift, st, d);
+  }
+  return launch_pass_width<FORM, L, SUB, FOLD, false>(p, inverse, x, out, rows, rshift, st, d);
+}
 template <int FORM, int L, int SUB = 1>
 int launch_pass(const bridct_plan* p, bool inverse, const float* x, float* out, size_t rows, int rshift,
                 cudaStream_t st, TcDevice* d) {
   if constexpr (L >= 128) {
     // TF32x3 inverses of 512 and 1024 points would accumulate 5..15% less exactly folded.
     constexpr int inv = L <= 256 || FORM == tc::BF16X3 ? tc::FOLD_INV : tc::FOLD_NONE;
-    if (!inverse) return launch_pass_fold<FORM, L, SUB, tc::FOLD_FWD>(p, inverse, x, out, rows, rshift, st, d);
-    if constexpr (inv != tc::FOLD_NONE) {
-      // A folded N-block holds twice the columns, so where its CTAs would leave half of the SMs idle the
-      // unfolded pass is faster (by 5..15% on 2^20 elements).  Both images are uploaded by the first call,
-      // whichever pass it takes, so that a later one can be captured.
-      const size_t mtiles = (rows + tc::kRows - 1) / tc::kRows;
-      if (!pass_image_device<FORM, L, SUB, inv>(d, inverse) || !pass_image_device<FORM, L, SUB, tc::FOLD_NONE>(d, inverse))
-        return cuda_fail(cudaGetLastError(), "tensor-core coefficient upload");
-      if (mtiles * tc::PassLayout<FORM, L, inv>::kBlocks * 2 > (size_t)p->dev->sm_count)
-        return launch_pass_fold<FORM, L, SUB, inv>(p, inverse, x, out, rows, rshift, st, d);
-    }
-    return launch_pass_fold<FORM, L, SUB, tc::FOLD_NONE>(p, inverse, x, out, rows, rshift, st, d);
+    return inverse ? launch_pass_fold<FORM, L, SUB, inv>(p, true, x, out, rows, rshift, st, d)
+                   : launch_pass_fold<FORM, L, SUB, tc::FOLD_FWD>(p, false, x, out, rows, rshift, st, d);
   } else {
     return launch_pass_fold<FORM, L, SUB, tc::FOLD_NONE>(p, inverse, x, out, rows, rshift, st, d);
   }
@@ -370,7 +376,7 @@ int launch_fused64(const bridct_plan* p, bool inverse, const float* x, float* y,
   using F = tc::Fused64;
   if (kernel_setup(reinterpret_cast<const void*>(tc::k_tc64), F::kDynamic, F::kThreads) <= 0)
     return cuda_fail(cudaErrorInvalidConfiguration, "k_tc64 shared memory");
-  const uint4* img = pass_image_device<tc::BF16X3, 64>(d, inverse);
+  const uint4* img = pass_image_device<tc::BF16X3, 64, 1, tc::FOLD_NONE, false>(d, inverse);
   if (!img) return cuda_fail(cudaGetLastError(), "tensor-core coefficient upload");
   CUtensorMap xm;
   if (!make_rows_map(&xm, x, batch * 64, 64)) {

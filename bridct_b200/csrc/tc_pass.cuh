@@ -68,7 +68,13 @@ enum PassFold { FOLD_NONE = 0, FOLD_FWD = 1, FOLD_INV = 2 };
 
 // Output columns per CTA (MMA N).  Folded forward passes of 256 points take 128, all columns of one
 // parity: with 64, every M-tile crosses from L2 four times, and that traffic (4.9 TB/s) bounds the pass.
+// NARROW: half as many, for calls whose wide CTAs would leave half of the SMs idle.  An accumulator's
+// products and their order are the same either way (PassAccs), so a row's results have the same
+// bits in a call of any size.
 __host__ __device__ constexpr int pass_nblock(int L, int fold) { return fold == FOLD_FWD && L == 256 ? 128 : 64; }
+__host__ __device__ constexpr bool pass_has_narrow(int L, int fold) {
+  return fold == FOLD_INV || (fold == FOLD_FWD && L == 256);
+}
 
 // Folded BF16x3 forward passes of 128 and 256 points run K-chunks of 32: the same ring then holds twice
 // the stages, and loads, splits and products of one M-tile overlap more finely (16 M elements at 256 x 256:
@@ -80,9 +86,11 @@ __host__ __device__ constexpr bool pass_half(int form, int L, int fold) {
 // Shared-memory plan of one row pass.  The CTA's slice of the coefficient matrix stays resident when it
 // fits beside a two-stage ring; otherwise every ring stage carries the slice's K-chunk next to the A
 // chunk (STREAM_B), brought in by a bulk copy from the pre-split image in global memory (L2-resident:
-// 0.2-1.5 MB per form and direction).  A folded forward stage holds both halves of the row's chunk, and
+// 0.2-1.5 MB per form and direction).  Narrow inverse passes always stream: their CTAs see one or two M-tiles,
+// and loading the slice first would stand before them (512x512 inverse on 2^20 elements 31.1 -> 28.0 us).  A
+// folded forward stage holds both halves of the row's chunk, and
 // the split parts fill it in place, so that it needs no A buffers.
-template <int FORM, int L, int FOLD = FOLD_NONE>
+template <int FORM, int L, int FOLD = FOLD_NONE, bool NARROW = false>
 struct PassLayout {
   using F = PassForm<FORM>;
   static constexpr bool kHalf = pass_half(FORM, L, FOLD);
@@ -90,7 +98,7 @@ struct PassLayout {
   static constexpr int kK = FOLD == FOLD_FWD ? L / 2 : L;                  // products per output
   static constexpr int kChunks = kK / kKC;
   static constexpr int kStageBytes = kRows * kKC * 4;
-  static constexpr int kNBlock = pass_nblock(L, FOLD);
+  static constexpr int kNBlock = pass_nblock(L, FOLD) / (NARROW ? 2 : 1);
   static constexpr int kBlocks = (FOLD == FOLD_INV ? L / 2 : L) / kNBlock;
   static constexpr int kBPart = kBAtom * kNBlock / 64;            // one split part of a K-chunk
   static constexpr int kBBytes = F::kSplits * (kK / F::kKC) * kBPart;   // this CTA's slice of C_L
@@ -98,7 +106,7 @@ struct PassLayout {
   static constexpr int kABufs = FOLD == FOLD_FWD ? 0 : 2;
   static constexpr int kABytes = (FOLD == FOLD_FWD ? 2 : 1) * kStageBytes;   // A data of a stage
   static constexpr int kBarBytes = 1024;
-  static constexpr bool kStreamB = kBBytes + kABufs * F::kABufBytes + kBarBytes + 1024 + 2 * kABytes > kPassSmemMax;
+  static constexpr bool kStreamB = (NARROW && FOLD == FOLD_INV) || kBBytes + kABufs * F::kABufBytes + kBarBytes + 1024 + 2 * kABytes > kPassSmemMax;
   static constexpr int kResident = kStreamB ? 0 : kBBytes;
   static constexpr int kStageStride = kABytes + (kStreamB ? kBChunk : 0);
   static constexpr int kStageTx = kStageStride;                  // bytes a stage's loads deliver
@@ -313,17 +321,19 @@ __device__ __forceinline__ void split_deint_tf32(uint8_t* stage, uint8_t* abuf, 
 // MERGE: BF16x3 adds all small products in one block, [big0 | small | big1 ..].  This makes room for the
 // second set of a 128-column N-block (forward, 256 points: 91.9 -> 67 us per call on 16 M elements, with
 // the errors of one K = 128 group per output, as in the unfolded pass) and of the inverses up to 256
-// points (104 -> 95 us; 128 points 73 -> 59), and at 512 and 1024 points keeps a big group to no more MMAs
+// points (104 -> 95 us; 128 points 73 -> 59; 86.5 and 56 with the products issued as in issue_merged_mmas), and at 512 and 1024 points keeps a big group to no more MMAs
 // than in an unfolded pass (errors against float64 1.75e-7 -> 1.57e-7 at 512 x 512, 2.77e-7 -> 2.65e-7 at
 // 1024 x 1024; with two groups 2.01e-7 and 3.73e-7).  TF32x3 has nothing to give up: its folded passes of
 // 256 points forward and 128 and 256 inverse keep one set, and its inverses of 512 and 1024 points are not
 // folded (launch_pass).
-template <int FORM, int CHUNKS, int SETS, int PARS, int NB, bool MERGE>
+// WIDE: the N-block that the number of group accumulators is counted for (NB, or twice NB in a narrow pass, so
+// that both spread a product over the same groups).
+template <int FORM, int CHUNKS, int SETS, int PARS, int NB, int WIDE, bool MERGE>
 struct PassAccs {
   static constexpr int kNBlock = NB;
   static constexpr bool kMerge = MERGE;
   static constexpr int kSmallBlocks = FORM == BF16X3 && !MERGE ? 2 : 1;
-  static constexpr int kMaxBig = 512 / (SETS * PARS * NB) - kSmallBlocks;
+  static constexpr int kMaxBig = 512 / (SETS * PARS * WIDE) - kSmallBlocks;
   static constexpr int kBig = CHUNKS < kMaxBig ? CHUNKS : kMaxBig;
   static constexpr int kPerParity = (1 + kSmallBlocks + (kBig - 1)) * NB;
   static constexpr int kPerTile = PARS * kPerParity;                               // columns
@@ -342,6 +352,42 @@ template <int FORM, int L, int FOLD> struct PassSets {
                                                                           : 1;
 };
 
+// Descriptor of the operand `bytes` (a multiple of 16) after that of d: the start address lies in the low
+// bits of the low word, which shared memory's size keeps from overflowing.
+__device__ __forceinline__ uint64_t desc_at(uint64_t d, uint32_t bytes) {
+  return (d & 0xFFFFFFFF00000000ull) | ((uint32_t)d + (bytes >> 4));
+}
+
+// The products of a chunk with the small ones merged (PassAccs::kMerge).  One thread issues them, and its
+// instructions bound the long inverse passes: descriptors by an addition each, and no choice within the
+// chunk (16 M elements, inverse: 1024x1024 412 -> 346 us, 512x512 208 -> 179; 2^18 of 512x512 28.3 -> 26.8).  The
+// products that are not merged gain nothing that way (512x512 forward 210 -> 213).  FIRST (group 0): the big block and the small one lie side by side, so one product reads Xh for both.
+template <typename A, int PARS, int NB, int STEPS, bool FIRST>
+__device__ __forceinline__ void issue_merged_mmas(uint32_t hi, uint32_t mid, uint32_t lo, uint32_t bchunk, int kc,
+                                                  uint32_t tmem) {
+  constexpr uint32_t kPart = kBAtom * NB / 64, i1 = instr_desc(1, NB);
+  constexpr int kSteps = STEPS / PARS;
+  const uint64_t dh = sw128_desc(hi), dm = sw128_desc(mid), dl = sw128_desc(lo), db = sw128_desc(bchunk);
+  const int g = A::group(kc);
+  const uint32_t clear = FIRST ? (kc != 0) : A::group(kc - 1) == g;
+#pragma unroll
+  for (int k = 0; k < STEPS; ++k) {
+    const uint32_t t = tmem + (uint32_t)(k / kSteps) * A::kPerParity;
+    const uint32_t c = k % kSteps == 0 ? clear : 1u;
+    const uint64_t bd = desc_at(db, k * 32u), bm = desc_at(db, kPart + k * 32u), ah = desc_at(dh, k * 32u);
+    if constexpr (FIRST) {
+      umma(t, ah, bd, instr_desc(1, 2 * NB), c, BF16X3);
+    } else {
+      umma(t + A::kExtraBig + (uint32_t)(g - 1) * NB, ah, bd, i1, c, BF16X3);
+      umma(t + NB, ah, bm, i1, 1u, BF16X3);
+    }
+    umma(t + NB, ah, desc_at(db, 2 * kPart + k * 32u), i1, 1u, BF16X3);
+    umma(t + NB, desc_at(dm, k * 32u), bd, i1, 1u, BF16X3);
+    umma(t + NB, desc_at(dm, k * 32u), bm, i1, 1u, BF16X3);
+    umma(t + NB, desc_at(dl, k * 32u), bd, i1, 1u, BF16X3);
+  }
+}
+
 // Split products of K-chunk kc (one thread): hi, mid, lo: shared addresses of the A parts (mid: BF16x3
 // only).  bchunk: shared address of the chunk's B splits, laid out [split][8 KB atom column of 64 rows].
 // tmem: column 0 of this M-tile's set.  With PARS = 2 the first half of a chunk's steps are e's.
@@ -349,6 +395,11 @@ template <int FORM, int L, int FOLD> struct PassSets {
 template <int FORM, typename A, int PARS, int NB, int STEPS>
 __device__ __forceinline__ void issue_pass_mmas(uint32_t hi, uint32_t mid, uint32_t lo, uint32_t bchunk, int kc,
                                                 uint32_t tmem) {
+  if constexpr (A::kMerge) {
+    if (A::kBig == 1 || A::group(kc) == 0) issue_merged_mmas<A, PARS, NB, STEPS, true>(hi, mid, lo, bchunk, kc, tmem);
+    else issue_merged_mmas<A, PARS, NB, STEPS, false>(hi, mid, lo, bchunk, kc, tmem);
+    return;
+  }
   constexpr uint32_t kPart = kBAtom * NB / 64;
   const int g = A::group(kc);
   const bool big_first = kc == 0 || A::group(kc - 1) != g;
@@ -361,21 +412,7 @@ __device__ __forceinline__ void issue_pass_mmas(uint32_t hi, uint32_t mid, uint3
     const uint64_t bd = sw128_desc(bchunk + k * 32u);
     const uint64_t ah = sw128_desc(hi + k * 32u);
     const uint32_t clear = (kc == 0 && first) ? 0u : 1u, clear_g = (big_first && first) ? 0u : 1u;
-    if constexpr (A::kMerge) {
-      constexpr uint32_t i1 = instr_desc(1, NB);
-      const uint64_t bm = sw128_desc(bchunk + kPart + k * 32u);
-      if constexpr (NB == 128) {
-        static_assert(NB != 128 || A::kBig == 1, "big and small side by side");
-        umma(t, ah, bd, instr_desc(1, 2 * NB), clear, BF16X3);
-      } else {
-        umma(g == 0 ? t : big_g, ah, bd, i1, g == 0 ? clear : clear_g, BF16X3);
-        umma(t + NB, ah, bm, i1, clear, BF16X3);
-      }
-      umma(t + NB, ah, sw128_desc(bchunk + 2 * kPart + k * 32u), i1, 1u, BF16X3);
-      umma(t + NB, sw128_desc(mid + k * 32u), bd, i1, 1u, BF16X3);
-      umma(t + NB, sw128_desc(mid + k * 32u), bm, i1, 1u, BF16X3);
-      umma(t + NB, sw128_desc(lo + k * 32u), bd, i1, 1u, BF16X3);
-    } else if constexpr (FORM == BF16X3) {
+    if constexpr (FORM == BF16X3) {
       constexpr uint32_t i3 = instr_desc(1, NB == 64 ? 192 : 256), i2 = instr_desc(1, 2 * NB), i1 = instr_desc(1, NB);
       if (g == 0 && NB == 64) {
         umma(t, ah, bd, i3, clear, BF16X3);
@@ -433,21 +470,21 @@ __device__ __forceinline__ void load_parts(uint32_t taddr, int q, float (&big)[1
 // column n = j * LS + c of super-row g is output column c of row g * SUB + j, and nrows counts
 // super-rows.
 // FOLD: see the file comment (L >= 128).  Folded forward, N-block i holds the columns
-// 2 (NB (i / 2) + n) + i % 2 (NB columns); folded inverse, the columns 64 i + n and L - 1 - (64 i + n).
-template <int FORM, int L, int SUB = 1, int FOLD = FOLD_NONE>
+// 2 (NB (i / 2) + n) + i % 2 (NB columns); folded inverse, the columns NB i + n and L - 1 - (NB i + n).
+template <int FORM, int L, int SUB = 1, int FOLD = FOLD_NONE, bool NARROW = false>
 __global__ void __launch_bounds__(kPassThreads, 1)
     k_tcpass(const __grid_constant__ CUtensorMap xmap, float* __restrict__ out,
              const uint4* __restrict__ bimage, long long nrows, int rshift, int* __restrict__ err) {
   static_assert(SUB == 1 || L == 64, "super-rows are 64 floats");
   static_assert(FOLD == FOLD_NONE || (SUB == 1 && L >= 128), "folded rows");
   constexpr int LS = L / SUB;   // points per original row
-  using PL = PassLayout<FORM, L, FOLD>;
+  using PL = PassLayout<FORM, L, FOLD, NARROW>;
   using F = PassForm<FORM>;
   constexpr int kStages = PL::kStages;
   constexpr int kChunks = PL::kChunks;
   constexpr int kSets = PassSets<FORM, L, FOLD>::value;
   constexpr int kPars = FOLD == FOLD_INV ? 2 : 1;
-  using ACC = PassAccs<FORM, kChunks, kSets, kPars, PL::kNBlock, PassSets<FORM, L, FOLD>::kMerge>;
+  using ACC = PassAccs<FORM, kChunks, kSets, kPars, PL::kNBlock, pass_nblock(L, FOLD), PassSets<FORM, L, FOLD>::kMerge>;
   constexpr uint32_t kTileCols = ACC::kPerTile;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
