@@ -543,7 +543,7 @@ def generate() -> str:
 
 # ----------------------------------------------------------------------------------------
 # Programs over a value type T (sj_packed.cuh): T = F2 runs two lines at once with the packed
-# f32x2 instructions.  A multiplication whose only use is an addition is fused here, explicitly.
+# f32x2 instructions, T = F1 one line.  Products are fused into additions here, explicitly.
 # ----------------------------------------------------------------------------------------
 
 PACKED_LINES = (8, 16, 32, 64)      # whole lines in registers
@@ -553,7 +553,11 @@ PACKED_STAGE2 = (8, 16)             # stage 2: complex FFT over the B residues o
 
 def emit_packed(g: Graph, name: str, in_names: Sequence[str], outputs: Sequence[int],
                 out_names: Sequence[str], signature: str, doc: str) -> str:
-    """Emits a device function template over T computing outputs from inputs (in_names None: zero)."""
+    """Emits a device function template over T computing outputs from inputs (in_names None: zero).
+
+    Every addition of a product is a fused multiply-add, also of a product with several uses: the
+    compiler would contract the packed ones anyway (and not the scalar ones of another T), so this leaves
+    it nothing to choose, and every T and every kernel gives the same bits."""
     order = g.live(outputs)
     uses: Dict[int, int] = {}
     for n in order:
@@ -562,17 +566,31 @@ def emit_packed(g: Graph, name: str, in_names: Sequence[str], outputs: Sequence[
             uses[d] = uses.get(d, 0) + 1
     for o in outputs:
         uses[o] = uses.get(o, 0) + 1
-    fused = set()
-    plan: Dict[int, tuple] = {}
+
+    def product(m):
+        """(base, factor) of a product or a negated product, else None."""
+        node = g.nodes[m]
+        if node[0] == "neg" and g.nodes[node[1]][0] == "mul":
+            return g.nodes[node[1]][1], -g.nodes[node[1]][2]
+        return (node[1], node[2]) if node[0] == "mul" else None
+
+    # operand of an addition that is fused: of two products the one with fewer uses, the second if equal
+    plan: Dict[int, int] = {}
     for n in order:
-        node = g.nodes[n]
-        if node[0] not in ("add", "sub"):
-            continue
-        for m in (node[2], node[1]):
-            if g.nodes[m][0] == "mul" and uses[m] == 1 and m not in fused:
-                fused.add(m)
-                plan[n] = (m,)
-                break
+        if g.nodes[n][0] in ("add", "sub"):
+            found = [m for m in (g.nodes[n][2], g.nodes[n][1]) if product(m)]
+            if found:
+                plan[n] = min(found, key=lambda m: uses[m])
+    needed = set(outputs)
+    for n in reversed(order):
+        if n in needed:
+            node = g.nodes[n]
+            if n in plan:
+                m = plan[n]
+                needed.add(product(m)[0])
+                needed.add(node[2] if node[1] == m else node[1])
+            else:
+                needed.update(node[1:3] if node[0] in ("add", "sub") else node[1:2] if node[0] in ("neg", "mul") else ())
     lines = [f"// {doc}", "template <typename T>", f"__device__ __forceinline__ void {name}({signature}) {{"]
     name_of: Dict[int, str] = {}
     tmp = 0
@@ -583,19 +601,20 @@ def emit_packed(g: Graph, name: str, in_names: Sequence[str], outputs: Sequence[
             name_of[n] = f"i{node[1]}"
             lines.append(f"  const T i{node[1]} = {in_names[node[1]]};")
             continue
-        if n in fused:
+        if n not in needed:
             continue
         t = f"t{tmp}"
         tmp += 1
         if n in plan:
-            m = plan[n][0]
-            base, c = name_of[g.nodes[m][1]], g.nodes[m][2]
+            m = plan[n]
+            base, c = product(m)
+            other = name_of[node[2] if node[1] == m else node[1]]
             if op == "add":
-                expr = f"vfma({base}, {fconst(c)}, {name_of[node[2] if node[1] == m else node[1]]})"
+                expr = f"vfma({name_of[base]}, {fconst(c)}, {other})"
             elif node[2] == m:
-                expr = f"vfma({base}, {fconst(-c)}, {name_of[node[1]]})"
+                expr = f"vfma({name_of[base]}, {fconst(-c)}, {other})"
             else:
-                expr = f"vfms({base}, {fconst(c)}, {name_of[node[2]]})"
+                expr = f"vfms({name_of[base]}, {fconst(c)}, {other})"
         elif op == "add":
             expr = f"vadd({name_of[node[1]]}, {name_of[node[2]]})"
         elif op == "sub":
@@ -648,7 +667,7 @@ def build_special(n: int):
 def generate_packed() -> str:
     parts = [
         "// Generated by gen_sj.py --packed: Shao-Johnson programs over a value type T (F2: two lines at",
-        "// once in packed f32x2 instructions).",
+        "// once in packed f32x2 instructions; F1: one line).",
         "// Do not edit by hand; rerun `python gen_sj.py --packed > sj_packed.cuh`.",
         "#pragma once",
         "",
