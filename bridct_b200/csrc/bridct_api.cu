@@ -217,7 +217,7 @@ using namespace bridct;
 
 namespace bridct {
 
-int kernel_setup(const void* kernel, int smem, int threads) {
+int kernel_setup(const void* kernel, int smem, int threads, bool all_shared) {
   static std::mutex mu;
   static std::map<std::tuple<const void*, int, int, int>, int> cache;
   int dev = 0;
@@ -229,6 +229,9 @@ int kernel_setup(const void* kernel, int smem, int threads) {
   int blocks = 0;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return 0;
+  if (all_shared && cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         cudaSharedmemCarveoutMaxShared) != cudaSuccess)
     return 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, smem) != cudaSuccess) return 0;
   cache[key] = blocks;

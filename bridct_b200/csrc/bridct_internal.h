@@ -49,8 +49,9 @@ cudaError_t launch_merged_pass(const DeviceCtx* d, bool col, int cls, int mode, 
                                const float* x, float* y, cudaStream_t st);
 // Opts `kernel` into `smem` bytes of dynamic shared memory on the current device and returns
 // its resident blocks per SM at `threads` threads (0 on failure); cached per device, since the
-// attribute belongs to the device's copy of the kernel.
-int kernel_setup(const void* kernel, int smem, int threads);
+// attribute belongs to the device's copy of the kernel.  all_shared: the kernel asks for the SM's largest
+// shared-memory configuration.
+int kernel_setup(const void* kernel, int smem, int threads, bool all_shared);
 int current_device(int* dev);
 const void* device_address(const void* p, bool* pinned);
 

@@ -15,7 +15,7 @@ struct LaunchCtx {
 using PlainLauncher = cudaError_t (*)(const float*, float*, long long, cudaStream_t,
                                       LineTables, const LaunchCtx&, const BatchLayout*, const BatchLayout*);
 
-int kernel_setup(const void* kernel, int smem, int threads);   // bridct_api.cu
+int kernel_setup(const void* kernel, int smem, int threads, bool all_shared = false);   // bridct_api.cu
 
 // Blocks per SM for a kernel at a given dynamic shared-memory size (set up once per device).
 template <typename Kernel>
@@ -86,23 +86,38 @@ cudaError_t launch_split_rows(float* y, long long batch, const BatchLayout& ly, 
   return launch_split(k_split_rows<W, GEN ? H : 0, MODE, 8>, Wide::kSmem, Wide::T, batch * H / Wide::RB, a, st);
 }
 
-// Arrays and threads per CTA and resident CTAs of the whole-array tiles (k_pair_tile), the fastest of
-// 3 to 8 combinations measured per shape on 128 MiB batches.  Shapes up to 64 x 64 run one warp per
-// CTA with a line pair per thread: 12 to 32 independent warps per SM overlap one another's loads,
-// transforms and stores, where 128-thread CTAs of the same tiles measured 5..30% slower.  Shapes with a
-// longer axis take the smallest tile that gives every thread a task of both stages, at the register
-// limit that keeps 12 or more warps per SM.
+// Arrays and threads per CTA, CTAs per SM that the registers are limited for, and whether short axes run one
+// line per thread (SINGLE), of the whole-array tiles (k_pair_tile): the fastest of 3 to 10 combinations measured
+// per shape.  Shapes up to 64 x 64 run one or two warps per CTA: 12 to 32 independent warps per SM overlap one
+// another's loads, transforms and stores, where 128-thread CTAs of the same tiles measured 5..30% slower.  Up to
+// 32 points a thread of a full batch runs a pair of lines (32 x 16 and 32 x 32 round trips +5..10% over
+// single lines, the others equal).  With 64 points single lines are the faster ones at every size: a pair's 128 values leave the
+// compiler no room to overlap anything, and a line at a time makes twice the warps (us a call on 2^25
+// elements, pairs / single: 16x64 45.5 / 42.5, 64x32 45.4 / 42.9, round trips 54.1 / 49.0 and 52.0 / 52.1; on 2^20
+// elements 4.26 / 3.02 and 3.80 / 3.07).  Shapes with a longer axis take the smallest tile that gives every
+// thread a task of both stages, at the register limit that keeps 12 or more warps per SM.
+//
+// resident: at most so many CTAs share an SM (by the shared memory asked for, in the SM's largest
+// configuration; 0: as many as fit).  Where the tiles of two launches fit side by side, each slows the other down,
+// and whether they do depended on the configuration that the kernel before had left (2^21 elements of 16x32 in
+// one-warp tiles 4.9 or 5.9 us).  16 for one-warp tiles measured fastest of 10 to 18 over 2^19 .. 2^23 elements
+// (2^21, 2^21.5 and 2^22 elements of 16x64, no limit / 16: 5.6 / 5.6, 8.8 / 8.1 and 9.7 / 8.9 us), 8 and 10 for two warps
+// (2^21.5 and 2^22 elements of 64x64 9.1 / 8.5 and 10.1 / 9.3, of 16x32 7.2 / 6.3 and 8.3 / 7.5).
 struct TileCfg {
   int arrays, threads, blocks;
+  bool single = false;
+  int resident = 0;
 };
 __host__ __device__ constexpr TileCfg tile_cfg(int h, int w) {
   const int m = cmax(h, w);
-  if (m <= 64) return {64 * m / (h * w), 32, m == 64 ? 12 : m == 32 ? 20 : 24};
+  if (m <= 32) return {64 * m / (h * w), 32, m == 32 ? 20 : 24};
+  if (m == 64) return h == w ? TileCfg{1, 64, 6, true, 8} : TileCfg{2048 / (h * w), 32, 12, true, 16};
   if (m == 128) {
     if (h <= 16) return {2048 / (h * w), 64, 16};
     if (w == 8) return {4, 64, 10};
     if (w == 16) return {2, 128, 8};
     if (h == 32 || w == 32) return {1, 64, 10};
+    if (w == 64) return {1, 128, 3, true};   // 2^21 and 2^25 elements 9.0 / 7.2 and 61 / 57 us, pairs in 64 threads / this
     return {1, 64, 6};
   }
   if (m == 256) {
@@ -118,31 +133,53 @@ __host__ __device__ constexpr TileCfg tile_cfg(int h, int w) {
   }
   return {w == 1024 ? 16 / h : 1, 128, 3};
 }
-// The same for batches that do not fill the GPU: half as many arrays per tile, or twice the threads
-// (16 MiB batches +8% on average over the shapes, up to +27%; 128 MiB batches 5..30% slower).
+// The same for batches that do not fill the GPU (few_tiles): smaller tiles or more threads for one, and single
+// lines for short axes, since with about a warp per scheduler a line's instructions are the whole latency and
+// a packed one takes two issue cycles (us a call on 2^19 elements, half tiles of pairs / these: 16x32 2.39 / 2.08,
+// 32x32 2.53 / 2.05, round trips 2.79 / 2.30 and 3.02 / 2.33; 8x64 round trips 3.87 / 2.77, 16x64 3.16 / 2.28, 32x64
+// round trips 4.81 / 2.78; 64x128 on 2^21 8.9 / 7.7).  One-warp tiles of 1024 floats measured up to 20% faster for 32
+// points on 2^20.5 and 2^21 elements, but 20..40% slower on 2^20 and 2^21 in processes with many streams.
 __host__ __device__ constexpr TileCfg tile_cfg_few(int h, int w) {
   const TileCfg c = tile_cfg(h, w);
   const int m = cmax(h, w);
-  if (m <= 16) return {h * w == 256 ? 4 : 8, 64, 12};
-  if (m <= 64) return c.arrays > 1 ? TileCfg{c.arrays / 2, 32, c.blocks} : TileCfg{1, 64, 6};
+  if (m <= 16) return {1024 / (h * w), 64, 16, true};
+  if (m == 32) return {2048 / (h * w), 64, 8, true, 10};
+  if (m == 64) return h == w ? c : TileCfg{2048 / (h * w), 64, 8, true, 10};
   if (m == 128) {
-    if (h <= 16 || w == 16) return c;
+    if (h <= 16 || w == 16 || w == 64) return c;
+    if (h == 64) return {1, 128, 3, true};
     if (h == 32) return {1, 128, 7};
-    return {c.arrays, 128, w == 8 || w == 32 ? 5 : 3};
+    return {c.arrays, 128, 5};
   }
   if (m == 256) {
     if (w == 8) return c;
     if (w == 16) return {1, 128, 5};
     return {c.arrays, c.threads * 2, c.threads == 64 ? 5 : c.blocks == 3 ? 2 : 3};
   }
-  if (m == 512) return h == 512 ? c : TileCfg{c.arrays, 256, c.blocks == 5 ? 3 : 2};
-  return h == 8 ? TileCfg{1, 128, 3} : c;
+  if (m == 512) return h == 512 ? (w == 8 ? TileCfg{1, 128, 4} : c) : TileCfg{c.arrays, 256, c.blocks == 5 ? 3 : 2};
+  return h == 8 ? TileCfg{1, 128, 3} : w == 8 ? TileCfg{1, 256, 2} : c;
 }
-// Whether a batch that makes `tiles` full tiles takes the smaller ones: below one wave, unless the full
-// tiles fit in less than half of the GPU's slots and the smaller ones (twice the slots) do not: back to
-// back launches then overlap (programmatic dependent launch), which is worth more (+5..25% at 8 MiB).
-static inline bool few_tiles(long long tiles, TileCfg c, const LaunchCtx& ctx) {
+// Whether a batch takes the tiles of tile_cfg_few.  waves: of full tiles.
+//   * Axes up to 16 points, 32 x 128 and 64 x 128: below a wave, or 1.3 where the second one would be nearly empty
+//     (2^22 elements of 8x16 9.4 / 7.9 us, 2^23 of 64x128 22.0 / 19.5; full / these).
+//   * 64 points: up to two tiles per SM, and where the last one-warp tiles decide the time (2^21.5 elements of 16x64
+//     7.9 / 6.9, 64x16 8.6 / 7.6; 2^21 5.6 / 6.1).
+//   * 512x8, 1024x8 and 16x512: where their own wave is nearly full (2^21 elements 10.2 / 8.5 and 11.5 / 10.5; a
+//     quarter fewer 7.3 / 7.9 and 9.1 / 9.9).
+//   * Others: below a wave, except where the full tiles fit in less than half of the GPU's slots and the smaller ones
+//     (twice the slots) do not: back-to-back launches then overlap (programmatic dependent launch), which is
+//     worth more (+5..25% at 8 MiB).
+static inline bool few_tiles(int h, int w, long long batch, const LaunchCtx& ctx) {
+  const TileCfg c = tile_cfg(h, w), f = tile_cfg_few(h, w);
+  const int m = cmax(h, w);
+  const long long tiles = (batch + c.arrays - 1) / c.arrays, few = (batch + f.arrays - 1) / f.arrays;
   const double waves = (double)tiles / ((double)c.blocks * ctx.sm_count);
+  if (m <= 16 || (w == 128 && (h == 32 || h == 64))) return waves < (h == 32 ? 1.0 : 1.3);
+  if (m == 64) return tiles <= 2 * ctx.sm_count || (waves > 0.65 && waves < 1);
+  if ((w == 8 && h >= 512) || (h == 16 && w == 512)) {
+    const double own = (double)few / ((double)f.blocks * ctx.sm_count);
+    return own > 0.75 && own <= 1;
+  }
   return waves < 1 && (tiles <= ctx.sm_count || waves < 0.225 || waves > 0.45);
 }
 // Whole arrays up to 16384 floats, except 128 x 128 (register lines of one thread each, below: +15..20%
@@ -151,12 +188,16 @@ __host__ __device__ constexpr bool pair_tile_route(int h, int w) {
   return h * w <= 16384 && !(h == 128 && w == 128) && !(h == 8 && w == 8);
 }
 
-template <int SMEM, typename Kernel>
-static cudaError_t launch_pair_tile(Kernel k, TileCfg c, long long batch, TileArgs a, cudaStream_t st) {
-  if (kernel_blocks_per_sm(k, SMEM, c.threads) <= 0) return cudaErrorInvalidConfiguration;
-  a.ntiles = (batch + c.arrays - 1) / c.arrays;
+constexpr int kSmemPerSm = 228 * 1024;   // of which a CTA takes 1024 bytes besides its own
+template <int H, int W, int MODE, bool GEN, int ARR, int T, int BLOCKS, bool SINGLE, int RESIDENT>
+static cudaError_t launch_pair_tile(long long batch, TileArgs a, cudaStream_t st) {
+  const auto k = k_pair_tile<H, W, ARR, MODE, T, BLOCKS, GEN, SINGLE>;
+  constexpr int need = PairTileGeo<H, W, ARR>::kSmem;
+  constexpr int smem = RESIDENT ? cmax(need, (kSmemPerSm / cmax(RESIDENT, 1) - 1024) / 128 * 128) : need;
+  if (kernel_setup(reinterpret_cast<const void*>(k), smem, T, RESIDENT > 0) <= 0) return cudaErrorInvalidConfiguration;
+  a.ntiles = (batch + ARR - 1) / ARR;
   if (a.ntiles > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
-  return launch_pdl(k, (unsigned)a.ntiles, (unsigned)c.threads, SMEM, st, a);
+  return launch_pdl(k, (unsigned)a.ntiles, (unsigned)T, smem, st, a);
 }
 
 // The classes of a ragged batch that the merged passes take (bridct_ragged_set_schedule): shapes above
@@ -203,11 +244,9 @@ cudaError_t launch_plain_impl(const float* x, float* y, long long batch, cudaStr
     constexpr TileCfg c = tile_cfg(H, W), f = tile_cfg_few(H, W);
     constexpr bool has_few = f.arrays != c.arrays || f.threads != c.threads;
     const TileArgs a{x, y, 0, batch * H, tab, lx, ly};
-    if (has_few && few_tiles((batch + c.arrays - 1) / c.arrays, c, ctx))
-      return launch_pair_tile<PairTileGeo<H, W, f.arrays>::kSmem>(
-          k_pair_tile<H, W, f.arrays, MODE, f.threads, f.blocks, GEN>, f, batch, a, st);
-    return launch_pair_tile<PairTileGeo<H, W, c.arrays>::kSmem>(
-        k_pair_tile<H, W, c.arrays, MODE, c.threads, c.blocks, GEN>, c, batch, a, st);
+    if (has_few && few_tiles(H, W, batch, ctx))
+      return launch_pair_tile<H, W, MODE, GEN, f.arrays, f.threads, f.blocks, f.single, f.resident>(batch, a, st);
+    return launch_pair_tile<H, W, MODE, GEN, c.arrays, c.threads, c.blocks, c.single, c.resident>(batch, a, st);
   } else if constexpr (H * W <= 16384) {
     // Register tiles, persistent CTAs.  The 128 x 128 round trip is given shared memory for two CTAs per
     // SM only, which measured 2-3% faster than three.

@@ -66,7 +66,17 @@ __device__ __forceinline__ F2 vneg(F2 a) {
 __device__ __forceinline__ F2 vmul(F2 a, float c) { return vmul(a, f2_make(c, c)); }
 __device__ __forceinline__ F2 vfma(F2 a, float c, F2 b) { return vfma(a, f2_make(c, c), b); }
 __device__ __forceinline__ F2 vfms(F2 a, float c, F2 b) { return vfma(a, f2_make(c, c), vneg(b)); }
-__device__ __forceinline__ F2 vbcast(float c, F2) { return f2_make(c, c); }
+// The same operations on one line.  The intrinsics round once each and are never contracted, so one line at
+// a time gives the bits of two at a time.
+struct F1 {
+  float v = 0.0f;
+};
+__device__ __forceinline__ F1 vadd(F1 a, F1 b) { return F1{__fadd_rn(a.v, b.v)}; }
+__device__ __forceinline__ F1 vsub(F1 a, F1 b) { return F1{__fsub_rn(a.v, b.v)}; }
+__device__ __forceinline__ F1 vmul(F1 a, float c) { return F1{__fmul_rn(a.v, c)}; }
+__device__ __forceinline__ F1 vneg(F1 a) { return F1{-a.v}; }
+__device__ __forceinline__ F1 vfma(F1 a, float c, F1 b) { return F1{__fmaf_rn(a.v, c, b.v)}; }
+__device__ __forceinline__ F1 vfms(F1 a, float c, F1 b) { return F1{__fmaf_rn(a.v, c, -b.v)}; }
 
 }  // namespace bridct
 
@@ -551,14 +561,14 @@ __global__ void __launch_bounds__(RowGeo<N, LP>::T, RowGeo<N, LP>::kBlocks) k_sp
   }
 }
 
-// ---- lines of 64 points and fewer: two per thread in registers -----------------------------------
-template <int N, int MODE>
-__device__ __forceinline__ void pair_line(F2 (&v)[N]) {
+// ---- lines of 64 points and fewer: two per thread (V = F2) or one (V = F1) in registers --------
+template <int N, int MODE, typename V>
+__device__ __forceinline__ void pair_line(V (&v)[N]) {
   static_assert(N <= 64, "register lines");
-  if constexpr (N == 8) MODE == LM_FWD ? sjp_fwd_8<F2>(v) : MODE == LM_INV ? sjp_inv_8<F2>(v) : sjp_rt_8<F2>(v);
-  if constexpr (N == 16) MODE == LM_FWD ? sjp_fwd_16<F2>(v) : MODE == LM_INV ? sjp_inv_16<F2>(v) : sjp_rt_16<F2>(v);
-  if constexpr (N == 32) MODE == LM_FWD ? sjp_fwd_32<F2>(v) : MODE == LM_INV ? sjp_inv_32<F2>(v) : sjp_rt_32<F2>(v);
-  if constexpr (N == 64) MODE == LM_FWD ? sjp_fwd_64<F2>(v) : MODE == LM_INV ? sjp_inv_64<F2>(v) : sjp_rt_64<F2>(v);
+  if constexpr (N == 8) MODE == LM_FWD ? sjp_fwd_8<V>(v) : MODE == LM_INV ? sjp_inv_8<V>(v) : sjp_rt_8<V>(v);
+  if constexpr (N == 16) MODE == LM_FWD ? sjp_fwd_16<V>(v) : MODE == LM_INV ? sjp_inv_16<V>(v) : sjp_rt_16<V>(v);
+  if constexpr (N == 32) MODE == LM_FWD ? sjp_fwd_32<V>(v) : MODE == LM_INV ? sjp_inv_32<V>(v) : sjp_rt_32<V>(v);
+  if constexpr (N == 64) MODE == LM_FWD ? sjp_fwd_64<V>(v) : MODE == LM_INV ? sjp_inv_64<V>(v) : sjp_rt_64<V>(v);
 }
 // Two rows in shared memory, in place: 128-bit accesses (8 consecutive rows at a pitch of 4 mod 32
 // floats are 4 banks apart).
@@ -584,6 +594,24 @@ __device__ __forceinline__ void pair_rows(float* r0, float* r1) {
     *reinterpret_cast<float4*>(r0 + i) = p;
     *reinterpret_cast<float4*>(r1 + i) = q;
   }
+}
+
+// One row in shared memory, in place.
+template <int N, int MODE>
+__device__ __forceinline__ void single_row(float* r) {
+  F1 v[N];
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const float4 p = *reinterpret_cast<const float4*>(r + i);
+    v[i].v = p.x;
+    v[i + 1].v = p.y;
+    v[i + 2].v = p.z;
+    v[i + 3].v = p.w;
+  }
+  pair_line<N, MODE>(v);
+#pragma unroll
+  for (int i = 0; i < N; i += 4)
+    *reinterpret_cast<float4*>(r + i) = make_float4(v[i].v, v[i + 1].v, v[i + 2].v, v[i + 3].v);
 }
 
 // Column pass of 32- and 64-point columns: a thread holds two adjacent columns, straight from and to
@@ -676,7 +704,9 @@ template <int H, int W, int ARR> struct PairTileGeo {
   static constexpr int kSmem = (kTile + kTabC + kTabR) * 4;
 };
 
-template <int H, int W, int ARR, int MODE, int T, int MINB, bool GEN>
+// SINGLE: a thread runs one line of a short axis at a time instead of two, for batches that leave most of
+// the GPU's issue slots idle (tile_cfg_few).
+template <int H, int W, int ARR, int MODE, int T, int MINB, bool GEN, bool SINGLE>
 __global__ void __launch_bounds__(T, MINB) k_pair_tile(TileArgs a) {
   using Geo = PairTileGeo<H, W, ARR>;
   constexpr int P = Geo::P, AP = Geo::AP, TR = Geo::TR;
@@ -713,6 +743,16 @@ __global__ void __launch_bounds__(T, MINB) k_pair_tile(TileArgs a) {
           return f2_make(v.x, v.y);
         },
         [&](int g, int i, F2 v) { *reinterpret_cast<F2*>(base(g) + i * P) = v; }, base, P, tcol);
+  } else if constexpr (SINGLE) {
+    for (int l = threadIdx.x; l < ARR * W; l += T) {
+      float* c = smem + (l / W) * AP + l % W;
+      F1 v[H];
+#pragma unroll
+      for (int i = 0; i < H; ++i) v[i].v = c[i * P];
+      pair_line<H, MODE>(v);
+#pragma unroll
+      for (int i = 0; i < H; ++i) c[i * P] = v[i].v;
+    }
   } else {
     for (int l = threadIdx.x; l < ARR * W / 2; l += T) {
       float* c = smem + (l / (W / 2)) * AP + 2 * (l % (W / 2));
@@ -727,6 +767,8 @@ __global__ void __launch_bounds__(T, MINB) k_pair_tile(TileArgs a) {
   __syncthreads();
   if constexpr (W >= 128) {
     split_rows<W, MODE, T, TR / (2 * Geo::kRowPairs), Geo::kRowPairs>(smem, trow);
+  } else if constexpr (SINGLE) {
+    for (int l = threadIdx.x; l < TR; l += T) single_row<W, MODE>(smem + srow(l));
   } else {
     for (int l = threadIdx.x; l < TR / 2; l += T) {
       const int r = (l / 8) * 16 + l % 8;
