@@ -135,13 +135,13 @@ void build_units(const bridct_ragged* r, RaggedTables& tables) {
       for (int i : c.arrays) queued[i] = 0;
   for (size_t i = 0; i < r->items.size(); ++i) {
     const bridct_ragged_item& it = r->items[i];
-    RaggedArray a{(long long)it.offset, it.height, it.width, it.mode, 0};
+    RaggedArray a{(long long)it.offset, (short)it.height, (short)it.width, (short)it.mode, 0};
     if (!queued[i]) {
       // run by its class's own launch: not in the queue
     } else if (one_unit(it.height, it.width, t)) {
       small.push_back((int)i);
     } else {
-      a.nstrips = it.width / strip_cols(it.height, it.width, t.strip_floats);
+      a.nstrips = (short)(it.width / strip_cols(it.height, it.width, t.strip_floats));
       big.push_back((int)i);
     }
     tables.arrays.push_back(a);
@@ -645,7 +645,7 @@ struct NaOff {
 
 }  // namespace
 
-// About 1.8 MB: queue (arrays, units), counters, error word, split-line tables.  Host code must
+// About 0.95 MB: queue (arrays, units), counters, error word, split-line tables.  Host code must
 // not use this name as a device address; the entry point resolves it per device below.
 static __device__ __align__(256) unsigned char g_ragged_scratch[NaOff::bytes];
 
@@ -709,14 +709,14 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
   long long limit = 0;   // units of the tuning's sizes
   for (size_t i = 0; i < count; ++i) {
     const bridct_ragged_item& it = items[i];
-    RaggedArray a{(long long)it.offset, it.height, it.width, it.mode, 0};
+    RaggedArray a{(long long)it.offset, (short)it.height, (short)it.width, (short)it.mode, 0};
     const bool tile = (long long)it.height * it.width <= t.tile_floats;
     limit += tile ? 1 : it.width / strip_cols(it.height, it.width, t.strip_floats) +
                             it.height / block_rows(it.height, it.width, t.row_floats);
     if (one_unit(it.height, it.width, t)) {
       g_na_small[nsmall++] = (int)i;
     } else {
-      a.nstrips = it.width / strip_cols(it.height, it.width, std::min(t.strip_floats, kRaggedUnit));
+      a.nstrips = (short)(it.width / strip_cols(it.height, it.width, std::min(t.strip_floats, kRaggedUnit)));
       g_na_big[nbig++] = (int)i;
     }
     g_na_arrays[i] = a;

@@ -26,16 +26,22 @@ enum UnitType { UNIT_TILE = 0, UNIT_COLSTRIP = 1, UNIT_ROWBLOCK = 2 };
 
 struct RaggedArray {
   long long offset;   // first float of the array in x and y
-  int h, w, mode;
-  int nstrips;        // column strips of a two-pass array (0 for tile arrays)
+  short h, w, mode;
+  short nstrips;      // column strips of a two-pass array (0 for tile arrays)
 };
 
+// Eight bytes: the queue of the allocation-free entry point lies in static device memory.
 struct RaggedUnit {
   int array;
-  int type;
-  int first;          // first column (COLSTRIP) or first row (ROWBLOCK)
-  int count;          // columns or rows covered
+  unsigned what;      // type, then 11 bits each of first and count
+  RaggedUnit() = default;
+  RaggedUnit(int array, UnitType type, int first, int count)
+      : array(array), what((unsigned)type | (unsigned)first << 2 | (unsigned)count << 13) {}
+  __host__ __device__ int type() const { return what & 3; }
+  __host__ __device__ int first() const { return what >> 2 & 0x7FF; }    // first column (COLSTRIP) or row (ROWBLOCK)
+  __host__ __device__ int count() const { return what >> 13; }           // columns or rows covered
 };
+static_assert(sizeof(RaggedUnit) == 8 && sizeof(RaggedArray) == 16, "queue entries");
 
 struct RaggedArgs {
   const float* x;
@@ -278,7 +284,7 @@ __global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged(RaggedArgs a) {
   // enough that no CTA runs dry for it; a held unit comes after the current one in the queue, so what
   // any row block waits for still makes progress.
   int ahead = -1;
-  RaggedUnit next{};
+  RaggedUnit next;
   for (;;) {
     if (threadIdx.x == 0) {
       int u = ahead;
@@ -304,15 +310,15 @@ __global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged(RaggedArgs a) {
     const int h = arr.h, w = arr.w, mode = arr.mode;
     const float* xa = a.x + arr.offset;
     float* ya = a.y + arr.offset;
-    const bool whole = unit.type == UNIT_TILE;
-    bool rows = unit.type != UNIT_COLSTRIP;
+    const bool whole = unit.type() == UNIT_TILE;
+    bool rows = unit.type() != UNIT_COLSTRIP;
     int first = 0, count = h;
     if (whole) {
       ragged_load(xa, h, w, tile, ragged_pitch(w));
       ragged_tile_cols_dyn(h, mode, tile, ragged_pitch(w), w, tabs);
       fetch();
-    } else if (unit.type == UNIT_COLSTRIP) {
-      ragged_cols_dyn(h, mode, xa + unit.first, ya + unit.first, w, unit.count, tile, tabs);
+    } else if (unit.type() == UNIT_COLSTRIP) {
+      ragged_cols_dyn(h, mode, xa + unit.first(), ya + unit.first(), w, unit.count(), tile, tabs);
       fetch();
       __threadfence();
       __syncthreads();
@@ -339,8 +345,8 @@ __global__ void __launch_bounds__(kRaggedThreads, 3) k_ragged(RaggedArgs a) {
       // rows through the async proxy.  No grid boundary lies between, so order the two here.
       asm volatile("fence.proxy.async.global;" ::: "memory");
       rows = s_ok;
-      first = unit.first;
-      count = unit.count;
+      first = unit.first();
+      count = unit.count();
     }
     if (rows) ragged_row_pass(ya + (long long)first * w, count, w, mode, whole, tile, tabs);
     __syncthreads();

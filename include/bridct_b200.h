@@ -197,7 +197,7 @@ BRIDCT_API int bridct_ragged_set_wait_limit(bridct_ragged *batch, unsigned polls
  * allocate device memory (a framework whose caching allocator owns the whole GPU, a loop that
  * cannot afford cudaMalloc's implicit synchronisation, a fixed device footprint): the items and
  * the input/output buffers are passed in, and the work queue, counters and tables live in one
- * static device array of about 1.8 MB that every GPU loading this library holds until exit.
+ * static device array of about 0.95 MB that every GPU loading this library holds until exit.
  * Limits: at most 4096 arrays and 49152 work units per call (default unit geometry), else
  * BRIDCT_INVALID_ARGUMENT with a message.  A successful call allocates nothing.  The first call
  * on a device resolves that array's address and uploads the split-line tables into it.  Every

@@ -25,3 +25,9 @@ def test_first_call_takes_no_table_from_the_heap(library, monkeypatch):
     assert L.bridct_ragged_apply_noalloc(items, 2, align(x), align(y), None) == _lib.OK, _lib.last_error()
     assert L.fake_largest_new() <= 256
     assert [n for n, _ in fake_cuda.launched(L) if "k_ragged" in n]
+
+
+def test_static_device_memory_stays_below_a_megabyte(library, monkeypatch):
+    L = fake_cuda.load(library, monkeypatch)
+    L.fake_symbol_bytes.restype = C.c_size_t
+    assert 0 < L.fake_symbol_bytes() < 1000000
