@@ -127,9 +127,7 @@ DeviceCtx* device_ctx(int device) {
   d->sm_count = prop.multiProcessorCount;
   d->major = prop.major;
   d->minor = prop.minor;
-  d->l2_bytes = prop.l2CacheSize;
   d->launch.sm_count = prop.multiProcessorCount;
-  // Two-pass chunk: a quarter of L2 keeps the column pass's output resident for the row pass.
   PlainLauncher (*tab)[8][3] = d->plain;
   plain_table_h8(tab[0]);
   plain_table_h16(tab[1]);

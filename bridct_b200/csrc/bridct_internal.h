@@ -15,7 +15,6 @@ struct DeviceCtx {
   int device = 0;
   int sm_count = 0;
   int major = 0, minor = 0;
-  long long l2_bytes = 0;
   LaunchCtx launch{};
   PlainLauncher plain[8][8][3] = {};
   SplitTables split[4] = {};            // rotation tables of N = 128, 256, 512, 1024

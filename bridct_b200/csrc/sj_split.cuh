@@ -1,6 +1,6 @@
 // Long lines (128..1024 points) of the plain form, two lines per thread.
 //
-// A line of N = A * B points is split as in sj_lines.cuh: stage 1 runs, for each residue b < B, the
+// A line of N = A * B points is split in two stages: stage 1 runs, for each residue b < B, the
 // SJ scaled real FFT of length A of v[B a + b] (v: Makhoul's reorder of x); stage 2 runs, for each
 // column c < A / 2, the SJ scaled complex FFT of length B over the twiddled stage-1 outputs and the
 // post rotation that gives y[c + A d] and y[N - c - A d].  The real columns 0 and A/2 make one
@@ -478,8 +478,9 @@ __global__ void __launch_bounds__(ColGeo<N, LP>::T, ColGeo<N, LP>::kBlocks) k_sp
 
 // ---- row pass ----------------------------------------------------------------------------------
 // Rows are staged whole in shared memory in groups of 2 LP, at pitch N + 32 / LP floats: a thread holds
-// rows p and p + LP of a group, and a warp LP such pairs at 32 / LP adjacent b's (or c's), so the
-// scalar walks along the rows hit bank (32 / LP) p + b: conflict-free.
+// rows p and p + LP of a group, and a warp LP such pairs at 32 / LP adjacent c's (or b's), so the
+// scalar walks along the rows hit bank (32 / LP) p + c in stage 2: conflict-free.  Stage 1 walks every
+// second sample (bank (32 / LP) p + 2 b), two lanes to a bank.
 // One group per CTA: 64 threads give 128- and 256-point lines a stage-1 task each, and ten to sixteen
 // such CTAs per SM hide one another's barriers and copies (32 M elements of 256-point rows: 49.7 us,
 // 53.7 as two groups in 128 threads, 63.1 without the register limit; 128: 48.8, 512: 52.0, 1024: 58.2).

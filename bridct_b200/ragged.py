@@ -103,8 +103,9 @@ class RaggedBatch:
         return out
 
     def set_schedule(self, schedule: dict) -> None:
-        """schedule = {"classes": {"HxW/mode": "queue"|"launch"|"launch_small"}, "streams": n};
-        classes not named keep the queue."""
+        """schedule = {"classes": {"HxW/mode": "queue"|"launch"|"launch_small"|"merged"}, "streams": n};
+        classes not named keep the queue.  Where classes are merged, queued ones that the queue would take
+        in two passes (axes of at least 32 points) join their launches from 2^21 elements on."""
         import ctypes as C
 
         names = schedule.get("classes", {})
@@ -137,8 +138,9 @@ class RaggedBatch:
         return y
 
     def apply(self, x, y=None, stream=None):
-        """The whole batch: the queued classes in one persistent launch, the others as their own
-        launches on forked side streams (asynchronous on the current stream)."""
+        """The whole batch: the queued classes in one persistent launch, merged ones (and the queued ones
+        that join them, see set_schedule) in merged launches, the others as their own launches, on forked
+        side streams (asynchronous on the current stream)."""
         return self._go(_lib.lib().bridct_ragged_apply_device, x, y, stream)
 
     def apply_loop(self, x, y=None, stream=None):

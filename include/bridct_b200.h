@@ -145,8 +145,8 @@ BRIDCT_API void bridct_ragged_destroy(bridct_ragged *batch);
 BRIDCT_API size_t bridct_ragged_units(const bridct_ragged *batch);
 /* Runs the whole batch (device pointers, asynchronous on `stream`, capturable in a CUDA graph):
  * the arrays of classes scheduled BRIDCT_RAGGED_QUEUE in one persistent launch (a counter reset and
- * one kernel), and every other class as its own launch on side streams forked from `stream` and
- * joined back into it.  A new batch schedules every class on the queue. */
+ * one kernel), the merged classes and the queued ones that join them in merged launches, and every other
+ * class as its own launch, on side streams forked from `stream` and joined back into it.  A new batch schedules every class on the queue. */
 BRIDCT_API int bridct_ragged_apply_device(bridct_ragged *batch, const float *input, float *output,
                                           void *stream);
 
@@ -159,24 +159,32 @@ BRIDCT_API int bridct_ragged_apply_device(bridct_ragged *batch, const float *inp
  * reference picks a per-(h, w, mode) policy from a table (src/generated/rect_policy.inc,
  * src/plan.c:140-148). */
 enum bridct_ragged_schedule {
-    BRIDCT_RAGGED_QUEUE = 0,               /* units in the persistent kernel's queue           */
+    BRIDCT_RAGGED_QUEUE = 0,               /* units in the persistent kernel's queue (but see
+                                              BRIDCT_RAGGED_MERGED)                           */
     BRIDCT_RAGGED_CLASS_LAUNCH = 1,        /* the class's own fixed-shape launch               */
     BRIDCT_RAGGED_CLASS_LAUNCH_SMALL = 2,  /* the same with the few-array geometry (two-pass)  */
     BRIDCT_RAGGED_MERGED = 3               /* two-pass classes only: column passes, then row
                                               passes, one launch per group of line lengths
-                                              over all MERGED classes                         */
+                                              over all MERGED classes.  Where a batch has such
+                                              classes, QUEUE classes whose arrays the queue
+                                              would take in two passes, with axes of at least
+                                              32 points, join these launches if 2^21 elements
+                                              or more come together: about three times as
+                                              fast as in the queue, with the same results     */
 };
 BRIDCT_API size_t bridct_ragged_class_count(const bridct_ragged *batch);
 /* Kernel launches of one bridct_ragged_apply_device call with the current schedule: the merged
  * passes, one or two per class with its own launches, and the persistent queue kernel when any
  * class is queued. */
 BRIDCT_API size_t bridct_ragged_launch_count(const bridct_ragged *batch);
-/* Shape, mode, array count and schedule of class `cls` (any output pointer may be NULL). */
+/* Shape, mode, array count and schedule of class `cls` (any output pointer may be NULL).  The schedule is
+ * the one that was set, also where a QUEUE class runs in the merged launches. */
 BRIDCT_API int bridct_ragged_class_info(const bridct_ragged *batch, size_t cls, int *height, int *width,
                                         int *mode, size_t *arrays, int *schedule);
 /* Sets every class's schedule (count = bridct_ragged_class_count) and the number of side streams
  * (1..8) that own launches spread over.  Rebuilds the queue: synchronizes the device and may
- * allocate, so call it outside stream capture and before capturing the batch's launches. */
+ * allocate, so call it outside stream capture and before capturing the batch's launches.  On failure the
+ * batch keeps the schedule it had. */
 BRIDCT_API int bridct_ragged_set_schedule(bridct_ragged *batch, const int *schedules, size_t count,
                                           int streams);
 /* One class alone as its own launch (schedule CLASS_LAUNCH or CLASS_LAUNCH_SMALL), for measuring. */
@@ -189,8 +197,10 @@ BRIDCT_API int bridct_ragged_apply_loop_device(bridct_ragged *batch, const float
 BRIDCT_API int bridct_ragged_timeout_flag(bridct_ragged *batch);
 /* Sets how many times (about 256 ns apart) a row block polls for its array's column strips
  * before it gives up, skips its rows and raises the batch's timeout flag; the default is
- * 2^22 (about a second).  0 makes every row block give up at once, which tests use to drive the
- * timeout path deterministically.  No reference counterpart. */
+ * 2^22 (about a second).  Queued arrays of more than 16384 floats have such waits, and so have smaller
+ * ones that one unit's shared memory does not hold (128x128, 64x256, 256x64, 32x512, 16x1024, and
+ * heights of 512 and 1024); all others are single units and never wait.  0 makes every row block give up
+ * at once, which tests use to drive the timeout path deterministically.  No reference counterpart. */
 BRIDCT_API int bridct_ragged_set_wait_limit(bridct_ragged *batch, unsigned polls);
 
 /* No counterpart in the reference.  The ragged batch for callers that cannot let a library
