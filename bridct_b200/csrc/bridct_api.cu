@@ -43,6 +43,11 @@ int cuda_fail(cudaError_t e, const char* what) {
   return BRIDCT_DEVICE_ERROR;
 }
 
+cudaError_t upload_table(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+}
+
 static int lg2(int n) {
   int k = 0;
   while ((8 << k) < n) ++k;
@@ -144,7 +149,7 @@ DeviceCtx* device_ctx(int device) {
     e = cudaMalloc(&mem, t.size() * sizeof(float));
     if (e == cudaSuccess) {
       d->table_mem.push_back(mem);
-      e = cudaMemcpy(mem, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice);
+      e = upload_table(mem, t.data(), t.size() * sizeof(float));
     }
     if (e != cudaSuccess) {
       cuda_fail(e, "split-line tables");

@@ -25,6 +25,10 @@ struct DeviceCtx {
 void set_error(const std::string& s);
 int cuda_fail(cudaError_t e, const char* what);
 double sj_scale(int n, int k);
+// Copies a table to the device and waits until it has arrived.  A plain cudaMemcpy from pageable memory may
+// return while the last part is still on its way, and the kernels that read the tables run on streams that
+// do not wait for the default stream.
+cudaError_t upload_table(void* dst, const void* src, size_t bytes);
 // Rotation tables of the split lines of N = 128..1024 points (sj_split.cuh, SplitTab), float64-derived:
 // their size, and their values to t.
 int split_table_floats(int N);

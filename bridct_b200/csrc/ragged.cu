@@ -195,7 +195,7 @@ int build_classes(bridct_ragged* r) {
     std::vector<long long> offs;
     for (int i : c.arrays) offs.push_back((long long)r->items[i].offset);
     cudaError_t e = cudaMalloc((void**)&c.d_offs, offs.size() * sizeof(long long));
-    if (e == cudaSuccess) e = cudaMemcpy(c.d_offs, offs.data(), offs.size() * sizeof(long long), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload_table(c.d_offs, offs.data(), offs.size() * sizeof(long long));
     if (e != cudaSuccess) return cuda_fail(e, "ragged class tables");
   }
   cudaError_t e = cudaEventCreateWithFlags(&r->fork_ev, cudaEventDisableTiming);
@@ -251,7 +251,7 @@ int build_merged(const bridct_ragged* r, RaggedTables& tables) {
       m.n = (long long)g.size();
       for (const MergedUnit& u : g) m.floats += (size_t)u.n * (col ? merged_strip_cols(u.n) : merged_block_rows(u.n));
       cudaError_t e = cudaMalloc((void**)&m.d_units, g.size() * sizeof(MergedUnit));
-      if (e == cudaSuccess) e = cudaMemcpy(m.d_units, g.data(), g.size() * sizeof(MergedUnit), cudaMemcpyHostToDevice);
+      if (e == cudaSuccess) e = upload_table(m.d_units, g.data(), g.size() * sizeof(MergedUnit));
       if (e != cudaSuccess) {
         cudaFree(m.d_units);
         return cuda_fail(e, "merged pass tables");
@@ -283,9 +283,9 @@ int upload(RaggedTables& t) {
   cudaError_t e = cudaMalloc((void**)&t.d_arrays, t.arrays.size() * sizeof(RaggedArray));
   if (e == cudaSuccess) e = cudaMalloc((void**)&t.d_units, std::max<size_t>(1, t.units.size()) * sizeof(RaggedUnit));
   if (e == cudaSuccess)
-    e = cudaMemcpy(t.d_arrays, t.arrays.data(), t.arrays.size() * sizeof(RaggedArray), cudaMemcpyHostToDevice);
+    e = upload_table(t.d_arrays, t.arrays.data(), t.arrays.size() * sizeof(RaggedArray));
   if (e == cudaSuccess && !t.units.empty())
-    e = cudaMemcpy(t.d_units, t.units.data(), t.units.size() * sizeof(RaggedUnit), cudaMemcpyHostToDevice);
+    e = upload_table(t.d_units, t.units.data(), t.units.size() * sizeof(RaggedUnit));
   return e == cudaSuccess ? BRIDCT_OK : cuda_fail(e, "ragged upload");
 }
 
@@ -373,7 +373,8 @@ BRIDCT_API bridct_ragged* bridct_ragged_create_tuned(const bridct_ragged_item* i
   }
   cudaError_t e = cudaMalloc((void**)&r->d_counters, (count + 1) * sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMalloc((void**)&r->d_err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(r->d_err, 0, sizeof(int));
+  const int zero = 0;
+  if (e == cudaSuccess) e = upload_table(r->d_err, &zero, sizeof(int));
   if (e != cudaSuccess || replace_tables(r) != BRIDCT_OK) {
     if (e != cudaSuccess) cuda_fail(e, "bridct_ragged_create");
     bridct_ragged_destroy(r);
@@ -579,7 +580,8 @@ BRIDCT_API int bridct_ragged_timeout_flag(bridct_ragged* r) {
   DeviceGuard guard(r->device);
   int v = 0;
   cudaMemcpy(&v, r->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (v) cudaMemset(r->d_err, 0, sizeof(int));
+  const int zero = 0;
+  if (v) upload_table(r->d_err, &zero, sizeof(int));
   return v;
 }
 
@@ -767,7 +769,7 @@ extern "C" BRIDCT_API int bridct_ragged_apply_noalloc(const bridct_ragged_item* 
     e = cudaGetSymbolAddress(&p, g_ragged_scratch);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_ragged_scratch)");
     unsigned char* base = static_cast<unsigned char*>(p);
-    e = cudaMemcpy(base + NaOff::tabs, g_na_tabs, sizeof(g_na_tabs), cudaMemcpyHostToDevice);
+    e = upload_table(base + NaOff::tabs, g_na_tabs, sizeof(g_na_tabs));
     if (e != cudaSuccess) return cuda_fail(e, "scratch tables");
     g_na_addr[dev] = base;
   }

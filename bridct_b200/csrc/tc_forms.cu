@@ -207,10 +207,11 @@ TcDevice* tc_device(int dev) {
     for (int inv = 0; inv < 2; ++inv) {
       const std::vector<uint8_t> img = b_image(form, inv != 0);
       if (cudaMalloc(&d.images[form][inv], img.size()) != cudaSuccess) return nullptr;
-      if (cudaMemcpy(d.images[form][inv], img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+      if (upload_table(d.images[form][inv], img.data(), img.size()) != cudaSuccess)
         return nullptr;
     }
-  if (cudaMalloc(&d.err, sizeof(int)) != cudaSuccess || cudaMemset(d.err, 0, sizeof(int)) != cudaSuccess)
+  const int zero = 0;
+  if (cudaMalloc(&d.err, sizeof(int)) != cudaSuccess || upload_table(d.err, &zero, sizeof(int)) != cudaSuccess)
     return nullptr;
   g_tc[dev] = d;
   return &g_tc[dev];
@@ -307,7 +308,7 @@ const uint4* pass_image_device(TcDevice* d, bool inverse) {
     const std::vector<uint8_t> img = pass_image<FORM, L, SUB, FOLD, NARROW>(inverse);
     void* ptr = nullptr;
     if (cudaMalloc(&ptr, img.size()) != cudaSuccess) return nullptr;
-    if (cudaMemcpy(ptr, img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (upload_table(ptr, img.data(), img.size()) != cudaSuccess) {
       cudaFree(ptr);
       return nullptr;
     }
@@ -417,8 +418,8 @@ bool fp8_tables(TcDevice* d, int L, bool inverse, const uint4** img, const float
     void* pi = nullptr;
     void* ps = nullptr;
     if (cudaMalloc(&pi, im.size()) != cudaSuccess || cudaMalloc(&ps, scl.size() * 4) != cudaSuccess) return false;
-    if (cudaMemcpy(pi, im.data(), im.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(ps, scl.data(), scl.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (upload_table(pi, im.data(), im.size()) != cudaSuccess ||
+        upload_table(ps, scl.data(), scl.size() * 4) != cudaSuccess)
       return false;
     d->fp8_images[li][iv] = pi;
     d->fp8_scales[li][iv] = static_cast<float*>(ps);
@@ -723,7 +724,8 @@ int tc_take_error(int device) {
   if (!d) return 0;
   int v = 0;
   cudaMemcpy(&v, d->err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (v) cudaMemset(d->err, 0, sizeof(int));
+  const int zero = 0;
+  if (v) upload_table(d->err, &zero, sizeof(int));
   return v;
 }
 
